@@ -178,10 +178,10 @@ rt_status rtTraceClosestHost(rt_ctx *ctx, rt_scene_id scene, const rt_ray *h_ray
  *                   to 256 rays (the sort's Morton cells) that walk the tree
  *                   once as a beam: the block expands the tile's cone, the
  *                   rays test the leaves it meets (each with its own slab
- *                   test first); 0 (default) = warp packets; 2 = beams on
- *                   Bvh.h's median-split tree (bvh.builder 0 or the caller's
- *                   nodes), whose overlapping boxes favour them, packets on
- *                   the LBVH and PLOC trees. Results are identical either way
+ *                   test first); 0 (default) = warp packets; 2 = beams where
+ *                   rays are cast on Bvh.h's median-split tree (bvh.cast_tree
+ *                   0 or the caller's nodes), whose overlapping boxes favour
+ *                   them, packets on the LBVH and PLOC trees. Results are identical either way
  *   "trace.beam_round"  leaves a beam collects before its rays test them
  *                   (16..256, default 64)
  *   "trace.spec"    1 (default) = per-lane traversal parks the first leaf it
@@ -251,9 +251,17 @@ rt_status rtTraceClosestHost(rt_ctx *ctx, rt_scene_id scene, const rt_ray *h_ray
  *                   the reference's tree, but closest hits are identical
  *                   (equal-t ties go to the lower triangle index in every
  *                   tree); rtDownloadBvh returns the tree that was built
+ *   "bvh.cast_tree" with bvh.builder 0: 1 (default) = rays are cast on a PLOC
+ *                   tree built beside the reference's, whose tighter boxes
+ *                   they cross faster; 0 = on the reference's own. The hits
+ *                   are identical; rtDownloadBvh and the 16-entry compat
+ *                   traversal read the reference's nodes either way. A tree
+ *                   deeper than 64 levels, no memory for its scratch, or a
+ *                   vertex coordinate above 1024 in magnitude leaves the
+ *                   casts on the reference's
  *   "bvh.ploc_radius"  positions on either side the PLOC builder
- *                   (bvh.builder 2) searches for nearest neighbours, 1..256
- *                   (default 16)
+ *                   (bvh.builder 2, bvh.cast_tree 1) searches for nearest
+ *                   neighbours, 1..256 (default 16)
  *   "bvh8.collapse"  how rtUploadScene folds the tree into the 8-wide
  *                   nodes the incoherent caster walks: 1 (default) the
  *                   folded pairs chosen by the surface area heuristic

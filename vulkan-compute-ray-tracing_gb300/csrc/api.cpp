@@ -24,6 +24,14 @@ using namespace rtgb;
 namespace {
 
 constexpr uint32_t kCounterRing = 1024;
+constexpr uint32_t kMaxTreeDepth = 64;     // the traversal stacks' largest size
+constexpr uint32_t kCastTreeRounds = 512;  // a PLOC tree of 64 levels takes fewer
+// A triangle whose fp32 t errs by more than the boxes' padding (1e-4) can be
+// found in one visiting order and pruned in another, so that a hit would
+// depend on the tree. Of 1M rays each into meshes moved by up to 1000 none
+// differed between the trees or between the casting kernels; moved by 3000,
+// up to 9 did between the kernels on one tree.
+constexpr float kCastTreeMaxCoord = 1024.0f;
 
 struct Scene {
   DevScene dev{};
@@ -32,6 +40,7 @@ struct Scene {
   rt_camera camera{};
   bool has_camera = false;
   float build_ms = 0.0f, relayout_ms = 0.0f;
+  uint32_t depth = 0;  // levels of the node array (dev.depth: of the tree rays are cast on)
   uint64_t last_use = 0;
 };
 
@@ -335,7 +344,10 @@ rt_status rtUploadScene(rt_ctx *ctx, const rt_triangle *tris, uint32_t nt, const
         mats[i].fuzz < 0.0f || mats[i].ior < 0.0f)
       return fail(ctx, RT_ERR_INVALID_SCENE, "material %u: non-finite or negative parameter", i);
   }
+  float max_coord = 0.0f;
   for (uint32_t i = 0; i < nt; i++) {
+    for (int k = 0; k < 3; k++)
+      max_coord = std::max({max_coord, std::fabs(tris[i].v0[k]), std::fabs(tris[i].v1[k]), std::fabs(tris[i].v2[k])});
     if (!finite3(tris[i].v0) || !finite3(tris[i].v1) || !finite3(tris[i].v2))
       return fail(ctx, RT_ERR_INVALID_SCENE, "triangle %u: non-finite vertex", i);
     if (tris[i].material_index >= nm)
@@ -403,7 +415,9 @@ rt_status rtUploadScene(rt_ctx *ctx, const rt_triangle *tris, uint32_t nt, const
   d.nspheres = ns;
   d.nnodes = nnodes;
   cudaStream_t st = ctx->stream;
+  rt_bvh_node *cast_scratch = nullptr;  // a cast tree of its own, until the traversal layout is derived
   auto abort_upload = [&](rt_status s) {
+    if (cast_scratch) cudaFreeAsync(cast_scratch, st);
     cudaStreamSynchronize(st);
     cudaFree(slab);
     delete sc;
@@ -421,15 +435,18 @@ rt_status rtUploadScene(rt_ctx *ctx, const rt_triangle *tris, uint32_t nt, const
   if (ns) UCK(cudaMemcpyAsync(slab + off_spheres, spheres, sizeof(rt_sphere) * ns, cudaMemcpyHostToDevice, st), "upload spheres");
   rt_bvh_node *dnodes = (rt_bvh_node *)(slab + off_nodes);
   bool median_tree = nodes != nullptr;
+  const rt_bvh_node *cast_nodes = dnodes;
+  float cast_ms = 0.0f;
   if (nodes) {
     UCK(cudaMemcpyAsync(dnodes, nodes, sizeof(rt_bvh_node) * nnodes, cudaMemcpyHostToDevice, st), "upload nodes");
   } else {
-    int builder = 0, test_error_level = -1, ploc_radius = 16;
+    int builder = 0, test_error_level = -1, ploc_radius = 16, cast_tree = 1;
     {
       std::lock_guard<std::mutex> g(ctx->mu);
       builder = ctx->build_opts.builder;
       test_error_level = ctx->build_opts.test_error_level;
       ploc_radius = ctx->build_opts.ploc_radius;
+      cast_tree = ctx->build_opts.cast_tree;
     }
     char errbuf[256] = {0};
     rt_status bs;
@@ -437,7 +454,7 @@ rt_status rtUploadScene(rt_ctx *ctx, const rt_triangle *tris, uint32_t nt, const
       bs = gpu_build_lbvh((const rt_triangle *)(slab + off_tris), nt, dnodes, st, &sc->build_ms, &depth, errbuf,
                           sizeof(errbuf));
     } else if (builder == 2) {
-      bs = gpu_build_ploc((const rt_triangle *)(slab + off_tris), nt, (uint32_t)ploc_radius, dnodes, st,
+      bs = gpu_build_ploc((const rt_triangle *)(slab + off_tris), nt, (uint32_t)ploc_radius, nt, dnodes, st,
                           &sc->build_ms, &depth, errbuf, sizeof(errbuf));
     } else {
       median_tree = true;
@@ -447,9 +464,34 @@ rt_status rtUploadScene(rt_ctx *ctx, const rt_triangle *tris, uint32_t nt, const
                          errbuf, sizeof(errbuf), test_error_level);
     }
     if (bs != RT_SUCCESS) return abort_upload(fail(ctx, bs, "%s", errbuf));
+    // The tree rays are cast on. Where its scratch memory cannot be had, or
+    // the boxes nest so that it grows too deep for the traversal stacks, they
+    // are cast on the reference's; also where coordinates are so large that
+    // an fp32 rounding nears the boxes' padding (kCastTreeMaxCoord).
+    if (builder == 0 && cast_tree && nt > 2 && max_coord <= kCastTreeMaxCoord) {
+      const cudaError_t ce = cudaMallocAsync((void **)&cast_scratch, sizeof(rt_bvh_node) * nnodes, st);
+      uint32_t cast_depth = 0;
+      if (ce != cudaSuccess) {
+        cast_scratch = nullptr;
+        cudaGetLastError();
+        if (ce != cudaErrorMemoryAllocation) return abort_upload(cuda_fail(ctx, ce, "cast tree scratch"));
+      } else {
+        bs = gpu_build_ploc((const rt_triangle *)(slab + off_tris), nt, (uint32_t)ploc_radius, kCastTreeRounds,
+                            cast_scratch, st, &cast_ms, &cast_depth, errbuf, sizeof(errbuf));
+        if (bs == RT_ERR_CUDA) return abort_upload(fail(ctx, bs, "%s", errbuf));
+        if (bs == RT_ERR_OUT_OF_MEMORY) cudaGetLastError();
+        if (bs == RT_SUCCESS && cast_depth <= kMaxTreeDepth) {
+          cast_nodes = cast_scratch;
+          d.depth = cast_depth;
+          median_tree = false;
+        }
+      }
+    }
   }
-  d.depth = depth;
-  if (depth > 64) return abort_upload(fail(ctx, RT_ERR_INVALID_SCENE, "tree depth %u exceeds 64", depth));
+  sc->depth = depth;
+  if (cast_nodes == dnodes) d.depth = depth;
+  if (d.depth > kMaxTreeDepth)
+    return abort_upload(fail(ctx, RT_ERR_INVALID_SCENE, "tree depth %u exceeds %u", d.depth, kMaxTreeDepth));
   d.median_tree = median_tree ? 1u : 0u;
   // Traversal layout.
   {
@@ -460,7 +502,7 @@ rt_status rtUploadScene(rt_ctx *ctx, const rt_triangle *tris, uint32_t nt, const
     cudaEventCreate(&a);
     cudaEventCreate(&b);
     cudaEventRecord(a, st);
-    cudaError_t le = launch_relayout(dnodes, nnodes, d.tris, (float4 *)d.bvh2, (float4 *)d.tpre,
+    cudaError_t le = launch_relayout(cast_nodes, nnodes, d.tris, (float4 *)d.bvh2, (float4 *)d.tpre,
                                      (int32_t *)d.leaf_tri, scratch, st);
     cudaEventRecord(b, st);
     cudaFreeAsync(scratch, st);
@@ -470,9 +512,12 @@ rt_status rtUploadScene(rt_ctx *ctx, const rt_triangle *tris, uint32_t nt, const
       return abort_upload(cuda_fail(ctx, le, "relayout"));
     }
     rt_bvh_node root;
-    UCK(cudaMemcpyAsync(&root, dnodes, sizeof(root), cudaMemcpyDeviceToHost, st), "read root");
+    UCK(cudaMemcpyAsync(&root, cast_nodes, sizeof(root), cudaMemcpyDeviceToHost, st), "read root");
+    if (cast_scratch) cudaFreeAsync(cast_scratch, st);
+    cast_scratch = nullptr;
     UCK(cudaStreamSynchronize(st), "upload");
     cudaEventElapsedTime(&sc->relayout_ms, a, b);
+    sc->relayout_ms += cast_ms;
     cudaEventDestroy(a);
     cudaEventDestroy(b);
     for (int k = 0; k < 3; k++) {
@@ -533,7 +578,7 @@ rt_status rtGetSceneInfo(rt_ctx *ctx, rt_scene_id id, rt_scene_info *out) {
   out->lights = sc->dev.nlights;
   out->spheres = sc->dev.nspheres;
   out->nodes = sc->dev.nnodes;
-  out->depth = sc->dev.depth;
+  out->depth = sc->depth;
   out->device_bytes = sc->bytes;
   out->build_ms = sc->build_ms;
   out->relayout_ms = sc->relayout_ms;
@@ -895,6 +940,11 @@ rt_status rtSetTuning(rt_ctx *ctx, const char *key, int64_t value) {
     ctx->build_opts.ploc_radius = (int)value;
     return RT_SUCCESS;
   }
+  if (k == "bvh.cast_tree") {
+    if (value < 0 || value > 1) return RT_ERR_INVALID_ARGUMENT;
+    ctx->build_opts.cast_tree = (int)value;
+    return RT_SUCCESS;
+  }
   if (k == "bvh8.collapse") {
     if (value < 0 || value > 1) return RT_ERR_INVALID_ARGUMENT;
     ctx->build_opts.collapse = (int)value;
@@ -1003,6 +1053,10 @@ rt_status rtGetTuning(rt_ctx *ctx, const char *key, int64_t *value) {
   }
   if (k == "bvh.builder") {
     *value = ctx->build_opts.builder;
+    return RT_SUCCESS;
+  }
+  if (k == "bvh.cast_tree") {
+    *value = ctx->build_opts.cast_tree;
     return RT_SUCCESS;
   }
   if (k == "bvh8.collapse") {

@@ -51,6 +51,7 @@
 #include <cstring>
 #include <vector>
 
+#include "grid_sync.cuh"
 #include "rt_internal.h"
 #include "sort_emul.cuh"
 
@@ -568,33 +569,6 @@ struct BigLists {
   uint2 *tile_count;        // !(x < p) and !(p < x) in each tile
   uint32_t max_ranges, max_tiles;
 };
-
-// Barrier over a cooperative grid on a counter that only grows. A CTA that
-// has polled for far longer than any phase takes records an error and leaves;
-// so do the others, at the same or their next barrier.
-__device__ __forceinline__ bool grid_barrier(uint32_t *counter, uint32_t *err, uint32_t &target) {
-  __shared__ int s_ok;
-  target += gridDim.x;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    atomicAdd(counter, 1u);
-    int ok = 0;
-    for (uint32_t poll = 0; poll < (1u << 28); poll++) {
-      const uint32_t at = *reinterpret_cast<volatile uint32_t *>(counter);
-      if ((int32_t)(at - target) >= 0) {
-        ok = 1;
-        break;
-      }
-      if (poll > 64) __nanosleep(32);
-    }
-    if (!ok) atomicOr(err, KERR_TIMEOUT);
-    __threadfence();
-    s_ok = ok;
-  }
-  __syncthreads();
-  return s_ok != 0;
-}
 
 // A range of a big level, added by one CTA: to the queue when one CTA can
 // finish it (or its depth limit has run out), else to the next round's

@@ -10,7 +10,7 @@
 // separately reported mode ("bvh.builder" = 1), not a replacement.
 //
 // Steps: centroid bounds -> 30-bit Morton code per triangle -> stable radix
-// sort (one bit per pass, scan-based split) -> one thread per inner node
+// sort (k_morton_sort) -> one thread per inner node
 // finds its key range and split from the longest common prefixes of
 // neighbouring (code, index) keys -> leaves walk to the root with an atomic
 // visit count per inner node; the second child to arrive writes the union.
@@ -19,6 +19,7 @@
 
 #include <cstdio>
 
+#include "grid_sync.cuh"
 #include "rt_internal.h"
 
 namespace rtgb {
@@ -37,36 +38,11 @@ __device__ __forceinline__ float3 centroid(const rt_triangle &t) {
                      (t.v0[2] + t.v1[2] + t.v2[2]) * (1.0f / 3.0f));
 }
 
-__global__ void k_init_bounds(uint32_t *ext) {
-  if (threadIdx.x < 3) {
-    ext[threadIdx.x] = 0xffffffffu;
-    ext[3 + threadIdx.x] = 0u;
-  }
-}
-
-__global__ void k_bounds(const rt_triangle *__restrict__ tris, uint32_t n, uint32_t *ext) {
-  float lo[3] = {3.4e38f, 3.4e38f, 3.4e38f}, hi[3] = {-3.4e38f, -3.4e38f, -3.4e38f};
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    float3 c = centroid(tris[i]);
-    lo[0] = fminf(lo[0], c.x);
-    lo[1] = fminf(lo[1], c.y);
-    lo[2] = fminf(lo[2], c.z);
-    hi[0] = fmaxf(hi[0], c.x);
-    hi[1] = fmaxf(hi[1], c.y);
-    hi[2] = fmaxf(hi[2], c.z);
-  }
-  for (int k = 0; k < 3; k++) {
-    for (int o = 16; o > 0; o >>= 1) {
-      lo[k] = fminf(lo[k], __shfl_xor_sync(0xffffffffu, lo[k], o));
-      hi[k] = fmaxf(hi[k], __shfl_xor_sync(0xffffffffu, hi[k], o));
-    }
-  }
-  if ((threadIdx.x & 31) == 0)
-    for (int k = 0; k < 3; k++) {
-      atomicMin(ext + k, f2o(lo[k]));
-      atomicMax(ext + 3 + k, f2o(hi[k]));
-    }
-}
+constexpr int kSortThreads = 512;
+constexpr uint32_t kSortWarps = kSortThreads / 32;
+constexpr uint32_t kSortPer = 8;                             // keys a lane holds at most
+constexpr uint32_t kSortMaxGrid = 512;
+constexpr uint32_t kRadix = 256;
 
 __device__ __forceinline__ uint32_t spread10(uint32_t v) {
   v &= 1023u;
@@ -77,38 +53,152 @@ __device__ __forceinline__ uint32_t spread10(uint32_t v) {
   return v;
 }
 
-__global__ void k_morton(const rt_triangle *__restrict__ tris, uint32_t n, const uint32_t *ext, uint32_t *codes,
-                         uint32_t *idx) {
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  float3 c = centroid(tris[i]);
-  float p[3] = {c.x, c.y, c.z};
-  uint32_t q[3];
-  for (int k = 0; k < 3; k++) {
-    float lo = o2f(ext[k]), span = o2f(ext[3 + k]) - lo;
-    float t = span > 0.0f ? (p[k] - lo) / span : 0.0f;
-    t = fminf(fmaxf(t, 0.0f), 1.0f);
-    q[k] = min(1023u, (uint32_t)(t * 1024.0f));
+
+// Morton codes of the centroids and their stable radix sort, in one
+// cooperative launch: centroid bounds; codes; four 8-bit passes, each a
+// digit histogram per CTA (over its contiguous run of keys), a scan of each
+// digit's row over the CTAs, and the scatter, a grid barrier apart. Within a
+// tile a warp ranks equal digits with match_any, in order, and the warps'
+// counts are prefixed per digit. Latency-bound (12 barriers). A run is short
+// (512 keys) rather than the grid small where there are few keys. Measured:
+// 0.17 ms for 1.31M triangles, 0.04 ms for 12K (one-bit passes of five
+// launches each: 1.0 and 0.4 ms).
+//   sync: barrier counter, error bits, then the ordered bounds (6 words)
+//   rows: kRadix x gridDim.x counts, then kRadix totals
+__global__ void __launch_bounds__(kSortThreads) k_morton_sort(const rt_triangle *__restrict__ tris, uint32_t n,
+                                                              uint32_t *sync, uint32_t *codes0, uint32_t *codes1,
+                                                              uint32_t *idx0, uint32_t *idx1, uint32_t *rows) {
+  __shared__ uint32_t s_warp[kSortWarps][kRadix], s_base[kRadix], s_part[kSortWarps];
+  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, lt = (1u << lane) - 1u;
+  uint32_t *err = sync + 1, *ext = sync + 2, *totals = rows + kRadix * gridDim.x;
+  uint32_t target = 0;
+  // Each CTA keeps to one run of keys, `per` a lane at a time.
+  const uint32_t run = (n + gridDim.x - 1) / gridDim.x;
+  const uint32_t per = min(kSortPer, (run + kSortThreads - 1) / kSortThreads), tile = per * kSortThreads;
+  const uint32_t beg = (uint32_t)min((uint64_t)blockIdx.x * run, (uint64_t)n);
+  const uint32_t end = min(n, beg + run);
+  {
+    float lo[3] = {3.4e38f, 3.4e38f, 3.4e38f}, hi[3] = {-3.4e38f, -3.4e38f, -3.4e38f};
+    for (uint32_t i = beg + tid; i < end; i += kSortThreads) {
+      const float3 c = centroid(tris[i]);
+      lo[0] = fminf(lo[0], c.x), lo[1] = fminf(lo[1], c.y), lo[2] = fminf(lo[2], c.z);
+      hi[0] = fmaxf(hi[0], c.x), hi[1] = fmaxf(hi[1], c.y), hi[2] = fmaxf(hi[2], c.z);
+    }
+    for (int k = 0; k < 3; k++) {
+      const uint32_t a = __reduce_min_sync(0xffffffffu, f2o(lo[k])), b = __reduce_max_sync(0xffffffffu, f2o(hi[k]));
+      if (lane == 0) {
+        atomicMin(ext + k, a);
+        atomicMax(ext + 3 + k, b);
+      }
+    }
   }
-  codes[i] = (spread10(q[0]) << 2) | (spread10(q[1]) << 1) | spread10(q[2]);
-  idx[i] = i;
-}
-
-__global__ void k_bitflag(const uint32_t *__restrict__ codes, uint32_t n, int bit, uint32_t *flag) {
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) flag[i] = ((codes[i] >> bit) & 1u) ? 0u : 1u;
-}
-
-// Stable split: keys with the bit clear keep their order first, then the rest.
-__global__ void k_split(const uint32_t *__restrict__ codes, const uint32_t *__restrict__ idx,
-                        const uint32_t *__restrict__ flag, const uint32_t *__restrict__ pos, uint32_t n,
-                        uint32_t *codes_out, uint32_t *idx_out) {
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const uint32_t zeros = pos[n - 1] + flag[n - 1];
-  uint32_t dst = flag[i] ? pos[i] : zeros + (i - pos[i]);
-  codes_out[dst] = codes[i];
-  idx_out[dst] = idx[i];
+  if (!grid_barrier(sync, err, target)) return;
+  float lo[3], span[3];
+  for (int k = 0; k < 3; k++) {
+    lo[k] = o2f(__ldcg(ext + k));
+    span[k] = o2f(__ldcg(ext + 3 + k)) - lo[k];
+  }
+  for (uint32_t i = beg + tid; i < end; i += kSortThreads) {
+    const float3 c = centroid(tris[i]);
+    const float p[3] = {c.x, c.y, c.z};
+    uint32_t q[3];
+    for (int k = 0; k < 3; k++) {
+      float t = span[k] > 0.0f ? (p[k] - lo[k]) / span[k] : 0.0f;
+      t = fminf(fmaxf(t, 0.0f), 1.0f);
+      q[k] = min(1023u, (uint32_t)(t * 1024.0f));
+    }
+    codes0[i] = (spread10(q[0]) << 2) | (spread10(q[1]) << 1) | spread10(q[2]);
+    idx0[i] = i;
+  }
+  for (int pass = 0; pass < 4; pass++) {
+    const uint32_t *ci = pass & 1 ? codes1 : codes0, *vi = pass & 1 ? idx1 : idx0;
+    uint32_t *co = pass & 1 ? codes0 : codes1, *vo = pass & 1 ? idx0 : idx1;
+    const int shift = 8 * pass;
+    __syncthreads();  // pass 0: the codes of this CTA's run (its own writes)
+    for (uint32_t d = tid; d < kRadix; d += kSortThreads) s_base[d] = 0u;
+    __syncthreads();
+    for (uint32_t i = beg + tid; i < end; i += kSortThreads) atomicAdd(&s_base[(__ldcg(ci + i) >> shift) & 255u], 1u);
+    __syncthreads();
+    for (uint32_t d = tid; d < kRadix; d += kSortThreads) rows[d * gridDim.x + blockIdx.x] = s_base[d];
+    if (!grid_barrier(sync, err, target)) return;
+    // Rows: exclusive prefix over the CTAs and the total, a warp each.
+    for (uint32_t d = blockIdx.x * kSortWarps + warp; d < kRadix; d += gridDim.x * kSortWarps) {
+      uint32_t before = 0;
+      for (uint32_t b0 = 0; b0 < gridDim.x; b0 += 32) {
+        const uint32_t v = b0 + lane < gridDim.x ? __ldcg(rows + d * gridDim.x + b0 + lane) : 0u;
+        uint32_t x = v;
+        for (int o = 1; o < 32; o <<= 1) {
+          const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+          if (lane >= (uint32_t)o) x += y;
+        }
+        if (b0 + lane < gridDim.x) rows[d * gridDim.x + b0 + lane] = before + x - v;
+        before += __shfl_sync(0xffffffffu, x, 31);
+      }
+      if (lane == 0) totals[d] = before;
+    }
+    if (!grid_barrier(sync, err, target)) return;
+    // This CTA's first slot per digit: the smaller digits, then its column of the digit's row.
+    if (tid < kRadix) {
+      const uint32_t v = __ldcg(totals + tid);
+      uint32_t x = v;
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= (uint32_t)o) x += y;
+      }
+      if (lane == 31) s_part[warp] = x;
+      s_base[tid] = x - v + __ldcg(rows + tid * gridDim.x + blockIdx.x);
+    }
+    __syncthreads();
+    if (tid < kRadix) {
+      uint32_t before = 0;
+      for (uint32_t w = 0; w < warp; w++) before += s_part[w];
+      s_base[tid] += before;
+    }
+    for (uint32_t t0 = beg; t0 < end; t0 += tile) {
+      for (uint32_t d = tid; d < kSortWarps * kRadix; d += kSortThreads) (&s_warp[0][0])[d] = 0u;
+      __syncthreads();
+      uint32_t c[kSortPer], v[kSortPer], rank[kSortPer];
+      const uint32_t w0 = t0 + warp * (32 * per);
+#pragma unroll
+      for (uint32_t j = 0; j < kSortPer; j++) {
+        const uint32_t i = w0 + j * 32 + lane;
+        c[j] = j < per && i < end ? __ldcg(ci + i) : 0u;
+        v[j] = j < per && i < end ? __ldcg(vi + i) : 0u;
+      }
+#pragma unroll
+      for (uint32_t j = 0; j < kSortPer; j++) {
+        if (j >= per) continue;
+        const bool in = w0 + j * 32 + lane < end;
+        const uint32_t d = in ? (c[j] >> shift) & 255u : kRadix;  // lanes past the end match only one another
+        const uint32_t same = __match_any_sync(0xffffffffu, d);
+        const uint32_t at = in ? s_warp[warp][d] : 0u;
+        __syncwarp();
+        if (in && (same & lt) == 0) s_warp[warp][d] = at + __popc(same);
+        __syncwarp();
+        rank[j] = at + __popc(same & lt);
+      }
+      __syncthreads();
+      if (tid < kRadix) {
+        uint32_t at = s_base[tid];
+        for (uint32_t w = 0; w < kSortWarps; w++) {
+          const uint32_t m = s_warp[w][tid];
+          s_warp[w][tid] = at;
+          at += m;
+        }
+        s_base[tid] = at;
+      }
+      __syncthreads();
+#pragma unroll
+      for (uint32_t j = 0; j < kSortPer; j++) {
+        if (j >= per || w0 + j * 32 + lane >= end) continue;
+        const uint32_t at = s_warp[warp][(c[j] >> shift) & 255u] + rank[j];
+        co[at] = c[j];
+        vo[at] = v[j];
+      }
+      __syncthreads();
+    }
+    if (pass < 3 && !grid_barrier(sync, err, target)) return;
+  }
 }
 
 // Longest common prefix of the keys (code, position) at i and j; -1 outside.
@@ -219,36 +309,31 @@ __global__ void k_lbvh_boxes(const rt_triangle *__restrict__ tris, const uint32_
 
 }  // namespace
 
-size_t lbvh_sorted_keys_words(uint32_t n) { return 16 + 6ull * n + (n / 1024 + 8); }
+size_t lbvh_sorted_keys_words(uint32_t n) { return 64 + 4ull * n + kRadix * (kSortMaxGrid + 1); }
 
 // Centroid bounds -> Morton codes -> stable radix sort. `scratch` holds
-// lbvh_sorted_keys_words(n) words: bounds 16 | codes 2n | indices 2n |
-// flags n | scan n | scan block sums n/1024+8. The sorted codes and triangle
-// indices are returned as pointers into it.
+// lbvh_sorted_keys_words(n) words: barrier, error bits and bounds 64 | codes
+// 2n | indices 2n | digit rows. The sorted codes and triangle indices are
+// returned as pointers into it.
 cudaError_t lbvh_sorted_keys(const rt_triangle *d_tris, uint32_t n, uint32_t *scratch, uint32_t **codes_out,
-                             uint32_t **idx_out, cudaStream_t st) {
-  uint32_t *ext = scratch;
-  uint32_t *codes[2] = {ext + 16, ext + 16 + n};
-  uint32_t *idx[2] = {ext + 16 + 2ull * n, ext + 16 + 3ull * n};
-  uint32_t *flag = ext + 16 + 4ull * n;
-  uint32_t *pos = flag + n;
-  uint32_t *sums = pos + n;
-  const uint32_t B = 256, G = (n + B - 1) / B;
-  k_init_bounds<<<1, 32, 0, st>>>(ext);
-  k_bounds<<<304, 256, 0, st>>>(d_tris, n, ext);
-  k_morton<<<G, B, 0, st>>>(d_tris, n, ext, codes[0], idx[0]);
-  int cur = 0;
-  cudaError_t e = cudaSuccess;
-  for (int bit = 0; bit < 30; bit++) {
-    k_bitflag<<<G, B, 0, st>>>(codes[cur], n, bit, flag);
-    e = exclusive_scan_u32(flag, pos, sums, n, st);
-    if (e != cudaSuccess) return e;
-    k_split<<<G, B, 0, st>>>(codes[cur], idx[cur], flag, pos, n, codes[cur ^ 1], idx[cur ^ 1]);
-    cur ^= 1;
-  }
-  *codes_out = codes[cur];
-  *idx_out = idx[cur];
-  return cudaGetLastError();
+                             uint32_t **idx_out, uint32_t **err_out, cudaStream_t st) {
+  uint32_t *sync = scratch, *codes0 = scratch + 64, *codes1 = codes0 + n, *idx0 = codes1 + n, *idx1 = idx0 + n;
+  uint32_t *rows = idx1 + n;
+  int dev = 0, sms = 0, per_sm = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_morton_sort, kSortThreads, 0);
+  if (e == cudaSuccess) e = cudaMemsetAsync(sync, 0, 4 * 64, st);
+  if (e == cudaSuccess) e = cudaMemsetAsync(sync + 2, 0xff, 4 * 3, st);  // lower bounds
+  if (e != cudaSuccess) return e;
+  const uint32_t grid =
+      min(min((uint32_t)sms * (uint32_t)max(1, min(per_sm, 2)), kSortMaxGrid), (n + kSortThreads - 1) / kSortThreads);
+  void *args[] = {&d_tris, &n, &sync, &codes0, &codes1, &idx0, &idx1, &rows};
+  e = cudaLaunchCooperativeKernel((const void *)k_morton_sort, dim3(grid), dim3(kSortThreads), args, 0, st);
+  *codes_out = codes0;  // four passes: back in the first pair
+  *idx_out = idx0;
+  *err_out = sync + 1;
+  return e;
 }
 
 rt_status gpu_build_lbvh(const rt_triangle *d_tris, uint32_t n, rt_bvh_node *d_nodes, cudaStream_t st, float *ms_out,
@@ -277,8 +362,8 @@ rt_status gpu_build_lbvh(const rt_triangle *d_tris, uint32_t n, rt_bvh_node *d_n
   uint32_t *dmax = visits + n;
   cudaEventRecord(e0, st);
   const uint32_t B = 256, G = (n + B - 1) / B;
-  uint32_t *codes = nullptr, *idx = nullptr;
-  e = lbvh_sorted_keys(d_tris, n, sortbuf, &codes, &idx, st);
+  uint32_t *codes = nullptr, *idx = nullptr, *sort_err = nullptr;
+  e = lbvh_sorted_keys(d_tris, n, sortbuf, &codes, &idx, &sort_err, st);
   if (e == cudaSuccess) {
     cudaMemsetAsync(visits, 0, 4ull * n + 32, st);  // visit counts and the depth word
     cudaMemsetAsync(parent, 0xff, 4ull * 2 * n, st);
@@ -286,8 +371,9 @@ rt_status gpu_build_lbvh(const rt_triangle *d_tris, uint32_t n, rt_bvh_node *d_n
     k_lbvh_boxes<<<G, B, 0, st>>>(d_tris, idx, (int)n, left, right, parent, visits, d_nodes, dmax);
   }
   cudaEventRecord(e1, st);
-  uint32_t depth = 0;
+  uint32_t depth = 0, sort_bits = 0;
   cudaMemcpyAsync(&depth, dmax, 4, cudaMemcpyDeviceToHost, st);
+  cudaMemcpyAsync(&sort_bits, sortbuf + 1, 4, cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   float ms = 0.0f;
@@ -299,7 +385,7 @@ rt_status gpu_build_lbvh(const rt_triangle *d_tris, uint32_t n, rt_bvh_node *d_n
     std::snprintf(errbuf, errlen, "lbvh build: %s", cudaGetErrorString(e));
     return RT_ERR_CUDA;
   }
-  if (depth == 0xffffffffu || depth == 0) {
+  if (depth == 0xffffffffu || depth == 0 || sort_bits) {
     std::snprintf(errbuf, errlen, "lbvh build: malformed tree");
     return RT_ERR_INTERNAL;
   }

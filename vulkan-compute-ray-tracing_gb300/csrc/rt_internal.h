@@ -211,6 +211,14 @@ struct BuildOpts {
   int builder = 0;  // 0 the reference's Bvh.h tree (bit-exact), 1 LBVH, 2 PLOC
   int collapse = 1;  // 8-wide fold: 1 SAH-chosen pairs, 0 largest child first ("bvh8.collapse")
   int ploc_radius = 16;  // PLOC's nearest-neighbour search radius ("bvh.ploc_radius")
+  // Builder 0: rays are cast on a PLOC tree built beside the reference's
+  // (1), or on the reference's own (0) ("bvh.cast_tree"). A closest hit does
+  // not depend on the tree; the nodes that rtDownloadBvh and the 16-entry
+  // compat traversal read are the reference's either way. Measured, cast on
+  // the reference's tree / on PLOC: 4.19M random rays into 1.31M triangles
+  // 7.4 / 4.9 ms, camera rays 4.9 / 4.5 ms, a 1080p frame of 2M triangles
+  // 14.4 / 5.1 ms, a 256 x 256 Cornell frame 1.27 / 0.80 ms.
+  int cast_tree = 1;
   int test_error_level = -1;  // test hook of gpu_build_bvh's error word (-1: off)
 };
 
@@ -272,11 +280,13 @@ rt_status gpu_build_lbvh(const rt_triangle *d_tris, uint32_t n, rt_bvh_node *d_n
 // Morton-sorted triangle centroids (lbvh.cu), shared by the LBVH and PLOC builders.
 size_t lbvh_sorted_keys_words(uint32_t n);
 cudaError_t lbvh_sorted_keys(const rt_triangle *d_tris, uint32_t n, uint32_t *scratch, uint32_t **codes_out,
-                             uint32_t **idx_out, cudaStream_t st);
+                             uint32_t **idx_out, uint32_t **err_out, cudaStream_t st);
 // Agglomerative-clustering tree (ploc.cu), Bvh.h node layout, root node 0;
-// nearest neighbours searched within `radius` (1..256) positions.
-rt_status gpu_build_ploc(const rt_triangle *d_tris, uint32_t n, uint32_t radius, rt_bvh_node *d_nodes,
-                         cudaStream_t st, float *ms_out, uint32_t *depth_out, char *errbuf, size_t errlen);
+// nearest neighbours searched within `radius` (1..256) positions. Fails with
+// RT_ERR_INTERNAL when max_rounds rounds leave more than one cluster.
+rt_status gpu_build_ploc(const rt_triangle *d_tris, uint32_t n, uint32_t radius, uint32_t max_rounds,
+                         rt_bvh_node *d_nodes, cudaStream_t st, float *ms_out, uint32_t *depth_out, char *errbuf,
+                         size_t errlen);
 
 // ---------------------------------------------------------------- glibc_rand.cpp
 // glibc's TYPE_3 random() (what rand() returns) after srand(seed).
