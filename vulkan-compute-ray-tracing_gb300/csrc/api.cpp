@@ -789,15 +789,24 @@ rt_status rtRender(rt_ctx *ctx, rt_scene_id id, const rt_render_params *p, float
     ropts = ctx->render_opts;
     topts = ctx->trace_opts;
   }
-  const uint64_t pixels = (uint64_t)p->width * p->height;
-  if (use_wavefront(ropts, *p)) {
+  // A call of several samples of a small image is a wavefront only where its
+  // scratch can be had and the stream is not being captured (a graph would
+  // get memory nodes it did not have as one launch); else one launch.
+  const bool small = ropts.mode == 2 && (uint64_t)p->width * p->height < ropts.wavefront_pixels;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (small && p->spp > 1) CK(cudaStreamIsCapturing(st, &capture), "capture status");
+  if (use_wavefront(ropts, *p) && !(small && capture != cudaStreamCaptureStatusNone)) {
     void *scratch = nullptr;
-    CK(cudaMallocAsync(&scratch, wavefront_scratch_bytes((uint32_t)pixels), st), "wavefront scratch");
-    cudaError_t e = launch_render_wavefront(d, cam, *p, accum, ctx->d_segments, next_counter(ctx), ctx->d_err, scratch,
-                                            ropts.sort != 0, use_wide(topts, d), st);
-    cudaFreeAsync(scratch, st);
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "render launch");
-    return RT_SUCCESS;
+    cudaError_t e = cudaMallocAsync(&scratch, wavefront_scratch_bytes(*p, ropts.sort != 0), st);
+    if (e == cudaSuccess) {
+      e = launch_render_wavefront(d, cam, *p, accum, ctx->d_segments, ctx->d_err, scratch, ropts.sort != 0,
+                                  use_wide(topts, d), st);
+      cudaFreeAsync(scratch, st);
+      if (e != cudaSuccess) return cuda_fail(ctx, e, "render launch");
+      return RT_SUCCESS;
+    }
+    if (!small || e != cudaErrorMemoryAllocation) return cuda_fail(ctx, e, "wavefront scratch");
+    cudaGetLastError();
   }
   cudaError_t e = launch_render(d, cam, *p, accum, ctx->d_segments, ctx->d_err, st);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "render launch");
@@ -1153,8 +1162,7 @@ struct rt_batch {
   std::vector<BatchJob> wf;    // wavefront jobs (host copies)
   BatchJob *d_wf = nullptr;    // their device copies: sample_index advances there
   // Wavefront jobs alternate between `sides` side streams (render.batch_streams,
-  // at most kSides), each with its own scratch and work counter
-  // (counter[64 * (1 + k)]).
+  // at most kSides), each with its own scratch.
   static constexpr int kSides = 16;
   int sides = 0;
   void *wf_scratch[kSides] = {};
@@ -1220,8 +1228,7 @@ cudaError_t batch_enqueue(rt_ctx *ctx, rt_batch *b, cudaStream_t st) {
     for (size_t j = 0; j < b->wf.size() && e == cudaSuccess; j++) {
       const BatchJob &J = b->wf[j];
       const int k = (int)(j % (size_t)sides);
-      e = launch_render_wavefront(J.sc, J.cam, J.p, J.accum, ctx->d_segments, b->counter + 64 * (1 + k), ctx->d_err,
-                                  b->wf_scratch[k], b->wf_sort, b->wf_wide && J.sc.ntris >= b->wf_wide_min,
+      e = launch_render_wavefront(J.sc, J.cam, J.p, J.accum, ctx->d_segments, ctx->d_err, b->wf_scratch[k], b->wf_sort, b->wf_wide && J.sc.ntris >= b->wf_wide_min,
                                   b->side[k], &b->d_wf[j].p.sample_index);
     }
     for (int k = 0; k < sides && e == cudaSuccess; k++) e = cudaEventRecord(b->join[k], b->side[k]);
@@ -1262,12 +1269,12 @@ rt_status rtBatchCreate(rt_ctx *ctx, const rt_render_job *jobs, uint32_t n_jobs,
   std::vector<BatchJob> tiles_jobs;
   rt_batch *b = new rt_batch();
   uint64_t tiles = 0;
-  uint32_t max_wf = 0;
+  size_t wf_bytes = 0;
   b->max_depth = 1;
   for (const BatchJob &J : host) {
     if (wavefront_job(ropts, J.p)) {
       b->wf.push_back(J);
-      max_wf = std::max(max_wf, J.p.width * J.p.height);
+      wf_bytes = std::max(wf_bytes, wavefront_scratch_bytes(J.p, ropts.sort != 0));
     } else {
       BatchJob T = J;
       T.tile_begin = (uint32_t)tiles;
@@ -1284,7 +1291,7 @@ rt_status rtBatchCreate(rt_ctx *ctx, const rt_render_job *jobs, uint32_t n_jobs,
   b->wf_wide = topts.wide != 0;
   b->wf_wide_min = topts.wide_min_tris;
   cudaError_t e = cudaMalloc((void **)&b->d_jobs, sizeof(BatchJob) * std::max(b->n, 1u));
-  if (e == cudaSuccess) e = cudaMalloc((void **)&b->counter, 256 * (1 + rt_batch::kSides));
+  if (e == cudaSuccess) e = cudaMalloc((void **)&b->counter, 256);
   if (e == cudaSuccess && b->n)
     e = cudaMemcpy(b->d_jobs, tiles_jobs.data(), sizeof(BatchJob) * b->n, cudaMemcpyHostToDevice);
   if (e == cudaSuccess && !b->wf.empty()) {
@@ -1296,7 +1303,7 @@ rt_status rtBatchCreate(rt_ctx *ctx, const rt_render_job *jobs, uint32_t n_jobs,
         (int)std::min<size_t>(b->wf.size(), (size_t)std::clamp(ropts.batch_streams, 1, rt_batch::kSides));
     b->sides = sides;
     for (int k = 0; k < sides && e == cudaSuccess; k++) {
-      e = cudaMalloc(&b->wf_scratch[k], wavefront_scratch_bytes(max_wf));
+      e = cudaMalloc(&b->wf_scratch[k], wf_bytes);
       if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->side[k], cudaStreamNonBlocking);
       if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->join[k], cudaEventDisableTiming);
     }

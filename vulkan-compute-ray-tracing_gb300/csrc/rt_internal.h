@@ -164,21 +164,25 @@ cudaError_t launch_render(const DevScene &sc, const rt_camera &cam, const rt_ren
                           unsigned long long *segments, uint32_t *err, cudaStream_t st);
 
 // Wavefront render (wavefront.cu): same images as launch_render; `scratch`
-// holds wavefront_scratch_bytes(width*height); `counter` is a launch-private
-// device word. With d_sample_index the kernels read the first sample index
-// from the device at run time instead of p.sample_index.
-size_t wavefront_scratch_bytes(uint32_t cap);
-// `wide`: bounce rays that fail the packet test are cast by the 8-wide
-// caster (launch_wide_leaf) instead of in place.
+// holds wavefront_scratch_bytes(p, sort). With d_sample_index the kernels read
+// the first sample index from the device at run time instead of
+// p.sample_index.
+size_t wavefront_scratch_bytes(const rt_render_params &p, bool sort);
+// `wide`: bounce rays are cast by the 8-wide caster (launch_wide_leaf).
 cudaError_t launch_render_wavefront(const DevScene &sc, const rt_camera &cam, const rt_render_params &p, float *accum,
-                                    unsigned long long *segments, uint32_t *counter, uint32_t *err, void *scratch,
-                                    bool sort, bool wide, cudaStream_t st,
-                                    const uint32_t *d_sample_index = nullptr);
+                                    unsigned long long *segments, uint32_t *err, void *scratch, bool sort, bool wide,
+                                    cudaStream_t st, const uint32_t *d_sample_index = nullptr);
 
 // Render launch-shape knobs (rtSetTuning "render.mode").
 struct RenderOpts {
   int mode = 2;                         // 0 megakernel, 1 wavefront, 2 choose by image size
-  uint64_t wavefront_pixels = 1u << 18;  // mode 2: wavefront from this many pixels up
+  // mode 2: calls of one sample run as a wavefront from this many pixels up,
+  // calls of several samples always: the samples share a wave, where the
+  // megakernel's threads run them one after the other. Megakernel / wavefront,
+  // Cornell box with 12K triangles, 8 bounces, us: 1 sample 256 x 256 762 /
+  // 1077, 384 x 384 1364 / 1294, 512 x 512 2261 / 1721; 4 samples 48 x 48
+  // 2354 / 983, 256 x 256 3009 / 1717, 512 x 512 8897 / 4344.
+  uint64_t wavefront_pixels = 1u << 18;
   int batch_streams = 16;                // side streams a batch spreads its wavefront jobs over (1..16)
   // Batches and the render server: jobs from this many pixels up run as
   // wavefronts on side streams (the rest in the persistent tile launch).
@@ -197,13 +201,15 @@ struct RenderOpts {
 inline bool use_wavefront(const RenderOpts &o, const rt_render_params &p) {
   if (p.flags & RT_COMPAT_STACK16) return false;  // the literal 16-entry traversal is megakernel-only
   const uint64_t pixels = (uint64_t)p.width * p.height;
-  return pixels < (1ull << 31) && (o.mode == 1 || (o.mode == 2 && pixels >= o.wavefront_pixels));
+  return pixels < (1ull << 31) && (o.mode == 1 || (o.mode == 2 && (p.spp > 1 || pixels >= o.wavefront_pixels)));
 }
 // True when a job of a batch or a server step goes to the wavefront kernels.
 inline bool use_wavefront_batched(const RenderOpts &o, const rt_render_params &p) {
+  rt_render_params one = p;
+  one.spp = 1;
   RenderOpts b = o;
   b.wavefront_pixels = o.batch_wavefront_pixels;
-  return use_wavefront(b, p);
+  return use_wavefront(b, one);
 }
 
 // Tree used when a scene is uploaded without nodes (rtSetTuning "bvh.builder").

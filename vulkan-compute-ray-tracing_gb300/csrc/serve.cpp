@@ -77,7 +77,7 @@ struct rt_server {
   double busy_since = -1.0;
   cudaStream_t stream = nullptr;
   BatchJob *d_jobs = nullptr, *h_jobs = nullptr;
-  uint32_t *d_counter = nullptr;  // [0] tile counter, [64 * (1 + k)] side k's work counter
+  uint32_t *d_counter = nullptr;  // tile counter
   int device = 0;
   // Wavefront side streams, their scratch (grown on demand) and join events.
   static constexpr int kSides = 16;
@@ -238,7 +238,7 @@ void scheduler(rt_server *s) {
     for (int k = 0; k < sides && e == cudaSuccess; k++) {
       size_t need = 0;
       for (size_t j = k; j < wf.size(); j += rt_server::kSides)
-        need = std::max(need, wavefront_scratch_bytes(wf[j].p.width * wf[j].p.height));
+        need = std::max(need, wavefront_scratch_bytes(wf[j].p, sort));
       if (need > s->scratch_bytes[k]) {
         if (s->scratch[k]) cudaFree(s->scratch[k]);
         s->scratch[k] = nullptr;
@@ -253,9 +253,8 @@ void scheduler(rt_server *s) {
       for (size_t j = 0; j < wf.size() && e == cudaSuccess; j++) {
         const int k = (int)(j % rt_server::kSides);
         const BatchJob &J = wf[j];
-        e = launch_render_wavefront(J.sc, J.cam, J.p, J.accum, ctx_segments(s->ctx), s->d_counter + 64 * (1 + k),
-                                    ctx_err(s->ctx), s->scratch[k], sort, wide && J.sc.ntris >= wide_min,
-                                    s->side[k]);
+        e = launch_render_wavefront(J.sc, J.cam, J.p, J.accum, ctx_segments(s->ctx), ctx_err(s->ctx), s->scratch[k],
+                                    sort, wide && J.sc.ntris >= wide_min, s->side[k]);
       }
       for (int k = 0; k < sides && e == cudaSuccess; k++) e = cudaEventRecord(s->join[k], s->side[k]);
     }
@@ -318,7 +317,7 @@ rt_status rtServerCreate(rt_ctx *ctx, const rt_server_desc *desc, rt_server **ou
   cudaError_t e = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaMalloc((void **)&s->d_jobs, sizeof(BatchJob) * cap);
   if (e == cudaSuccess) e = cudaMallocHost((void **)&s->h_jobs, sizeof(BatchJob) * cap);
-  if (e == cudaSuccess) e = cudaMalloc((void **)&s->d_counter, 256 * (1 + rt_server::kSides));
+  if (e == cudaSuccess) e = cudaMalloc((void **)&s->d_counter, 256);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->fork, cudaEventDisableTiming);
   for (int k = 0; k < rt_server::kSides && e == cudaSuccess; k++) {
     e = cudaStreamCreateWithFlags(&s->side[k], cudaStreamNonBlocking);

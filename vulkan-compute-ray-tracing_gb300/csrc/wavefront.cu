@@ -1,12 +1,15 @@
 // Wavefront render: the bounce loop of ray-trace-compute.comp:314-338 split
-// into kernels over queues of live paths.
+// into kernels over queues of live paths. A path is one sample of one pixel;
+// the samples of a call run together, as many at a time as kWavePaths holds.
 //
-//   raygen      one path per pixel for sample s (colour 1, the pixel's RNG
-//               seed, the normalised camera ray) -> queue 0
-//   per bounce  [Morton reorder of the queue's rays, render.sort] -> extend (closest
-//               triangle per ray) -> shade (record, spheres, scatter, colour;
-//               surviving paths are compacted into the other queue)
-//   accumulate  the running mean of comp:375-377 for sample s
+//   camera      closest triangle of every pixel's camera ray, once per call
+//               (the ray carries no jitter), 8 x 4 pixel tiles as packets
+//   first       per path: record, spheres, scatter of the camera hit with the
+//               path's own RNG stream; surviving paths go to the queue
+//   per bounce  [Morton reorder of the queue's rays, render.sort] -> closest
+//               triangle per ray (the 8-wide caster) -> shade (as above, into
+//               the other queue)
+//   accumulate  the running mean of comp:375-377, sample by sample
 //
 // Every floating-point step is the megakernel's (shade.cuh); only the order
 // in which paths are processed changes, so images are identical to the
@@ -20,29 +23,58 @@
 // a CUDA graph).
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "rt_internal.h"
 #include "shade.cuh"
 
 namespace rtgb {
 namespace {
 
-constexpr int kWfBlock = 128;
+constexpr int kWfBlock = 128, kShadeBlock = 256;
+
+// Paths of one wave: samples of a call are added until this many run
+// together. A wave of fewer leaves the GPU idle in every bounce's tail: 500 x
+// 375, 4 samples, 100K triangles in one wave 5.3 ms, a sample at a time 12.3.
+// Larger waves gain nothing and cost scratch (108 B a path).
+constexpr uint32_t kWavePaths = 1u << 20;
+
+// Device words of a wave. Queue lengths and the caster's work counters are
+// used in turn; shading clears the ones its next bounce needs.
+enum : uint32_t { kCountQueue = 0, kCountWork = 4, kCountWords = 64 };
 
 struct WfBufs {
   rt_ray *rays[2];
   uint32_t *slots[2];
   int2 *hits;
-  int2 *cam_hits;  // bounce-0 hits of the call's first sample, reused by the others
+  int2 *cam_hits;  // of the camera rays, by tile position
   float4 *color;
   uint32_t *rng;
-  uint32_t *counts;  // [0], [1]: queue lengths; [2] listed chunks, [3] wide-caster counter
-  uint32_t *list;    // chunks of the queue left to the 8-wide caster
+  uint32_t *counts;
   void *sort;
 };
 
 size_t a256(size_t x) { return (x + 255) & ~size_t(255); }
 
-WfBufs carve(void *scratch, uint32_t cap) {
+// The image's 8 x 4 tiles: positions 32 t .. 32 t + 31 are tile t's pixels.
+struct Tiles {
+  uint32_t W, H, across, positions;
+};
+Tiles tiles_of(const rt_render_params &p) {
+  const uint32_t across = (p.width + 7) / 8;
+  return Tiles{p.width, p.height, across, across * ((p.height + 3) / 4) * 32};
+}
+__device__ __forceinline__ bool tile_pixel(const Tiles &t, uint32_t pos, uint32_t &x, uint32_t &y) {
+  const uint32_t tile = pos >> 5, at = pos & 31u;
+  x = (tile % t.across) * 8 + (at & 7u);
+  y = (tile / t.across) * 4 + (at >> 3);
+  return x < t.W && y < t.H;
+}
+uint32_t wave_samples(const rt_render_params &p, const Tiles &t) {
+  return std::max(1u, std::min(p.spp, kWavePaths / std::max(t.positions, 1u)));
+}
+
+WfBufs carve(void *scratch, uint32_t cap, uint32_t positions) {
   char *p = static_cast<char *>(scratch);
   WfBufs b;
   for (int i = 0; i < 2; i++) {
@@ -54,15 +86,13 @@ WfBufs carve(void *scratch, uint32_t cap) {
   b.hits = reinterpret_cast<int2 *>(p);
   p += a256(8ull * cap);
   b.cam_hits = reinterpret_cast<int2 *>(p);
-  p += a256(8ull * cap);
+  p += a256(8ull * positions);
   b.color = reinterpret_cast<float4 *>(p);
   p += a256(16ull * cap);
   b.rng = reinterpret_cast<uint32_t *>(p);
   p += a256(4ull * cap);
   b.counts = reinterpret_cast<uint32_t *>(p);
-  p += 256;
-  b.list = reinterpret_cast<uint32_t *>(p);
-  p += a256(4ull * ((cap + 31) / 32));
+  p += a256(4ull * kCountWords);
   b.sort = p;
   return b;
 }
@@ -71,32 +101,43 @@ WfBufs carve(void *scratch, uint32_t cap) {
 // device (batched jobs advanced by a captured graph).
 __device__ __forceinline__ uint32_t sample_of(uint32_t s, const uint32_t *d_s) { return d_s ? *d_s + s : s; }
 
-__global__ void k_wf_raygen(rt_camera cam, uint32_t W, uint32_t H, uint32_t s, const uint32_t *d_s, rt_ray *rays,
-                            uint32_t *slots, float4 *color, uint32_t *rng, uint32_t *count) {
-  s = sample_of(s, d_s);
-  uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p == 0) *count = W * H;
-  if (p >= W * H) return;
-  uint32_t x = p % W, y = p / W;
-  f3 d = normalize3(camera_dir(cam, x, y, W, H));
-  rays[p] = rt_ray{{cam.origin[0], cam.origin[1], cam.origin[2]}, kTmin, {d.x, d.y, d.z}, kTmax};
-  slots[p] = p;
-  color[p] = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
-  rng[p] = (600u * x + y) * (s + 1u);
+// The camera rays, a warp per tile: a packet where the tile's rays suit one
+// (warp_is_coherent), else each lane's own traversal.
+template <int STACK>
+__global__ void __launch_bounds__(kWfBlock, 12) k_wf_camera(DevScene sc, rt_camera cam, Tiles tiles,
+                                                            int2 *__restrict__ hits, uint32_t *err) {
+  __shared__ int s_stack[kWfBlock / 32][STACK];
+  const uint32_t pos = blockIdx.x * kWfBlock + threadIdx.x;
+  if (pos >= tiles.positions) return;  // whole warps
+  uint32_t x, y;
+  const bool active = tile_pixel(tiles, pos, x, y);
+  const f3 o = ld3(cam.origin);
+  const f3 d = active ? normalize3(camera_dir(cam, x, y, tiles.W, tiles.H)) : mk3(1.0f, 0.0f, 0.0f);
+  const TraceRay r = make_ray(o, d, kTmin);
+  float closest = kTmax, u = 0.0f, v = 0.0f;
+  int k;
+  const int oct = warp_octant(active, r);
+  if (warp_is_coherent(active, r)) {
+#define RTGB_CALL(O) k = traverse_packet<STACK, O>(sc, r, active, closest, u, v, s_stack[threadIdx.x >> 5], err)
+    RTGB_OCT_DISPATCH(oct, RTGB_CALL)
+#undef RTGB_CALL
+  } else {
+#define RTGB_CALL(O) k = traverse_spec<STACK, O>(sc, r, active, closest, u, v, err)
+    RTGB_OCT_DISPATCH(oct, RTGB_CALL)
+#undef RTGB_CALL
+  }
+  if (active) hits[pos] = make_int2(k, __float_as_int(closest));
 }
 
-// Closest triangle per queued ray. A warp whose 32 rays are coherent (the
-// camera rays of bounce 0 in pixel order, or any bundle sharing an origin)
-// traverses them as one packet; other warps list their chunk for the 8-wide
-// caster (list != NULL) or run each lane's ray with postponed leaves. All
-// return every ray's own closest hit.
+// Bounce rays where the 8-wide caster is not used: a warp takes 32 queued
+// rays at a time, a packet if they suit one, else each lane its own ray with
+// postponed leaves.
 template <int STACK>
 __global__ void __launch_bounds__(kWfBlock, 12) k_wf_extend(DevScene sc, const float4 *__restrict__ rays,
                                                             uint32_t cap, const uint32_t *count,
                                                             const uint32_t *__restrict__ perm,
                                                             int2 *__restrict__ hits, uint32_t *counter,
-                                                            uint32_t *err, uint32_t *__restrict__ list,
-                                                            uint32_t *__restrict__ list_count) {
+                                                            uint32_t *err) {
   __shared__ int s_stack[kWfBlock / 32][STACK];
   const uint32_t n = min(cap, *count);
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -125,9 +166,6 @@ __global__ void __launch_bounds__(kWfBlock, 12) k_wf_extend(DevScene sc, const f
 #define RTGB_CALL(O) k = traverse_packet<STACK, O>(sc, r, active, closest, u, v, s_stack[warp], err)
       RTGB_OCT_DISPATCH(oct, RTGB_CALL)
 #undef RTGB_CALL
-    } else if (list) {
-      if (lane == 0) list[atomicAdd(list_count, 1u)] = base;
-      continue;
     } else {
 #define RTGB_CALL(O) k = traverse_spec<STACK, O>(sc, r, active, closest, u, v, err)
       RTGB_OCT_DISPATCH(oct, RTGB_CALL)
@@ -137,147 +175,216 @@ __global__ void __launch_bounds__(kWfBlock, 12) k_wf_extend(DevScene sc, const f
   }
 }
 
-__global__ void __launch_bounds__(kWfBlock) k_wf_shade(DevScene sc, uint32_t flags, const rt_ray *__restrict__ rays_in,
-                                                       const uint32_t *__restrict__ slots_in, const uint32_t *count_in,
-                                                       const int2 *__restrict__ hits, float4 *color, uint32_t *rng,
-                                                       rt_ray *rays_out, uint32_t *slots_out, uint32_t *count_out,
-                                                       int last, unsigned long long *segments) {
-  const uint32_t n = *count_in;
-  const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q == 0 && segments) atomicAdd(segments, (unsigned long long)n);
-  bool push = false;
-  HitRec rec;
-  f3 nd;
-  uint32_t s = 0;
-  if (q < n) {
-    PathState ps = path_state(sc, flags);
-    s = slots_in[q];
-    const rt_ray ray = rays_in[q];
-    f3 o = ld3(ray.o), d = ld3(ray.d);
-    int2 h = hits[q];
-    float4 c4 = color[s];
-    f3 c = mk3(c4.x, c4.y, c4.z);
-    if (!resolve_hit(sc, ps, o, d, h.x, __int_as_float(h.y), rec)) {
-      c = mul3(0.0f, c);
-    } else {
-      Rng g{rng[s]};
-      f3 albedo;
-      bool emits = scatter(sc, ps, d, rec, g, albedo, nd);
-      c = mulv3(c, albedo);
-      rng[s] = g.s;
-      push = !emits && !last;
-    }
-    color[s] = make_float4(c.x, c.y, c.z, 0.0f);
+// Appends the block's surviving paths to the queue, with one atomic a block
+// (a warp's own atomic each, on one address, took a third of the shading time).
+__device__ __forceinline__ void push_paths(bool push, const HitRec &rec, f3 nd, uint32_t slot, rt_ray *rays_out,
+                                           uint32_t *slots_out, uint32_t *count_out) {
+  __shared__ uint32_t s_count[kShadeBlock / 32], s_base;
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t mask = __ballot_sync(0xffffffffu, push);
+  if (lane == 0) s_count[warp] = __popc(mask);
+  __syncthreads();
+  if (warp == 0) {
+    const uint32_t c = lane < kShadeBlock / 32 ? s_count[lane] : 0u;
+    const uint32_t total = __reduce_add_sync(0xffffffffu, c);
+    if (lane == 0 && total) s_base = atomicAdd(count_out, total);
   }
-  // Warp-aggregated append of the surviving paths.
-  const uint32_t lane = threadIdx.x & 31;
-  uint32_t mask = __ballot_sync(0xffffffffu, push);
-  if (mask) {
-    uint32_t base = 0;
-    uint32_t leader = __ffs(mask) - 1;
-    if (lane == leader) base = atomicAdd(count_out, (uint32_t)__popc(mask));
-    base = __shfl_sync(0xffffffffu, base, leader);
-    if (push) {
-      uint32_t pos = base + __popc(mask & ((1u << lane) - 1u));
-      rays_out[pos] = rt_ray{{rec.p.x, rec.p.y, rec.p.z}, kTmin, {nd.x, nd.y, nd.z}, kTmax};
-      slots_out[pos] = s;
+  __syncthreads();
+  if (push) {
+    uint32_t pos = s_base + __popc(mask & ((1u << lane) - 1u));
+    for (uint32_t w = 0; w < warp; w++) pos += s_count[w];
+    rays_out[pos] = rt_ray{{rec.p.x, rec.p.y, rec.p.z}, kTmin, {nd.x, nd.y, nd.z}, kTmax};
+    slots_out[pos] = slot;
+  }
+  __syncthreads();  // the shared words are free again
+}
+
+// Shades the first segment of a wave's paths: sample s0 + k of the call at
+// tile position q is path (slot) k * positions + q.
+__global__ void __launch_bounds__(kShadeBlock) k_wf_first(DevScene sc, uint32_t flags, rt_camera cam, Tiles tiles,
+                                                          uint32_t paths, uint32_t s0, const uint32_t *d_s,
+                                                          const int2 *__restrict__ hits, float4 *color, uint32_t *rng,
+                                                          rt_ray *rays_out, uint32_t *slots_out, uint32_t *count_out,
+                                                          int last, unsigned long long *segments) {
+  if (blockIdx.x == 0 && threadIdx.x == 0 && segments)
+    atomicAdd(segments, (unsigned long long)tiles.W * tiles.H);
+  const PathState ps = path_state(sc, flags);
+  for (uint32_t base = blockIdx.x * kShadeBlock; base < paths; base += gridDim.x * kShadeBlock) {
+    const uint32_t slot = base + threadIdx.x;
+    const uint32_t k = slot / tiles.positions, q = slot - k * tiles.positions;
+    uint32_t x, y;
+    bool push = false;
+    HitRec rec;
+    f3 nd;
+    if (slot < paths && tile_pixel(tiles, q, x, y)) {
+      const f3 o = ld3(cam.origin), d = normalize3(camera_dir(cam, x, y, tiles.W, tiles.H));
+      const int2 h = hits[q];
+      f3 c = mk3(1.0f, 1.0f, 1.0f);
+      if (!resolve_hit(sc, ps, o, d, h.x, __int_as_float(h.y), rec)) {
+        c = mul3(0.0f, c);
+      } else {
+        Rng g{(600u * x + y) * (sample_of(s0 + k, d_s) + 1u)};
+        f3 albedo;
+        const bool emits = scatter(sc, ps, d, rec, g, albedo, nd);
+        c = mulv3(c, albedo);
+        rng[slot] = g.s;
+        push = !emits && !last;
+      }
+      color[slot] = make_float4(c.x, c.y, c.z, 0.0f);
     }
+    push_paths(push, rec, nd, slot, rays_out, slots_out, count_out);
   }
 }
 
-__global__ void k_wf_accumulate(uint32_t W, uint32_t H, uint32_t s, const uint32_t *d_s, uint32_t flags,
-                                const float4 *__restrict__ color, float4 *accum) {
-  s = sample_of(s, d_s);
-  uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= W * H) return;
-  float4 c = color[p];
-  float4 acc = accum[p];
-  float sf = (float)s;
-  float keep = gmin(sf, 1.0f);
-  float den = __fadd_rn(sf, 1.0f);
-  acc.x = __fdiv_rn(__fadd_rn(c.x, __fmul_rn(__fmul_rn(acc.x, keep), sf)), den);
-  acc.y = __fdiv_rn(__fadd_rn(c.y, __fmul_rn(__fmul_rn(acc.y, keep), sf)), den);
-  acc.z = __fdiv_rn(__fadd_rn(c.z, __fmul_rn(__fmul_rn(acc.z, keep), sf)), den);
-  acc.w = __fdiv_rn(__fadd_rn(1.0f, __fmul_rn(__fmul_rn(acc.w, keep), sf)), den);
-  if (flags & RT_COMPAT_UNORM8) {
-    acc.x = unorm8(acc.x);
-    acc.y = unorm8(acc.y);
-    acc.z = unorm8(acc.z);
-    acc.w = unorm8(acc.w);
+__global__ void __launch_bounds__(kShadeBlock) k_wf_shade(DevScene sc, uint32_t flags,
+                                                          const rt_ray *__restrict__ rays_in,
+                                                          const uint32_t *__restrict__ slots_in, uint32_t cap,
+                                                          const uint32_t *count_in, const int2 *__restrict__ hits,
+                                                          float4 *color, uint32_t *rng, rt_ray *rays_out,
+                                                          uint32_t *slots_out, uint32_t *count_out,
+                                                          uint32_t *clear_count, uint32_t *clear_work, int last,
+                                                          unsigned long long *segments) {
+  const uint32_t n = min(cap, *count_in);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (segments) atomicAdd(segments, (unsigned long long)n);
+    *clear_count = 0u;
+    *clear_work = 0u;
   }
-  accum[p] = acc;
+  const PathState ps = path_state(sc, flags);
+  for (uint32_t base = blockIdx.x * kShadeBlock; base < n; base += gridDim.x * kShadeBlock) {
+    const uint32_t q = base + threadIdx.x;
+    bool push = false;
+    HitRec rec;
+    f3 nd;
+    uint32_t s = 0;
+    if (q < n) {
+      s = slots_in[q];
+      const rt_ray ray = rays_in[q];
+      f3 o = ld3(ray.o), d = ld3(ray.d);
+      int2 h = hits[q];
+      float4 c4 = color[s];
+      f3 c = mk3(c4.x, c4.y, c4.z);
+      if (!resolve_hit(sc, ps, o, d, h.x, __int_as_float(h.y), rec)) {
+        c = mul3(0.0f, c);
+      } else {
+        Rng g{rng[s]};
+        f3 albedo;
+        bool emits = scatter(sc, ps, d, rec, g, albedo, nd);
+        c = mulv3(c, albedo);
+        rng[s] = g.s;
+        push = !emits && !last;
+      }
+      color[s] = make_float4(c.x, c.y, c.z, 0.0f);
+    }
+    push_paths(push, rec, nd, s, rays_out, slots_out, count_out);
+  }
+}
+
+// The wave's samples into the running mean, in order. `white`: no bounce was
+// asked for, every path's colour is 1.
+__global__ void k_wf_accumulate(Tiles tiles, uint32_t s0, uint32_t samples, const uint32_t *d_s, uint32_t flags,
+                                bool white, const float4 *__restrict__ color, float4 *accum) {
+  const uint32_t pos = blockIdx.x * blockDim.x + threadIdx.x;
+  uint32_t x, y;
+  if (pos >= tiles.positions || !tile_pixel(tiles, pos, x, y)) return;
+  float4 *out = accum + (size_t)y * tiles.W + x;
+  float4 acc = *out;
+  for (uint32_t k = 0; k < samples; k++) {
+    const float4 c = white ? make_float4(1.0f, 1.0f, 1.0f, 0.0f) : color[(size_t)k * tiles.positions + pos];
+    float sf = (float)sample_of(s0 + k, d_s);
+    float keep = gmin(sf, 1.0f);
+    float den = __fadd_rn(sf, 1.0f);
+    acc.x = __fdiv_rn(__fadd_rn(c.x, __fmul_rn(__fmul_rn(acc.x, keep), sf)), den);
+    acc.y = __fdiv_rn(__fadd_rn(c.y, __fmul_rn(__fmul_rn(acc.y, keep), sf)), den);
+    acc.z = __fdiv_rn(__fadd_rn(c.z, __fmul_rn(__fmul_rn(acc.z, keep), sf)), den);
+    acc.w = __fdiv_rn(__fadd_rn(1.0f, __fmul_rn(__fmul_rn(acc.w, keep), sf)), den);
+    if (flags & RT_COMPAT_UNORM8) {
+      acc.x = unorm8(acc.x);
+      acc.y = unorm8(acc.y);
+      acc.z = unorm8(acc.z);
+      acc.w = unorm8(acc.w);
+    }
+  }
+  *out = acc;
 }
 
 int g_sms = 0;
 
 }  // namespace
 
-size_t wavefront_scratch_bytes(uint32_t cap) {
-  return 2 * (a256(sizeof(rt_ray) * (size_t)cap) + a256(4ull * cap)) + 2 * a256(8ull * cap) + a256(16ull * cap) +
-         a256(4ull * cap) + 256 + a256(4ull * ((cap + 31) / 32)) + a256(raysort_scratch_bytes(cap));
+size_t wavefront_scratch_bytes(const rt_render_params &p, bool sort) {
+  const Tiles t = tiles_of(p);
+  const size_t cap = (size_t)t.positions * wave_samples(p, t);
+  return 2 * (a256(sizeof(rt_ray) * cap) + a256(4 * cap)) + a256(8 * cap) + a256(8ull * t.positions) + a256(16 * cap) +
+         a256(4 * cap) + a256(4ull * kCountWords) + (sort ? a256(raysort_scratch_bytes((uint32_t)cap)) : 0);
 }
 
 cudaError_t launch_render_wavefront(const DevScene &sc, const rt_camera &cam, const rt_render_params &p, float *accum,
-                                    unsigned long long *segments, uint32_t *counter, uint32_t *err, void *scratch,
-                                    bool sort, bool wide, cudaStream_t st, const uint32_t *d_sample_index) {
-  const uint32_t W = p.width, H = p.height, cap = W * H;
-  if (cap == 0 || p.spp == 0) return cudaSuccess;
+                                    unsigned long long *segments, uint32_t *err, void *scratch, bool sort, bool wide,
+                                    cudaStream_t st, const uint32_t *d_sample_index) {
+  const Tiles tiles = tiles_of(p);
+  if (p.width == 0 || p.height == 0 || p.spp == 0) return cudaSuccess;
   const bool use_wide = wide && wide_ok(sc);
   if (g_sms == 0) {
     int dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&g_sms, cudaDevAttrMultiProcessorCount, dev);
   }
-  WfBufs b = carve(scratch, cap);
-  const uint32_t grid = (cap + kWfBlock - 1) / kWfBlock;
-  int bps = 0;
-  if (sc.depth <= 32)
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_wf_extend<32>, kWfBlock, 0);
-  else
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_wf_extend<64>, kWfBlock, 0);
-  uint32_t egrid = (uint32_t)(g_sms * (bps > 0 ? bps : 1));
-  if (egrid > grid) egrid = grid;
+  const uint32_t samples = wave_samples(p, tiles), cap = tiles.positions * samples;
+  WfBufs b = carve(scratch, cap, tiles.positions);
+  uint32_t *queue = b.counts + kCountQueue, *work = b.counts + kCountWork;
+  float4 *image = reinterpret_cast<float4 *>(accum);
+  const uint32_t tile_grid = (tiles.positions + kWfBlock - 1) / kWfBlock;
+  const uint32_t shade_grid = std::min((cap + kShadeBlock - 1) / kShadeBlock, (uint32_t)g_sms * 8u);
+  uint32_t extend_grid = 0;
   cudaError_t e = cudaSuccess;
-  for (uint32_t k = 0; k < p.spp; k++) {
-    const uint32_t s = d_sample_index ? k : p.sample_index + k;
-    k_wf_raygen<<<grid, kWfBlock, 0, st>>>(cam, W, H, s, d_sample_index, b.rays[0], b.slots[0], b.color, b.rng,
-                                           b.counts);
-    for (uint32_t bounce = 0; bounce < p.max_bounces; bounce++) {
-      const int in = bounce & 1, out = in ^ 1;
-      if ((e = cudaMemsetAsync(b.counts + out, 0, 4, st)) != cudaSuccess) return e;
-      // Camera rays carry no jitter: bounce 0 is the same for every sample
-      // of the call (queue slot = pixel), so later samples reuse its hits.
-      if (bounce == 0 && k > 0) {
-        k_wf_shade<<<grid, kWfBlock, 0, st>>>(sc, p.flags, b.rays[in], b.slots[in], b.counts + in, b.cam_hits,
-                                              b.color, b.rng, b.rays[out], b.slots[out], b.counts + out,
-                                              bounce + 1 == p.max_bounces, nullptr);
-        continue;
-      }
-      uint32_t *perm = nullptr;
-      if (sort && (e = launch_raysort(b.rays[in], cap, b.counts + in, b.sort, &perm, st)) != cudaSuccess) return e;
-      if ((e = cudaMemsetAsync(counter, 0, 4, st)) != cudaSuccess) return e;
-      const float4 *r4 = reinterpret_cast<const float4 *>(b.rays[in]);
-      uint32_t *list = use_wide ? b.list : nullptr;
-      if (use_wide && (e = cudaMemsetAsync(b.counts + 2, 0, 8, st)) != cudaSuccess) return e;
-      if (sc.depth <= 32)
-        k_wf_extend<32><<<egrid, kWfBlock, 0, st>>>(sc, r4, cap, b.counts + in, perm, b.hits, counter, err, list,
-                                                    b.counts + 2);
-      else
-        k_wf_extend<64><<<egrid, kWfBlock, 0, st>>>(sc, r4, cap, b.counts + in, perm, b.hits, counter, err, list,
-                                                    b.counts + 2);
-      if (use_wide &&
-          (e = launch_wide_leaf(sc, b.rays[in], cap, b.counts + in, perm, b.list, b.counts + 2, b.hits,
-                                b.counts + 3, err, 6, 4, st)) != cudaSuccess)
-        return e;
-      if (bounce == 0 && p.spp > 1 &&
-          (e = cudaMemcpyAsync(b.cam_hits, b.hits, 8ull * cap, cudaMemcpyDeviceToDevice, st)) != cudaSuccess)
-        return e;
-      k_wf_shade<<<grid, kWfBlock, 0, st>>>(sc, p.flags, b.rays[in], b.slots[in], b.counts + in, b.hits, b.color,
-                                            b.rng, b.rays[out], b.slots[out], b.counts + out,
-                                            bounce + 1 == p.max_bounces, segments);
+  if (p.max_bounces > 0) {
+    if (sc.depth <= 32)
+      k_wf_camera<32><<<tile_grid, kWfBlock, 0, st>>>(sc, cam, tiles, b.cam_hits, err);
+    else
+      k_wf_camera<64><<<tile_grid, kWfBlock, 0, st>>>(sc, cam, tiles, b.cam_hits, err);
+  }
+  if (p.max_bounces > 1 && !use_wide) {
+    int bps = 0;
+    if (sc.depth <= 32)
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_wf_extend<32>, kWfBlock, 0);
+    else
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_wf_extend<64>, kWfBlock, 0);
+    extend_grid = std::min((uint32_t)(g_sms * std::max(bps, 1)), (cap + kWfBlock - 1) / kWfBlock);
+  }
+  for (uint32_t k = 0; k < p.spp; k += samples) {
+    const uint32_t s0 = d_sample_index ? k : p.sample_index + k, now = std::min(samples, p.spp - k);
+    if (p.max_bounces > 0) {
+      if ((e = cudaMemsetAsync(b.counts, 0, 4 * kCountWords, st)) != cudaSuccess) return e;
+      // The camera segments count once a call.
+      k_wf_first<<<shade_grid, kShadeBlock, 0, st>>>(sc, p.flags, cam, tiles, tiles.positions * now, s0,
+                                                     d_sample_index, b.cam_hits, b.color, b.rng, b.rays[1],
+                                                     b.slots[1], queue + 1, p.max_bounces == 1,
+                                                     k == 0 ? segments : nullptr);
     }
-    k_wf_accumulate<<<grid, kWfBlock, 0, st>>>(W, H, s, d_sample_index, p.flags, b.color,
-                                               reinterpret_cast<float4 *>(accum));
+    for (uint32_t bounce = 1; bounce < p.max_bounces; bounce++) {
+      const int in = bounce & 1, out = in ^ 1;
+      const uint32_t *count = queue + bounce % 3;
+      uint32_t *perm = nullptr;
+      if (sort && (e = launch_raysort(b.rays[in], cap, count, b.sort, &perm, st)) != cudaSuccess) return e;
+      if (use_wide) {
+        if ((e = launch_wide_leaf(sc, b.rays[in], cap, count, perm, nullptr, nullptr, b.hits, work + (bounce & 1),
+                                  err, 6, 4, st)) != cudaSuccess)
+          return e;
+      } else if (sc.depth <= 32) {
+        k_wf_extend<32><<<extend_grid, kWfBlock, 0, st>>>(sc, reinterpret_cast<const float4 *>(b.rays[in]), cap,
+                                                          count, perm, b.hits, work + (bounce & 1), err);
+      } else {
+        k_wf_extend<64><<<extend_grid, kWfBlock, 0, st>>>(sc, reinterpret_cast<const float4 *>(b.rays[in]), cap,
+                                                          count, perm, b.hits, work + (bounce & 1), err);
+      }
+      k_wf_shade<<<shade_grid, kShadeBlock, 0, st>>>(
+          sc, p.flags, b.rays[in], b.slots[in], cap, count, b.hits, b.color, b.rng, b.rays[out], b.slots[out],
+          queue + (bounce + 1) % 3, queue + (bounce + 2) % 3, work + ((bounce + 1) & 1), bounce + 1 == p.max_bounces,
+          segments);
+    }
+    k_wf_accumulate<<<tile_grid, kWfBlock, 0, st>>>(tiles, s0, now, d_sample_index, p.flags, p.max_bounces == 0,
+                                                    b.color, image);
   }
   return cudaGetLastError();
 }
