@@ -25,13 +25,11 @@ template <int STACK>
 __global__ void __launch_bounds__(kTileX *kTileY) k_render(DevScene sc, rt_camera cam, rt_render_params p,
                                                            float4 *accum, unsigned long long *segments,
                                                            uint32_t *err) {
-  __shared__ int s_stack[kTileX * kTileY / 32][STACK];
-  const uint32_t warp = (threadIdx.y * kTileX + threadIdx.x) >> 5;
   uint32_t x = blockIdx.x * kTileX + threadIdx.x;
   uint32_t y = blockIdx.y * kTileY + threadIdx.y;
   const bool active = x < p.width && y < p.height;
   PathState ps = path_state(sc, p.flags);
-  uint32_t seg = render_pixel<STACK>(sc, ps, cam, p, x, y, active, accum, err, s_stack[warp]);
+  uint32_t seg = render_pixel<STACK>(sc, ps, cam, p, x, y, active, accum, err);
   count_segments(seg, segments);
 }
 
@@ -45,8 +43,6 @@ __global__ void __launch_bounds__(kTileX *kTileY) k_render_batch(const BatchJob 
                                                                  uint32_t total_tiles, uint32_t *counter,
                                                                  unsigned long long *segments, uint32_t *err) {
   __shared__ uint32_t s_tile;
-  __shared__ int s_stack[kTileX * kTileY / 32][STACK];
-  const uint32_t warp = (threadIdx.y * kTileX + threadIdx.x) >> 5;
   const bool leader = threadIdx.x == 0 && threadIdx.y == 0;
   for (;;) {
     if (leader) s_tile = atomicAdd(counter, 1u);
@@ -68,7 +64,7 @@ __global__ void __launch_bounds__(kTileX *kTileY) k_render_batch(const BatchJob 
     const bool active = x < p.width && y < p.height;
     PathState ps = path_state(sc, p.flags);
     uint32_t seg =
-        render_pixel<STACK>(sc, ps, J.cam, p, x, y, active, reinterpret_cast<float4 *>(J.accum), err, s_stack[warp]);
+        render_pixel<STACK>(sc, ps, J.cam, p, x, y, active, reinterpret_cast<float4 *>(J.accum), err);
     count_segments(seg, segments);
   }
 }

@@ -306,14 +306,14 @@ __device__ __forceinline__ f3 ray_color(const DevScene &sc, const PathState &ps,
 // traversal, which stays per sample as in the shader.
 template <int STACK>
 __device__ __forceinline__ int camera_hit(const DevScene &sc, const PathState &ps, f3 o, f3 d, bool active,
-                                          float &t, uint32_t *err, volatile int *s_stack) {
+                                          float &t, uint32_t *err) {
   if (ps.flags & RT_COMPAT_STACK16) return kTraceFirst;
   TraceRay r = make_ray(o, d, kTmin);
   float closest = kTmax, u = 0.0f, v = 0.0f;
   int k;
   const int oct = warp_octant(active, r);
   if (warp_is_coherent(active, r)) {
-#define RTGB_CALL(O) k = traverse_packet<STACK, O>(sc, r, active, closest, u, v, s_stack, err)
+#define RTGB_CALL(O) k = traverse_packet<STACK, O>(sc, r, active, closest, u, v, err)
     RTGB_OCT_DISPATCH(oct, RTGB_CALL)
 #undef RTGB_CALL
   } else {
@@ -347,14 +347,14 @@ __device__ __forceinline__ float unorm8(float x) {
 template <int STACK>
 __device__ __forceinline__ uint32_t render_pixel(const DevScene &sc, const PathState &ps, const rt_camera &cam,
                                                  const rt_render_params &p, uint32_t x, uint32_t y, bool active,
-                                                 float4 *accum, uint32_t *err, volatile int *s_stack) {
+                                                 float4 *accum, uint32_t *err) {
   f3 org = ld3(cam.origin);
   f3 d0 = active ? normalize3(camera_dir(cam, x, y, p.width, p.height)) : mk3(1.0f, 0.0f, 0.0f);
   int k0 = kTraceFirst;
   float t0 = 0.0f;
   uint32_t segments = 0;
   if (p.max_bounces > 0 && p.spp > 0) {  // uniform across the warp (one job per tile)
-    k0 = camera_hit<STACK>(sc, ps, org, d0, active, t0, err, s_stack);
+    k0 = camera_hit<STACK>(sc, ps, org, d0, active, t0, err);
     if (k0 != kTraceFirst && active) segments = 1;
   }
   if (!active) return 0;

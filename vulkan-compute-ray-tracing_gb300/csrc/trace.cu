@@ -202,7 +202,7 @@ template <int STACK>
 __device__ __forceinline__ void cast_chunk(const DevScene &sc, const float4 *__restrict__ rays, uint32_t n,
                                            int4 *__restrict__ hits, uint32_t *err, const uint32_t *__restrict__ perm,
                                            uint32_t *__restrict__ list, uint32_t *__restrict__ list_count,
-                                           bool refine, uint32_t base, uint32_t lane, int *s_stack) {
+                                           bool refine, uint32_t base, uint32_t lane) {
   uint32_t i = base + lane;
   const bool active = i < n;
   f3 o = mk3(0.0f, 0.0f, 0.0f), d = mk3(1.0f, 0.0f, 0.0f);
@@ -216,7 +216,7 @@ __device__ __forceinline__ void cast_chunk(const DevScene &sc, const float4 *__r
   int k;
   if (warp_is_coherent(active, r)) {
     const int oct = warp_octant(active, r);
-#define RTGB_CALL(O) k = traverse_packet<STACK, O>(sc, r, active, closest, u, v, s_stack, err)
+#define RTGB_CALL(O) k = traverse_packet<STACK, O>(sc, r, active, closest, u, v, err)
     RTGB_OCT_DISPATCH(oct, RTGB_CALL)
 #undef RTGB_CALL
   } else if (list) {
@@ -239,15 +239,13 @@ __global__ void __maxnreg__(regs_for<MINB>()) k_trace_packets(DevScene sc, const
                                                                    const uint32_t *__restrict__ perm,
                                                                    uint32_t *__restrict__ list,
                                                                    uint32_t *__restrict__ list_count, bool refine) {
-  extern __shared__ int s_dyn_stack[];  // STACK entries per warp
-  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int *const s_stack = s_dyn_stack + warp * STACK;
+  const uint32_t lane = threadIdx.x & 31;
   for (;;) {
     uint32_t base = 0;
     if (lane == 0) base = atomicAdd(counter, 32u);
     base = __shfl_sync(0xffffffffu, base, 0);
     if (base >= n) return;
-    cast_chunk<STACK>(sc, rays, n, hits, err, perm, list, list_count, refine, base, lane, s_stack);
+    cast_chunk<STACK>(sc, rays, n, hits, err, perm, list, list_count, refine, base, lane);
   }
 }
 
@@ -310,9 +308,7 @@ __global__ void __launch_bounds__(kBeamRays, MINB)
                   const uint32_t *__restrict__ cell_tiles, const uint32_t *__restrict__ cell_count,
                   const uint32_t *__restrict__ ext, int round_leaves, bool refine) {
   __shared__ BeamShared s;
-  extern __shared__ int s_dyn_stack[];  // STACK entries per warp (packet casts)
   const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  int *const s_stack = s_dyn_stack + warp * STACK;
   const float INF = __int_as_float(0x7f800000);
   const bool one_origin = __ldg(ext + 0) == __ldg(ext + 5) && __ldg(ext + 1) == __ldg(ext + 6) &&
                           __ldg(ext + 2) == __ldg(ext + 7);
@@ -322,7 +318,7 @@ __global__ void __launch_bounds__(kBeamRays, MINB)
       if (lane == 0) base = atomicAdd(counter, 32u);
       base = __shfl_sync(0xffffffffu, base, 0);
       if (base >= n) return;
-      cast_chunk<STACK>(sc, rays, n, hits, err, perm, list, list_count, refine, base, lane, s_stack);
+      cast_chunk<STACK>(sc, rays, n, hits, err, perm, list, list_count, refine, base, lane);
     }
   }
   const uint32_t ntiles = __ldg(cell_count);
@@ -471,7 +467,7 @@ __global__ void __launch_bounds__(kBeamRays, MINB)
     int k;
     if (warp_is_coherent(active, r)) {
       const int oct = warp_octant(active, r);
-#define RTGB_CALL(O) k = traverse_packet<STACK, O>(sc, r, active, closest, bu, bv, s_stack, err)
+#define RTGB_CALL(O) k = traverse_packet<STACK, O>(sc, r, active, closest, bu, bv, err)
       RTGB_OCT_DISPATCH(oct, RTGB_CALL)
 #undef RTGB_CALL
     } else {
@@ -853,8 +849,8 @@ cudaError_t launch_wide(const DevScene &sc, const float4 *rays, uint32_t n, int4
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
   }
-  kern<<<persistent_grid(kern, n, block, smem), block, smem, st>>>(sc, rays, n, nullptr, hits, counter, err, perm,
-                                                                   list, list_count, refill, refine);
+  kern<<<persistent_grid(kern, n, block, smem), block, smem, st>>>(
+      sc, rays, n, nullptr, hits, counter, err, perm, list, list_count, refill, refine);
   return cudaGetLastError();
 }
 
@@ -891,17 +887,15 @@ cudaError_t launch_variant(const DevScene &sc, const rt_ray *rays, uint32_t n, r
       uint32_t *plist = opts.defer ? chunk_scratch + 64 : nullptr;
       if ((opts.beam == 1 || (opts.beam == 2 && sc.median_tree)) && cells && perm) {
         auto bk = k_trace_beams<STACK, 4>;
-        const size_t smem = (size_t)(kBeamRays / 32) * STACK * sizeof(int);
-        bk<<<persistent_grid(bk, n, kBeamRays, smem), kBeamRays, smem, st>>>(
+        bk<<<persistent_grid(bk, n, kBeamRays), kBeamRays, 0, st>>>(
             sc, r4, n, h4, counter, err, perm, plist, chunk_scratch, cells->tiles, cells->count, cells->ext,
             opts.beam_round, refine);
       } else {
         auto pk = opts.packet_minblocks >= 16   ? k_trace_packets<STACK, 16>
                   : opts.packet_minblocks >= 12 ? k_trace_packets<STACK, 12>
                                                 : k_trace_packets<STACK, 10>;
-        const size_t smem = (size_t)(block / 32) * STACK * sizeof(int);
-        pk<<<persistent_grid(pk, n, block, smem), block, smem, st>>>(sc, r4, n, h4, counter, err, perm, plist,
-                                                                     chunk_scratch, refine);
+        pk<<<persistent_grid(pk, n, block), block, 0, st>>>(sc, r4, n, h4, counter, err, perm, plist, chunk_scratch,
+                                                            refine);
       }
       if (!opts.defer) return cudaGetLastError();
       list = chunk_scratch + 64;
@@ -944,9 +938,8 @@ cudaError_t launch_wide_leaf(const DevScene &sc, const rt_ray *rays, uint32_t ca
   // minblocks 8: one node step per iteration (64 registers); otherwise three.
   auto go = [&](auto kern, size_t warp_smem) {
     const size_t smem = (size_t)(kTraceBlock / 32) * warp_smem;
-    kern<<<persistent_grid(kern, cap, kTraceBlock, smem), kTraceBlock, smem, st>>>(sc, r4, cap, d_n, hits, counter,
-                                                                                   err, perm, list, list_count,
-                                                                                   refill, false);
+    kern<<<persistent_grid(kern, cap, kTraceBlock, smem), kTraceBlock, smem, st>>>(
+        sc, r4, cap, d_n, hits, counter, err, perm, list, list_count, refill, false);
     return cudaGetLastError();
   };
   const bool narrow = minblocks >= 8;

@@ -35,8 +35,8 @@ constexpr int kWfBlock = 128, kShadeBlock = 256;
 
 // Paths of one wave: samples of a call are added until this many run
 // together. A wave of fewer leaves the GPU idle in every bounce's tail: 500 x
-// 375, 4 samples, 100K triangles in one wave 5.3 ms, a sample at a time 12.3.
-// Larger waves gain nothing and cost scratch (108 B a path).
+// 375, 4 samples, 100K triangles in one wave 6.1 ms, in the megakernel 12.3;
+// larger waves cost scratch (108 B a path).
 constexpr uint32_t kWavePaths = 1u << 20;
 
 // Device words of a wave. Queue lengths and the caster's work counters are
@@ -106,7 +106,6 @@ __device__ __forceinline__ uint32_t sample_of(uint32_t s, const uint32_t *d_s) {
 template <int STACK>
 __global__ void __launch_bounds__(kWfBlock, 12) k_wf_camera(DevScene sc, rt_camera cam, Tiles tiles,
                                                             int2 *__restrict__ hits, uint32_t *err) {
-  __shared__ int s_stack[kWfBlock / 32][STACK];
   const uint32_t pos = blockIdx.x * kWfBlock + threadIdx.x;
   if (pos >= tiles.positions) return;  // whole warps
   uint32_t x, y;
@@ -118,7 +117,7 @@ __global__ void __launch_bounds__(kWfBlock, 12) k_wf_camera(DevScene sc, rt_came
   int k;
   const int oct = warp_octant(active, r);
   if (warp_is_coherent(active, r)) {
-#define RTGB_CALL(O) k = traverse_packet<STACK, O>(sc, r, active, closest, u, v, s_stack[threadIdx.x >> 5], err)
+#define RTGB_CALL(O) k = traverse_packet<STACK, O>(sc, r, active, closest, u, v, err)
     RTGB_OCT_DISPATCH(oct, RTGB_CALL)
 #undef RTGB_CALL
   } else {
@@ -138,9 +137,8 @@ __global__ void __launch_bounds__(kWfBlock, 12) k_wf_extend(DevScene sc, const f
                                                             const uint32_t *__restrict__ perm,
                                                             int2 *__restrict__ hits, uint32_t *counter,
                                                             uint32_t *err) {
-  __shared__ int s_stack[kWfBlock / 32][STACK];
   const uint32_t n = min(cap, *count);
-  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t lane = threadIdx.x & 31;
   for (;;) {
     uint32_t base = 0;
     if (lane == 0) base = atomicAdd(counter, 32u);
@@ -163,7 +161,7 @@ __global__ void __launch_bounds__(kWfBlock, 12) k_wf_extend(DevScene sc, const f
     int k;
     const int oct = warp_octant(active, r);
     if (warp_is_coherent(active, r)) {
-#define RTGB_CALL(O) k = traverse_packet<STACK, O>(sc, r, active, closest, u, v, s_stack[warp], err)
+#define RTGB_CALL(O) k = traverse_packet<STACK, O>(sc, r, active, closest, u, v, err)
       RTGB_OCT_DISPATCH(oct, RTGB_CALL)
 #undef RTGB_CALL
     } else {
