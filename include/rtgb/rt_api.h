@@ -169,7 +169,14 @@ rt_status rtTraceClosestHost(rt_ctx *ctx, rt_scene_id scene, const rt_ray *h_ray
  *   "trace.sort"    1 (default) = cast batches of >= 65536 rays in Morton
  *                   order of origin and direction (hits still land at their
  *                   ray's input index; scratch comes from the stream-ordered
- *                   pool)
+ *                   pool), except those that trace.packet_min_rays leaves as
+ *                   they are
+ *   "trace.packet_min_rays"  batches below this many rays (default 2^20)
+ *                   go to the 8-wide caster in input order, without the sort
+ *                   or the packet pass; so do larger ones whose rays mostly
+ *                   have origins of their own. Only while trace.wide,
+ *                   trace.packet and trace.defer are 1, trace.refill is 32 and
+ *                   no beams are asked for. Results are identical either way
  *   "trace.packet"  1 (default) = a warp whose 32 rays share an origin and
  *                   point within ~18 degrees traverses them as one packet
  *                   (one node sequence, every lane busy); 0 = always one

@@ -27,7 +27,8 @@ __global__ void k_flags(const rt_bvh_node *nodes, uint32_t n, uint32_t *flag) {
 }
 
 // Block-local exclusive scan; writes the block total to sums[blockIdx.x].
-__global__ void k_scan_local(const uint32_t *in, uint32_t *out, uint32_t *sums, uint32_t n) {
+__global__ void k_scan_local(const uint32_t *in, uint32_t *out, uint32_t *sums, uint32_t n, const uint32_t *gate) {
+  if (gate && !*gate) return;
   __shared__ uint32_t warp_tot[32];
   uint32_t i = blockIdx.x * kScanBlock + threadIdx.x;
   uint32_t v = i < n ? in[i] : 0u;
@@ -56,7 +57,8 @@ __global__ void k_scan_local(const uint32_t *in, uint32_t *out, uint32_t *sums, 
 }
 
 // Exclusive scan of the block totals in place (one block, serial over chunks).
-__global__ void k_scan_sums(uint32_t *sums, uint32_t nb) {
+__global__ void k_scan_sums(uint32_t *sums, uint32_t nb, const uint32_t *gate) {
+  if (gate && !*gate) return;
   __shared__ uint32_t warp_tot[32];
   __shared__ uint32_t carry;
   if (threadIdx.x == 0) carry = 0;
@@ -92,7 +94,8 @@ __global__ void k_scan_sums(uint32_t *sums, uint32_t nb) {
   }
 }
 
-__global__ void k_scan_add(uint32_t *out, const uint32_t *sums, uint32_t n) {
+__global__ void k_scan_add(uint32_t *out, const uint32_t *sums, uint32_t n, const uint32_t *gate) {
+  if (gate && !*gate) return;
   uint32_t i = blockIdx.x * kScanBlock + threadIdx.x;
   if (i < n) out[i] += sums[blockIdx.x];
 }
@@ -151,13 +154,14 @@ __global__ void k_emit(const rt_bvh_node *nodes, uint32_t n, const rt_triangle *
 }  // namespace
 
 // Exclusive scan of n uint32 values (in may equal out). `sums` needs
-// ceil(n / 1024) words.
-cudaError_t exclusive_scan_u32(const uint32_t *in, uint32_t *out, uint32_t *sums, uint32_t n, cudaStream_t st) {
+// ceil(n / 1024) words. With a `gate`, nothing is done when *gate is 0.
+cudaError_t exclusive_scan_u32(const uint32_t *in, uint32_t *out, uint32_t *sums, uint32_t n, cudaStream_t st,
+                               const uint32_t *gate) {
   if (n == 0) return cudaSuccess;
   uint32_t nb = (n + kScanBlock - 1) / kScanBlock;
-  k_scan_local<<<nb, kScanBlock, 0, st>>>(in, out, sums, n);
-  k_scan_sums<<<1, kScanBlock, 0, st>>>(sums, nb);
-  k_scan_add<<<nb, kScanBlock, 0, st>>>(out, sums, n);
+  k_scan_local<<<nb, kScanBlock, 0, st>>>(in, out, sums, n, gate);
+  k_scan_sums<<<1, kScanBlock, 0, st>>>(sums, nb, gate);
+  k_scan_add<<<nb, kScanBlock, 0, st>>>(out, sums, n, gate);
   return cudaGetLastError();
 }
 

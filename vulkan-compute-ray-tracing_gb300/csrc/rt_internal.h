@@ -75,7 +75,9 @@ cudaError_t build_bvh8(const DevScene &d, bool sah, void *bvh8q, uint32_t cap, u
 
 // ---------------------------------------------------------------- relayout.cu
 // Exclusive scan of n words (in may equal out); `sums` needs ceil(n/1024).
-cudaError_t exclusive_scan_u32(const uint32_t *in, uint32_t *out, uint32_t *sums, uint32_t n, cudaStream_t st);
+// With a `gate`, nothing is done when *gate is 0.
+cudaError_t exclusive_scan_u32(const uint32_t *in, uint32_t *out, uint32_t *sums, uint32_t n, cudaStream_t st,
+                               const uint32_t *gate = nullptr);
 // Derives bvh2 / tpre / leaf_tri from the reference node array. `scratch`
 // holds 2*nnodes uint32 words.
 cudaError_t launch_relayout(const rt_bvh_node *nodes, uint32_t nnodes, const rt_triangle *tris, float4 *bvh2,
@@ -87,6 +89,12 @@ struct TraceOpts {
   int refill = 32;  // idle lanes per warp that trigger a fetch of new rays (32: whole-warp batches)
   int sort = 1;     // 1: cast rays in Morton order of origin and direction (raysort.cu)
   int packet = 1;   // 1: warps of coherent rays traverse as one packet (traverse_packet)
+  // Smaller batches go straight to the 8-wide caster, in input order: neither
+  // the sort nor the packets pay there. Sorted packets / direct, us: 2^18
+  // camera rays into 20K, 328K, 1.31M triangles 161 / 120, 625 / 315, 1423 /
+  // 812; 2^20 271 / 340, 765 / 864, 1815 / 1899; 2^18 random rays 173 / 108,
+  // 355 / 286, 755 / 658.
+  uint32_t packet_min_rays = 1u << 20;
   int beam = 0;     // sorted one-origin batches traverse the sort's cell tiles as beams (beam.cuh):
                     // 1 always, 0 never, 2 on Bvh.h's median-split trees (DevScene::median_tree)
   int beam_round = 64;  // leaves a beam round collects before its rays test them (16..256)
@@ -112,6 +120,10 @@ inline int trace_stack_entries(const TraceOpts &o, const DevScene &sc) {
   return o.stack > need ? (o.stack <= 32 ? 32 : 64) : need;
 }
 
+// True when a batch of n rays goes to the 8-wide caster as it is.
+inline bool beam_cast(const TraceOpts &o, const DevScene &sc) { return o.beam == 1 || (o.beam == 2 && sc.median_tree); }
+inline bool cast_direct(const TraceOpts &o, const DevScene &sc, uint32_t n);
+
 // `counter` is a device word private to this launch (work distribution);
 // `refine` recomputes t, u, v of the winning triangle in fp64.
 // `perm` (may be NULL) gives the order rays are cast in; hits always land
@@ -120,11 +132,13 @@ inline int trace_stack_entries(const TraceOpts &o, const DevScene &sc) {
 // chunks left for the per-lane pass); without it packets are not used.
 // `cells` (with perm, from the same sort) lets one-origin batches be cast
 // as beams over the sort's cell tiles (trace.beam).
+// With a `gate` (launch_raysort) of 0 on the device, perm and the packet pass
+// are skipped and every ray goes to the 8-wide caster.
 struct RayCells;
 cudaError_t launch_trace(const DevScene &sc, const rt_ray *rays, uint32_t n, rt_hit *hits, uint32_t *counter,
                          uint32_t *err, bool refine, const TraceOpts &opts, cudaStream_t st,
                          const uint32_t *perm = nullptr, uint32_t *chunk_scratch = nullptr,
-                         const RayCells *cells = nullptr);
+                         const RayCells *cells = nullptr, const uint32_t *gate = nullptr);
 size_t trace_chunk_scratch_bytes(uint32_t n);
 // The 8-wide caster over listed 32-ray chunks of a device-sized queue
 // (*d_n rays, at most cap), writing (leaf k, t) hits; wide_ok tells whether
@@ -132,6 +146,14 @@ size_t trace_chunk_scratch_bytes(uint32_t n);
 bool wide_ok(const DevScene &sc);
 inline bool use_wide(const TraceOpts &o, const DevScene &sc) {
   return o.wide && sc.ntris >= o.wide_min_tris && wide_ok(sc);
+}
+inline bool cast_direct(const TraceOpts &o, const DevScene &sc, uint32_t n) {
+  return o.refill >= 32 && o.packet && o.defer && !beam_cast(o, sc) && use_wide(o, sc) && n < o.packet_min_rays;
+}
+// True when a sorted batch's order and packets are worth having only if its
+// rays share origins (gate_out of launch_raysort): the rest are cast directly.
+inline bool cast_gated(const TraceOpts &o, const DevScene &sc) {
+  return o.refill >= 32 && o.packet && o.defer && !beam_cast(o, sc) && use_wide(o, sc);
 }
 cudaError_t launch_wide_leaf(const DevScene &sc, const rt_ray *rays, uint32_t cap, const uint32_t *d_n,
                              const uint32_t *perm, const uint32_t *list, const uint32_t *list_count, int2 *hits,
@@ -151,9 +173,11 @@ struct RayCells {
   const uint32_t *count = nullptr;
 };
 // With d_n != NULL only the first *d_n of the n rays are sorted. With
-// `cells`, the cell tiles are listed too (not with d_n).
+// `cells`, the cell tiles are listed too (not with d_n). With `gate_out`, the
+// device word it returns is 1 when most sampled rays share their origin with
+// one of the next two, and at 0 nothing is sorted.
 cudaError_t launch_raysort(const rt_ray *rays, uint32_t n, const uint32_t *d_n, void *scratch, uint32_t **perm_out,
-                           cudaStream_t st, RayCells *cells = nullptr);
+                           cudaStream_t st, RayCells *cells = nullptr, const uint32_t **gate_out = nullptr);
 // The shader-literal 16-entry-stack traversal over the Bvh.h node array.
 cudaError_t launch_trace_literal16(const DevScene &sc, const rt_ray *rays, uint32_t n, rt_hit *hits,
                                    cudaStream_t st);

@@ -238,7 +238,9 @@ __global__ void __maxnreg__(regs_for<MINB>()) k_trace_packets(DevScene sc, const
                                                                    uint32_t *__restrict__ counter, uint32_t *err,
                                                                    const uint32_t *__restrict__ perm,
                                                                    uint32_t *__restrict__ list,
-                                                                   uint32_t *__restrict__ list_count, bool refine) {
+                                                                   uint32_t *__restrict__ list_count,
+                                                                   const uint32_t *gate, bool refine) {
+  if (gate && !*gate) return;
   const uint32_t lane = threadIdx.x & 31;
   for (;;) {
     uint32_t base = 0;
@@ -559,7 +561,8 @@ __global__ void __maxnreg__(regs_for<MINB>()) k_trace_wide(DevScene sc, const fl
                                                                const uint32_t *__restrict__ perm,
                                                                const uint32_t *__restrict__ list,
                                                                const uint32_t *__restrict__ list_count,
-                                                               int refill, bool refine) {
+                                                               const uint32_t *gate, int refill, bool refine) {
+  if (gate && !*gate) list = perm = nullptr;  // the whole batch, as it is
   // Per warp (wide_warp_smem bytes, dynamic): the lanes' rays (32 x 2
   // float4), closest-hit keys (32 x u64), winning t/u/v/leaf (32 x float4),
   // the leaf pool (kPool x u32), the ring of finished rays waiting for
@@ -830,7 +833,8 @@ cudaError_t launch_lanes(const DevScene &sc, const float4 *rays, uint32_t n, int
 template <int GSTACK>
 cudaError_t launch_wide(const DevScene &sc, const float4 *rays, uint32_t n, int4 *hits, uint32_t *counter,
                         uint32_t *err, const uint32_t *perm, const uint32_t *list, const uint32_t *list_count,
-                        int minblocks, int refill, int block, int visits, bool refine, cudaStream_t st) {
+                        const uint32_t *gate, int minblocks, int refill, int block, int visits, bool refine,
+                        cudaStream_t st) {
   auto kern = visits >= 3 ? (minblocks >= 8   ? k_trace_wide<GSTACK, 8, false, 3>
                             : minblocks >= 7 ? k_trace_wide<GSTACK, 7, false, 3>
                             : minblocks >= 6 ? k_trace_wide<GSTACK, 6, false, 3>
@@ -850,30 +854,30 @@ cudaError_t launch_wide(const DevScene &sc, const float4 *rays, uint32_t n, int4
     if (e != cudaSuccess) return e;
   }
   kern<<<persistent_grid(kern, n, block, smem), block, smem, st>>>(
-      sc, rays, n, nullptr, hits, counter, err, perm, list, list_count, refill, refine);
+      sc, rays, n, nullptr, hits, counter, err, perm, list, list_count, gate, refill, refine);
   return cudaGetLastError();
 }
 
 // Group stack of the 8-wide caster: one entry per bvh8 level at most.
 cudaError_t launch_wide_any(const DevScene &sc, const float4 *rays, uint32_t n, int4 *hits, uint32_t *counter,
                             uint32_t *err, const uint32_t *perm, const uint32_t *list, const uint32_t *list_count,
-                            const TraceOpts &opts, bool refine, cudaStream_t st) {
+                            const uint32_t *gate, const TraceOpts &opts, bool refine, cudaStream_t st) {
   const int want = std::max<int>(opts.stack, (int)sc.levels8);
   const int block = cast_block(opts.block);
   if (want <= 16)
-    return launch_wide<16>(sc, rays, n, hits, counter, err, perm, list, list_count, opts.wide_minblocks,
+    return launch_wide<16>(sc, rays, n, hits, counter, err, perm, list, list_count, gate, opts.wide_minblocks,
                                    opts.wide_refill, block, opts.wide_visits, refine, st);
   if (want <= 32)
-    return launch_wide<32>(sc, rays, n, hits, counter, err, perm, list, list_count, opts.wide_minblocks,
+    return launch_wide<32>(sc, rays, n, hits, counter, err, perm, list, list_count, gate, opts.wide_minblocks,
                                    opts.wide_refill, block, opts.wide_visits, refine, st);
-  return launch_wide<64>(sc, rays, n, hits, counter, err, perm, list, list_count, opts.wide_minblocks,
+  return launch_wide<64>(sc, rays, n, hits, counter, err, perm, list, list_count, gate, opts.wide_minblocks,
                                  opts.wide_refill, block, opts.wide_visits, refine, st);
 }
 
 template <int STACK>
 cudaError_t launch_variant(const DevScene &sc, const rt_ray *rays, uint32_t n, rt_hit *hits, uint32_t *counter,
                            uint32_t *err, const TraceOpts &opts, const uint32_t *perm, uint32_t *chunk_scratch,
-                           const RayCells *cells, bool refine, cudaStream_t st) {
+                           const RayCells *cells, const uint32_t *gate, bool refine, cudaStream_t st) {
   const float4 *r4 = reinterpret_cast<const float4 *>(rays);
   int4 *h4 = reinterpret_cast<int4 *>(hits);
   if (opts.refill >= 32) {
@@ -885,7 +889,7 @@ cudaError_t launch_variant(const DevScene &sc, const rt_ray *rays, uint32_t n, r
       cudaError_t e = cudaMemsetAsync(chunk_scratch, 0, 256, st);
       if (e != cudaSuccess) return e;
       uint32_t *plist = opts.defer ? chunk_scratch + 64 : nullptr;
-      if ((opts.beam == 1 || (opts.beam == 2 && sc.median_tree)) && cells && perm) {
+      if (beam_cast(opts, sc) && cells && perm) {
         auto bk = k_trace_beams<STACK, 4>;
         bk<<<persistent_grid(bk, n, kBeamRays), kBeamRays, 0, st>>>(
             sc, r4, n, h4, counter, err, perm, plist, chunk_scratch, cells->tiles, cells->count, cells->ext,
@@ -895,7 +899,7 @@ cudaError_t launch_variant(const DevScene &sc, const rt_ray *rays, uint32_t n, r
                   : opts.packet_minblocks >= 12 ? k_trace_packets<STACK, 12>
                                                 : k_trace_packets<STACK, 10>;
         pk<<<persistent_grid(pk, n, block), block, 0, st>>>(sc, r4, n, h4, counter, err, perm, plist, chunk_scratch,
-                                                            refine);
+                                                            gate, refine);
       }
       if (!opts.defer) return cudaGetLastError();
       list = chunk_scratch + 64;
@@ -903,7 +907,7 @@ cudaError_t launch_variant(const DevScene &sc, const rt_ray *rays, uint32_t n, r
       lane_counter = chunk_scratch + 1;
     }
     if (use_wide(opts, sc))
-      return launch_wide_any(sc, r4, n, h4, lane_counter, err, perm, list, list_count, opts, refine, st);
+      return launch_wide_any(sc, r4, n, h4, lane_counter, err, perm, list, list_count, gate, opts, refine, st);
     if (opts.minblocks >= 16)
       return launch_lanes<STACK, 16>(sc, r4, n, h4, lane_counter, err, perm, list, list_count, opts.spec,
                                              block, refine, st);
@@ -939,7 +943,7 @@ cudaError_t launch_wide_leaf(const DevScene &sc, const rt_ray *rays, uint32_t ca
   auto go = [&](auto kern, size_t warp_smem) {
     const size_t smem = (size_t)(kTraceBlock / 32) * warp_smem;
     kern<<<persistent_grid(kern, cap, kTraceBlock, smem), kTraceBlock, smem, st>>>(
-        sc, r4, cap, d_n, hits, counter, err, perm, list, list_count, refill, false);
+        sc, r4, cap, d_n, hits, counter, err, perm, list, list_count, nullptr, refill, false);
     return cudaGetLastError();
   };
   const bool narrow = minblocks >= 8;
@@ -955,7 +959,7 @@ size_t trace_chunk_scratch_bytes(uint32_t n) { return 4ull * (64 + (n + 31) / 32
 
 cudaError_t launch_trace(const DevScene &sc, const rt_ray *rays, uint32_t n, rt_hit *hits, uint32_t *counter,
                          uint32_t *err, bool refine, const TraceOpts &opts, cudaStream_t st, const uint32_t *perm,
-                         uint32_t *chunk_scratch, const RayCells *cells) {
+                         uint32_t *chunk_scratch, const RayCells *cells, const uint32_t *gate) {
   if (n == 0) return cudaSuccess;
   if (g_num_sms == 0) {
     int dev = 0;
@@ -968,10 +972,10 @@ cudaError_t launch_trace(const DevScene &sc, const rt_ray *rays, uint32_t n, rt_
   // Traversal stack: trace.stack entries (16, 32 or 64), raised to the
   // smallest size that holds the tree's depth.
   const int stk = trace_stack_entries(opts, sc);
-  return stk <= 16 ? launch_variant<16>(sc, rays, n, hits, counter, err, opts, perm, chunk_scratch, cells, refine, st)
+  return stk <= 16 ? launch_variant<16>(sc, rays, n, hits, counter, err, opts, perm, chunk_scratch, cells, gate, refine, st)
          : stk <= 32
-             ? launch_variant<32>(sc, rays, n, hits, counter, err, opts, perm, chunk_scratch, cells, refine, st)
-             : launch_variant<64>(sc, rays, n, hits, counter, err, opts, perm, chunk_scratch, cells, refine, st);
+             ? launch_variant<32>(sc, rays, n, hits, counter, err, opts, perm, chunk_scratch, cells, gate, refine, st)
+             : launch_variant<64>(sc, rays, n, hits, counter, err, opts, perm, chunk_scratch, cells, gate, refine, st);
 }
 
 cudaError_t launch_trace_literal16(const DevScene &sc, const rt_ray *rays, uint32_t n, rt_hit *hits,
