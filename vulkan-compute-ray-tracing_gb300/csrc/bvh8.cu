@@ -46,10 +46,12 @@
 // one node are consecutive, in slot order.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <climits>
 #include <cstdio>
 #include <cstring>
 
+#include "grid_sync.cuh"
 #include "rt_internal.h"
 
 namespace rtgb {
@@ -83,23 +85,35 @@ __host__ __device__ inline bool quantize_node8(const float box[8][6], const int3
     int e = -126;
     if (E > 0.0) {
       int e0 = 0;
-      frexp(E / 255.0, &e0);  // E / 255 <= 2^e0
-      e = (E <= 255.0 * ldexp(1.0, e0 - 1)) ? e0 - 1 : e0;
+      frexp(E, &e0);  // 2^(e0 - 1) <= E < 2^e0, so 2^(e0 - 9) is too small a step
+      e = (E <= 255.0 * ldexp(1.0, e0 - 8)) ? e0 - 8 : e0 - 7;
       e = e < -126 ? -126 : (e > 127 ? 127 : e);
     }
-    const double sc = ldexp(1.0, e);
+    // Steps are powers of two: multiplying by the inverse divides exactly.
+    const double sc = ldexp(1.0, e), inv = ldexp(1.0, -e);
     if (E > 255.0 * sc) ok = false;
     for (int s = 0; s < 8; s++) {
       int ql = 255, qh = 0;
       if ((fmask >> s) & 1u) {
         const double lo = box[s][k], hi = box[s][3 + k];
-        ql = (int)floor((lo - (double)ulo) / sc);
+        ql = (int)floor((lo - (double)ulo) * inv);
         ql = ql < 0 ? 0 : (ql > 255 ? 255 : ql);
-        while (ql > 0 && (double)ulo + ql * sc > lo) ql--;
-        qh = (int)ceil((hi - (double)ulo) / sc);
+        while ((double)ulo + ql * sc > lo) {
+          if (ql == 0) {
+            ok = false;
+            break;
+          }
+          ql--;
+        }
+        qh = (int)ceil((hi - (double)ulo) * inv);
         qh = qh < 0 ? 0 : (qh > 255 ? 255 : qh);
-        while (qh < 255 && (double)ulo + qh * sc < hi) qh++;
-        if ((double)ulo + ql * sc > lo || (double)ulo + qh * sc < hi) ok = false;
+        while ((double)ulo + qh * sc < hi) {
+          if (qh == 255) {
+            ok = false;
+            break;
+          }
+          qh++;
+        }
       }
       w[4 + 2 * k + (s >> 2)] |= (uint32_t)ql << (8 * (s & 3));
       w[10 + 2 * k + (s >> 2)] |= (uint32_t)qh << (8 * (s & 3));
@@ -317,16 +331,13 @@ __device__ __forceinline__ int sah_slots(const float4 *__restrict__ bvh2, uint32
   return cnt;
 }
 
-// One frontier node per thread: bvh2 pair frontier[f] becomes bvh8 node
-// base + f. inner_cnt[f] receives its number of inner children.
-__global__ void k_collapse8(const float4 *__restrict__ bvh2, uint32_t n_pairs, const int32_t *__restrict__ frontier,
-                            uint32_t count, uint32_t base, float4 *__restrict__ bvh8, uint32_t *__restrict__ inner_cnt,
-                            const uint32_t *__restrict__ choice, uint32_t *__restrict__ err) {
-  const uint32_t f = blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= count) return;
+// One frontier node: bvh2 pair p0 expanded into the 8 slots at `o`. Returns
+// its number of inner children.
+__device__ __forceinline__ uint32_t expand_node(const float4 *__restrict__ bvh2, uint32_t n_pairs, int32_t p0,
+                                                float4 *__restrict__ o, const uint32_t *__restrict__ choice,
+                                                uint32_t *__restrict__ err) {
   Slot S[8];
   int cnt = 0;
-  const int32_t p0 = frontier[f];
   if (p0 < 0 || (uint32_t)p0 >= n_pairs) {
     atomicOr(err, 1u);
   } else if (choice) {
@@ -355,7 +366,6 @@ __global__ void k_collapse8(const float4 *__restrict__ bvh2, uint32_t n_pairs, c
       cnt++;
     }
   }
-  float4 *o = bvh8 + 16ull * (base + f);
   const float inf = __int_as_float(0x7f800000);
   for (int s = 0; s < 8; s++) {
     o[2 * s] = make_float4(inf, inf, inf, inf);
@@ -378,67 +388,133 @@ __global__ void k_collapse8(const float4 *__restrict__ bvh2, uint32_t n_pairs, c
       inner += S[i].ref >= 0 ? 1u : 0u;
     }
   }
-  inner_cnt[f] = inner;
+  return inner;
 }
 
-// Numbers the inner children of the level's nodes (next_base + offs[f] + i)
-// and lists their bvh2 pairs as the next frontier.
-__global__ void k_link8(uint32_t count, uint32_t base, uint32_t next_base, const uint32_t *__restrict__ offs,
-                        float4 *__restrict__ bvh8, int32_t *__restrict__ next_frontier, uint32_t cap,
-                        uint32_t *__restrict__ err) {
-  const uint32_t f = blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= count) return;
-  float4 *o = bvh8 + 16ull * (base + f);
-  uint32_t r = offs[f];
-  for (int s = 0; s < 8; s++) {
-    float4 w = o[2 * s + 1];
-    const int32_t ref = __float_as_int(w.z);
-    if (ref < 0) continue;
-    if (next_base + r >= cap) {
-      atomicOr(err, 2u);
+constexpr int kFoldThreads = 128;
+constexpr uint32_t kFoldWarps = kFoldThreads / 32;
+// Device words of a fold: barrier counter, error bits (1, 2 bad reference, 4
+// capacity, 8 box off its grid, KERR_TIMEOUT << 4), nodes, levels.
+enum : uint32_t { kFoldBarrier = 0, kFoldErr = 1, kFoldNodes = 2, kFoldLevels = 3, kFoldWords = 8 };
+constexpr uint32_t kFoldTimeout = KERR_TIMEOUT << 4;
+
+// The whole fold, level by level, in one cooperative launch: node base + f of
+// a level is pair frontier[f]; its inner children are numbered after the
+// level, in order, and are the next frontier. Each CTA keeps to one run of
+// the frontier: it expands its nodes and counts their inner children, then
+// (after a barrier) knows the counts before it and numbers them. 13 levels of
+// 1.31M triangles in 0.55 ms (1.6 with three launches and a host round trip a
+// level), 12,012 triangles in 0.2 (0.6).
+__global__ void __launch_bounds__(kFoldThreads) k_fold8(const float4 *__restrict__ bvh2, uint32_t n_pairs,
+                                                        const uint32_t *__restrict__ choice, float4 *bvh8,
+                                                        uint32_t cap, int32_t *fr0, int32_t *fr1, uint32_t *inner_cnt,
+                                                        uint32_t *counts, uint32_t *ctr) {
+  __shared__ uint32_t s_part[kFoldWarps], s_sum[2][kFoldWarps];
+  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  uint32_t *err = ctr + kFoldErr;
+  uint32_t target = 0, count = 1, base = 0, levels = 0;
+  int32_t *fr = fr0, *next = fr1;  // fr0[0] is the root pair, 0
+  while (count > 0) {
+    if ((uint64_t)base + count > cap || levels >= 128) {
+      if (blockIdx.x == 0 && tid == 0) atomicOr(err, 4u);
       return;
     }
-    next_frontier[r] = ref;
-    w.z = __int_as_float((int32_t)(next_base + r));
-    o[2 * s + 1] = w;
-    r++;
+    const uint32_t run = (count + gridDim.x - 1) / gridDim.x;
+    const uint32_t beg = min(count, blockIdx.x * run), end = min(count, beg + run);
+    uint32_t mine = 0;
+    for (uint32_t f = beg + tid; f < end; f += kFoldThreads) {
+      const uint32_t c = expand_node(bvh2, n_pairs, __ldcg(fr + f), bvh8 + 16ull * (base + f), choice, err);
+      inner_cnt[f] = c;
+      mine += c;
+    }
+    mine = __reduce_add_sync(0xffffffffu, mine);
+    if (lane == 0) s_part[warp] = mine;
+    __syncthreads();
+    if (warp == 0) {
+      mine = __reduce_add_sync(0xffffffffu, lane < kFoldWarps ? s_part[lane] : 0u);
+      if (lane == 0) counts[blockIdx.x] = mine;
+    }
+    if (!grid_barrier_bit(ctr + kFoldBarrier, err, kFoldTimeout, target)) return;
+    uint32_t before = 0, total = 0;
+    for (uint32_t b = tid; b < gridDim.x; b += kFoldThreads) {
+      const uint32_t c = __ldcg(counts + b);
+      total += c;
+      if (b < blockIdx.x) before += c;
+    }
+    before = __reduce_add_sync(0xffffffffu, before);
+    total = __reduce_add_sync(0xffffffffu, total);
+    if (lane == 0) s_sum[0][warp] = before, s_sum[1][warp] = total;
+    __syncthreads();
+    before = __reduce_add_sync(0xffffffffu, lane < kFoldWarps ? s_sum[0][lane] : 0u);
+    total = __reduce_add_sync(0xffffffffu, lane < kFoldWarps ? s_sum[1][lane] : 0u);
+    const uint32_t next_base = base + count;
+    if ((uint64_t)next_base + total > cap) {
+      if (blockIdx.x == 0 && tid == 0) atomicOr(err, 4u);
+      return;  // every CTA: the same sums
+    }
+    for (uint32_t f0 = beg; f0 < end; f0 += kFoldThreads) {
+      const uint32_t f = f0 + tid;
+      const uint32_t c = f < end ? inner_cnt[f] : 0u;  // this thread's own write
+      uint32_t x = c;
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= (uint32_t)o) x += y;
+      }
+      __syncthreads();
+      if (lane == 31) s_part[warp] = x;
+      __syncthreads();
+      const uint32_t part = lane < kFoldWarps ? s_part[lane] : 0u;
+      uint32_t r = before + x - c + __reduce_add_sync(0xffffffffu, lane < warp ? part : 0u);
+      before += __reduce_add_sync(0xffffffffu, part);
+      if (c == 0) continue;
+      float4 *o = bvh8 + 16ull * (base + f);
+      for (int s = 0; s < 8; s++) {
+        const int32_t ref = __float_as_int(o[2 * s + 1].z);
+        if (ref < 0) continue;
+        next[r] = ref;
+        o[2 * s + 1].z = __int_as_float((int32_t)(next_base + r));
+        r++;
+      }
+    }
+    base = next_base;
+    count = total;
+    levels++;
+    int32_t *t = fr;
+    fr = next;
+    next = t;
+    if (!grid_barrier_bit(ctr + kFoldBarrier, err, kFoldTimeout, target)) return;
+  }
+  if (blockIdx.x == 0 && tid == 0) {
+    ctr[kFoldNodes] = base;
+    ctr[kFoldLevels] = levels;
   }
 }
 
-// Range-checks every child ref once all levels are built (inner refs
-// against the node count, leaf refs against the triangle count); the
-// traversal then uses leaf refs without a check.
-__global__ void k_encode8(uint32_t n8, uint32_t ntris, const float4 *__restrict__ bvh8, uint32_t *__restrict__ err) {
-  const uint32_t f = blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= n8) return;
-  const float4 *o = bvh8 + 16ull * f;
-  for (int s = 0; s < 8; s++) {
-    const int32_t ref = __float_as_int(o[2 * s + 1].z);
-    if (ref == INT_MIN) continue;
-    if (ref < 0 ? (uint32_t)~ref >= ntris : (uint32_t)ref >= n8) atomicOr(err, 2u);
+// fp32 fold -> 96-byte quantized nodes, every child ref range-checked (inner
+// refs against the node count, leaf refs against the triangle count): the
+// traversal uses leaf refs without a check.
+__global__ void k_quantize8(const float4 *__restrict__ wide, const uint32_t *__restrict__ n8_at, uint32_t ntris,
+                            uint4 *__restrict__ out, uint32_t *__restrict__ err) {
+  const uint32_t n8 = *n8_at;
+  for (uint32_t f = blockIdx.x * blockDim.x + threadIdx.x; f < n8; f += gridDim.x * blockDim.x) {
+    const float4 *W = wide + 16ull * f;
+    float box[8][6];
+    int32_t ref[8];
+    uint32_t fmask = 0;
+    for (int s = 0; s < 8; s++) {
+      const float4 a = W[2 * s], b = W[2 * s + 1];
+      box[s][0] = a.x, box[s][1] = a.y, box[s][2] = a.z;
+      box[s][3] = a.w, box[s][4] = b.x, box[s][5] = b.y;
+      ref[s] = __float_as_int(b.z);
+      if (ref[s] == INT_MIN) continue;
+      fmask |= 1u << s;
+      if (ref[s] < 0 ? (uint32_t)~ref[s] >= ntris : (uint32_t)ref[s] >= n8) atomicOr(err, 2u);
+    }
+    uint32_t w[24];
+    if (!quantize_node8(box, ref, fmask, w)) atomicOr(err, 8u);
+    uint4 *o = out + 6ull * f;
+    for (int i = 0; i < 6; i++) o[i] = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
   }
-}
-
-// fp32 fold -> 96-byte quantized nodes.
-__global__ void k_quantize8(const float4 *__restrict__ wide, uint32_t n8, uint4 *__restrict__ out,
-                            uint32_t *__restrict__ err) {
-  const uint32_t f = blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= n8) return;
-  const float4 *W = wide + 16ull * f;
-  float box[8][6];
-  int32_t ref[8];
-  uint32_t fmask = 0;
-  for (int s = 0; s < 8; s++) {
-    const float4 a = W[2 * s], b = W[2 * s + 1];
-    box[s][0] = a.x, box[s][1] = a.y, box[s][2] = a.z;
-    box[s][3] = a.w, box[s][4] = b.x, box[s][5] = b.y;
-    ref[s] = __float_as_int(b.z);
-    if (ref[s] != INT_MIN) fmask |= 1u << s;
-  }
-  uint32_t w[24];
-  if (!quantize_node8(box, ref, fmask, w)) atomicOr(err, 8u);
-  uint4 *o = out + 6ull * f;
-  for (int i = 0; i < 6; i++) o[i] = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
 }
 
 }  // namespace
@@ -463,138 +539,92 @@ cudaError_t collapse_choices(const DevScene &d, uint32_t *scr, uint32_t *choice,
   return cudaGetLastError();
 }
 
-// The fp32 fold (256-byte nodes) into `bvh8`, which holds `cap` nodes:
-// pairs chosen by the SAH (sah) or by opening the largest child first.
-cudaError_t build_wide_fp32(const DevScene &d, bool sah, float4 *bvh8, uint32_t cap, uint32_t *n8_out,
-                            uint32_t *levels_out, int32_t *root_out, char *errbuf, size_t errlen, cudaStream_t st) {
-  *n8_out = 0;
-  *levels_out = 0;
-  *root_out = 0;  // node 0
-  if (d.ntris == 0 || cap == 0 || !bvh8) return cudaErrorInvalidValue;
-  if (d.root_ref < 0) {
-    // One triangle: a single node with the root leaf in slot 0.
-    auto bits = [](int32_t i) {
-      float f;
-      std::memcpy(&f, &i, 4);
-      return f;
-    };
-    float4 h[16];
-    const float inf = bits(0x7f800000);
-    for (int s = 0; s < 8; s++) {
-      h[2 * s] = make_float4(inf, inf, inf, inf);
-      h[2 * s + 1] = make_float4(inf, inf, bits(INT_MIN), 0.0f);
-    }
-    h[0] = make_float4(d.root_lo[0], d.root_lo[1], d.root_lo[2], d.root_hi[0]);
-    h[1] = make_float4(d.root_hi[1], d.root_hi[2], bits(d.root_ref), 0.0f);
-    cudaError_t e = cudaMemcpyAsync(bvh8, h, sizeof(h), cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) return e;
-    *n8_out = 1;
-    *levels_out = 1;
-    *root_out = 0;  // node 0: one leaf in slot 0
-    return cudaSuccess;
-  }
-  const uint32_t n_pairs = d.ntris - 1;
-  // Scratch: two frontiers, counts, offsets (cap words each), scan sums, error word.
-  // With the SAH: the pairs' choices, and for their computation the parent
-  // links, arrival counters and costs (11 words per pair, 1 per leaf).
-  const size_t sah_words = sah ? 11ull * n_pairs + d.ntris : 0;
-  const size_t words = 4ull * cap + cap / 1024 + 8 + sah_words;
-  uint32_t *scr = nullptr;
-  cudaError_t e = cudaMallocAsync((void **)&scr, 4 * words, st);
-  if (e != cudaSuccess) return e;
-  int32_t *fr = (int32_t *)scr, *fr_next = (int32_t *)(scr + cap);
-  uint32_t *cnt = scr + 2ull * cap, *offs = scr + 3ull * cap, *errw = scr + 4ull * cap;
-  uint32_t *sums = errw + 4;
-  uint32_t *choice = sah ? sums + cap / 1024 + 4 : nullptr;
-  e = cudaMemsetAsync(errw, 0, 4, st);
-  if (e == cudaSuccess) e = cudaMemsetAsync(fr, 0, 4, st);  // the root pair is bvh2 record 0
-  if (e == cudaSuccess && sah) e = collapse_choices(d, choice + n_pairs, choice, errw, st);
-  uint32_t count = 1, base = 0, levels = 0, bad = 0;
-  while (e == cudaSuccess && count > 0) {
-    if (base + count > cap) {
-      bad = 4;
-      break;
-    }
-    const uint32_t grid = (count + 255) / 256;
-    k_collapse8<<<grid, 256, 0, st>>>(d.bvh2, n_pairs, fr, count, base, bvh8, cnt, choice, errw);
-    e = exclusive_scan_u32(cnt, offs, sums, count, st);
-    if (e != cudaSuccess) break;
-    k_link8<<<grid, 256, 0, st>>>(count, base, base + count, offs, bvh8, fr_next, cap, errw);
-    e = cudaGetLastError();
-    uint32_t tail[3] = {0, 0, 0};
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&tail[0], offs + count - 1, 4, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&tail[1], cnt + count - 1, 4, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&tail[2], errw, 4, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) break;
-    levels++;
-    base += count;
-    count = tail[0] + tail[1];
-    bad = tail[2];
-    if (bad) break;
-    int32_t *t = fr;
-    fr = fr_next;
-    fr_next = t;
-  }
-  if (e == cudaSuccess && !bad) {
-    if (base >= (1u << 28)) {
-      bad = 4;
-    } else {
-      k_encode8<<<(base + 255) / 256, 256, 0, st>>>(base, d.ntris, bvh8, errw);
-      e = cudaGetLastError();
-      uint32_t tail = 0;
-      if (e == cudaSuccess) e = cudaMemcpyAsync(&tail, errw, 4, cudaMemcpyDeviceToHost, st);
-      if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-      bad = tail;
-    }
-  }
-  cudaFreeAsync(scr, st);
-  if (e != cudaSuccess) return e;
-  if (bad) {
-    snprintf(errbuf, errlen, "bvh8 collapse: %s", bad & 4 ? "node capacity exceeded" : "bad child reference");
-    return cudaErrorInvalidValue;
-  }
-  *n8_out = base;
-  *levels_out = levels;
-  return cudaSuccess;
-}
-
 }  // namespace
 
 cudaError_t build_bvh8(const DevScene &d, bool sah, void *bvh8q, uint32_t cap, uint32_t *n8_out,
                        uint32_t *levels_out, int32_t *root_out, char *errbuf, size_t errlen, cudaStream_t st) {
   *n8_out = 0;
   *levels_out = 0;
+  *root_out = 0;  // node 0
   if (d.ntris == 0 || cap == 0 || !bvh8q) return cudaErrorInvalidValue;
-  float4 *wide = nullptr;
-  cudaError_t e = cudaMallocAsync((void **)&wide, 256ull * cap + 256, st);
+  const bool leaf_root = d.root_ref < 0;  // one triangle: a single node with the root leaf in slot 0
+  const uint32_t n_pairs = leaf_root ? 0 : d.ntris - 1;
+  int dev = 0, sms = 0, per_sm = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_fold8, kFoldThreads, 0);
   if (e != cudaSuccess) return e;
-  uint32_t *errw = reinterpret_cast<uint32_t *>(wide + 16ull * cap);
-  uint32_t n8 = 0, levels = 0;
-  e = build_wide_fp32(d, sah, wide, cap, &n8, &levels, root_out, errbuf, errlen, st);
+  const uint32_t grid = std::max(1u, std::min((uint32_t)(sms * std::max(1, std::min(per_sm, 4))),
+                                              (cap + kFoldThreads - 1) / kFoldThreads));
+  // Scratch: the fp32 nodes (256 bytes each), control words, two frontiers and
+  // the inner counts (cap words each), the CTAs' counts; for the SAH the
+  // pairs' choices, and for their computation the parent links, arrival
+  // counters and costs (11 words per pair, 1 per leaf).
+  const size_t sah_words = sah && !leaf_root ? 11ull * n_pairs + d.ntris : 0;
+  const size_t words = 64ull * cap + 64 + 3ull * cap + grid + sah_words;
+  uint32_t *mem = nullptr;
+  if ((e = cudaMallocAsync((void **)&mem, 4 * words, st)) != cudaSuccess) return e;
+  float4 *wide = reinterpret_cast<float4 *>(mem);
+  uint32_t *ctr = mem + 64ull * cap;
+  int32_t *fr0 = reinterpret_cast<int32_t *>(ctr + 64), *fr1 = fr0 + cap;
+  uint32_t *cnt = reinterpret_cast<uint32_t *>(fr1 + cap), *counts = cnt + cap;
+  uint32_t *choice = sah && !leaf_root ? counts + grid : nullptr;
+  uint32_t h[kFoldWords] = {0};
+  auto fold = [&](uint32_t *ch) {
+    cudaError_t r = cudaMemsetAsync(ctr, 0, 4 * kFoldWords, st);
+    if (leaf_root) {
+      auto bits = [](int32_t i) {
+        float f;
+        std::memcpy(&f, &i, 4);
+        return f;
+      };
+      float4 node[16];
+      const float inf = bits(0x7f800000);
+      for (int s = 0; s < 8; s++) {
+        node[2 * s] = make_float4(inf, inf, inf, inf);
+        node[2 * s + 1] = make_float4(inf, inf, bits(INT_MIN), 0.0f);
+      }
+      node[0] = make_float4(d.root_lo[0], d.root_lo[1], d.root_lo[2], d.root_hi[0]);
+      node[1] = make_float4(d.root_hi[1], d.root_hi[2], bits(d.root_ref), 0.0f);
+      const uint32_t one[2] = {1u, 1u};
+      if (r == cudaSuccess) r = cudaMemcpyAsync(wide, node, sizeof(node), cudaMemcpyHostToDevice, st);
+      if (r == cudaSuccess) r = cudaMemcpyAsync(ctr + kFoldNodes, one, sizeof(one), cudaMemcpyHostToDevice, st);
+    } else {
+      if (r == cudaSuccess) r = cudaMemsetAsync(fr0, 0, 4, st);  // the root pair is bvh2 record 0
+      if (r == cudaSuccess && ch) r = collapse_choices(d, ch + n_pairs, ch, ctr + kFoldErr, st);
+      if (r != cudaSuccess) return r;
+      const float4 *bvh2 = d.bvh2;
+      uint32_t np = n_pairs, cp = cap;
+      const uint32_t *cc = ch;
+      void *args[] = {&bvh2, &np, &cc, &wide, &cp, &fr0, &fr1, &cnt, &counts, &ctr};
+      r = cudaLaunchCooperativeKernel((const void *)k_fold8, dim3(grid), dim3(kFoldThreads), args, 0, st);
+    }
+    if (r != cudaSuccess) return r;
+    k_quantize8<<<(uint32_t)std::min<uint64_t>(((uint64_t)cap + 127) / 128, (uint64_t)sms * 16), 128, 0, st>>>(
+        wide, ctr + kFoldNodes, d.ntris, static_cast<uint4 *>(bvh8q), ctr + kFoldErr);
+    r = cudaGetLastError();
+    if (r == cudaSuccess) r = cudaMemcpyAsync(h, ctr, sizeof(h), cudaMemcpyDeviceToHost, st);
+    if (r == cudaSuccess) r = cudaStreamSynchronize(st);
+    return r;
+  };
+  e = fold(choice);
   // The SAH fold has no node bound below one per pair: past the capacity
   // sized for the largest-first fold, take that fold instead.
-  if (e == cudaErrorInvalidValue && sah && strstr(errbuf, "capacity")) {
-    errbuf[0] = 0;
-    e = build_wide_fp32(d, false, wide, cap, &n8, &levels, root_out, errbuf, errlen, st);
-  }
-  uint32_t bad = 0;
-  if (e == cudaSuccess) e = cudaMemsetAsync(errw, 0, 4, st);
-  if (e == cudaSuccess) {
-    k_quantize8<<<(n8 + 127) / 128, 128, 0, st>>>(wide, n8, static_cast<uint4 *>(bvh8q), errw);
-    e = cudaGetLastError();
-  }
-  if (e == cudaSuccess) e = cudaMemcpyAsync(&bad, errw, 4, cudaMemcpyDeviceToHost, st);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  cudaFreeAsync(wide, st);
+  if (e == cudaSuccess && choice && (h[kFoldErr] & 4u)) e = fold(nullptr);
+  cudaFreeAsync(mem, st);
   if (e != cudaSuccess) return e;
-  if (bad) {
-    snprintf(errbuf, errlen, "bvh8: a child box does not fit its node's 8-bit grid");
+  const uint32_t bad = h[kFoldErr], n8 = h[kFoldNodes];
+  if (bad || n8 >= (1u << 28)) {
+    if (bad & 8u)
+      snprintf(errbuf, errlen, "bvh8: a child box does not fit its node's 8-bit grid");
+    else
+      snprintf(errbuf, errlen, "bvh8 collapse: %s",
+               bad & kFoldTimeout ? "device wait timed out"
+                                  : (bad & 3u ? "bad child reference" : "node capacity exceeded"));
     return cudaErrorInvalidValue;
   }
   *n8_out = n8;
-  *levels_out = levels;
+  *levels_out = h[kFoldLevels];
   return cudaSuccess;
 }
 

@@ -12,7 +12,9 @@
 //   r[i] = r[i-31] for 31 <= i < 34;
 //   r[i] = r[i-31] + r[i-3] (mod 2^32) for i >= 34;
 //   the k-th rand() is r[k + 344] >> 1.
-// The tests pin it against the C library's rand().
+// The tests pin it against the C library's rand(). The builder's draws are
+// made on the GPU (bvh_build.cu: k_axes), a run of the sequence per warp; the
+// powers a warp jumps ahead by are prepared here.
 #include <cstdint>
 #include <vector>
 
@@ -59,9 +61,37 @@ void glibc_rand_values(uint32_t seed, uint64_t count, int32_t *out) {
   for (uint64_t k = 0; k < count; k++) out[k] = g.next();
 }
 
-void glibc_rand_axes(uint32_t seed, uint64_t count, uint8_t *out_mod3) {
+// The sequence is linear over the integers mod 2^32 with the characteristic
+// polynomial x^31 - x^28 - 1: with x^n = sum c[k] x^k modulo it,
+// r[n + j] = sum c[k] r[k + j]. pow2[b] holds x^(kAxisRun 2^b).
+AxisJump glibc_axis_jump(uint32_t seed) {
+  struct Table {
+    uint32_t p[AxisJump::kPowers][31];
+    Table() {
+      uint32_t cur[31] = {0, 1};  // x
+      for (int bit = 0; bit < AxisJump::kRunLog2 + AxisJump::kPowers; bit++) {
+        if (bit >= AxisJump::kRunLog2)
+          for (int k = 0; k < 31; k++) p[bit - AxisJump::kRunLog2][k] = cur[k];
+        uint32_t sq[61] = {0};
+        for (int i = 0; i < 31; i++)
+          for (int j = 0; j < 31; j++) sq[i + j] += cur[i] * cur[j];
+        for (int k = 60; k >= 31; k--) {  // x^k = x^(k-3) + x^(k-31)
+          sq[k - 3] += sq[k];
+          sq[k - 31] += sq[k];
+        }
+        for (int k = 0; k < 31; k++) cur[k] = sq[k];
+      }
+    }
+  };
+  static const Table table;
+  AxisJump a;
   GlibcRand g(seed);
-  for (uint64_t k = 0; k < count; k++) out_mod3[k] = (uint8_t)(g.next() % 3);
+  // The 31 words before the first draw, and the 30 after them.
+  for (int k = 0; k < 31; k++) a.first[k] = g.ring[(g.i - 31 + k) % 34];
+  for (int k = 31; k < 61; k++) a.first[k] = g.step();
+  for (int b = 0; b < AxisJump::kPowers; b++)
+    for (int k = 0; k < 31; k++) a.pow2[b][k] = table.p[b][k];
+  return a;
 }
 
 }  // namespace rtgb

@@ -9,7 +9,7 @@ namespace rtgb {
 // longer than any phase takes records an error and gets false, and so do the
 // others, at the same or their next barrier: every caller returns on false.
 // Data written before the barrier by other CTAs is read past L1 (__ldcg).
-__device__ __forceinline__ bool grid_barrier(uint32_t *counter, uint32_t *err, uint32_t &target) {
+__device__ __forceinline__ bool grid_barrier_bit(uint32_t *counter, uint32_t *err, uint32_t bit, uint32_t &target) {
   __shared__ int s_ok;
   target += gridDim.x;
   __syncthreads();
@@ -25,12 +25,15 @@ __device__ __forceinline__ bool grid_barrier(uint32_t *counter, uint32_t *err, u
       }
       if (poll > 64) __nanosleep(32);
     }
-    if (!ok) atomicOr(err, KERR_TIMEOUT);
+    if (!ok) atomicOr(err, bit);
     __threadfence();
     s_ok = ok;
   }
   __syncthreads();
   return s_ok != 0;
+}
+__device__ __forceinline__ bool grid_barrier(uint32_t *counter, uint32_t *err, uint32_t &target) {
+  return grid_barrier_bit(counter, err, KERR_TIMEOUT, target);
 }
 
 }  // namespace rtgb

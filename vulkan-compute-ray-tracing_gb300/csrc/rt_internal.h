@@ -270,12 +270,12 @@ cudaError_t launch_render_batch(const BatchJob *d_jobs, uint32_t n_jobs, uint32_
 cudaError_t launch_batch_advance(BatchJob *d_jobs, uint32_t n_jobs, cudaStream_t st);
 
 // ---------------------------------------------------------------- bvh_build.cu
-// Builds the Bvh.h node array on the GPU. `axes` holds rand() % 3 for every
-// node in pop order (2*n - 1 values, host-generated from glibc's rand()).
+// Builds the Bvh.h node array on the GPU, the split axes drawn from glibc's
+// rand() after srand(bvh_seed), one rand() % 3 per node in pop order.
 // test_error_level >= 0 (a test hook, "bvh.test_error_level") records an
 // error bit after that level's sort, as an overflow would; the build must
 // then fail with RT_ERR_INTERNAL.
-rt_status gpu_build_bvh(const rt_triangle *d_tris, uint32_t n, const uint8_t *h_axes, rt_bvh_node *d_nodes,
+rt_status gpu_build_bvh(const rt_triangle *d_tris, uint32_t n, uint32_t bvh_seed, rt_bvh_node *d_nodes,
                         cudaStream_t st, float *ms_out, uint32_t *depth_out, char *errbuf, size_t errlen,
                         int test_error_level = -1);
 
@@ -302,6 +302,16 @@ bool ctx_wavefront_render(rt_ctx *ctx, const rt_render_params &p, bool *sort, bo
 // Device bytes rtUploadScene allocates for a scene of these counts.
 uint64_t scene_device_bytes(uint32_t n_triangles, uint32_t n_materials, uint32_t n_lights, uint32_t n_spheres);
 
+// ---------------------------------------------------------------- scene_check.cu
+// What a pass over a scene's triangles finds: the complement of the first
+// triangle that is not finite or names a material out of range (0: none),
+// the largest coordinate's bits, and the number of light triangles.
+struct SceneCheck {
+  uint32_t bad, max_coord, lights, _pad;
+};
+cudaError_t launch_check_scene(const rt_triangle *tris, uint32_t n, const rt_material *mats, uint32_t nm,
+                               SceneCheck *out, uint32_t *lights, cudaStream_t st);
+
 // ---------------------------------------------------------------- lbvh.cu
 // A linear BVH (Morton order) in the Bvh.h node layout; not the reference's
 // tree — a separately reported traversal mode.
@@ -320,7 +330,16 @@ rt_status gpu_build_ploc(const rt_triangle *d_tris, uint32_t n, uint32_t radius,
 
 // ---------------------------------------------------------------- glibc_rand.cpp
 // glibc's TYPE_3 random() (what rand() returns) after srand(seed).
-void glibc_rand_axes(uint32_t seed, uint64_t count, uint8_t *out_mod3);
+// What a warp needs to start anywhere in that sequence (glibc_rand.cpp): the
+// sequence's 61 words from 31 before the first draw, and the powers of x that
+// jump 2^(kRunLog2 + b) words ahead. Small enough for a kernel parameter; the
+// powers cover the 2^31 draws of the largest build.
+struct AxisJump {
+  static constexpr int kRunLog2 = 10, kPowers = 22;
+  uint32_t first[61];
+  uint32_t pow2[kPowers][31];
+};
+AxisJump glibc_axis_jump(uint32_t seed);
 void glibc_rand_values(uint32_t seed, uint64_t count, int32_t *out);
 
 }  // namespace rtgb
