@@ -174,7 +174,9 @@ rt_status rtTraceClosestHost(rt_ctx *ctx, rt_scene_id scene, const rt_ray *h_ray
  *   "trace.packet_min_rays"  batches below this many rays (default 2^20)
  *                   go to the 8-wide caster in input order, without the sort
  *                   or the packet pass; so do larger ones whose rays mostly
- *                   have origins of their own. Only while trace.wide,
+ *                   have origins of their own. The smallest (up to 32,768
+ *                   rays, 65,536 from 2^20 triangles up) are cast a few rays a
+ *                   warp. Only while trace.wide,
  *                   trace.packet and trace.defer are 1, trace.refill is 32 and
  *                   no beams are asked for. Results are identical either way
  *   "trace.packet"  1 (default) = a warp whose 32 rays share an origin and
@@ -234,7 +236,9 @@ rt_status rtTraceClosestHost(rt_ctx *ctx, rt_scene_id scene, const rt_ray *h_ray
  *   "render.mode"   0 megakernel (one thread runs a pixel's whole path),
  *                   1 wavefront (per-bounce kernels over compacted queues),
  *                   2 (default) wavefront for calls of several samples and
- *                   from render.wavefront_pixels up;
+ *                   from render.wavefront_pixels up, and up to 65,536 pixels
+ *                   one launch whose warps follow a few paths each; 3 the
+ *                   same without the wavefront;
  *                   images are identical in every mode
  *   "render.wavefront_pixels"  the mode-2 threshold of rtRender for calls of
  *                   one sample (default 2^18 pixels: 512 x 512 and up)

@@ -893,13 +893,19 @@ rt_status rtRender(rt_ctx *ctx, rt_scene_id id, const rt_render_params *p, float
     cudaError_t e = cudaMallocAsync(&scratch, wavefront_scratch_bytes(*p, ropts.sort != 0), st);
     if (e == cudaSuccess) {
       e = launch_render_wavefront(d, cam, *p, accum, ctx->d_segments, ctx->d_err, scratch, ropts.sort != 0,
-                                  use_wide(topts, d), st);
+                                  use_wide(topts, d), st, nullptr, true);
       cudaFreeAsync(scratch, st);
       if (e != cudaSuccess) return cuda_fail(ctx, e, "render launch");
       return RT_SUCCESS;
     }
     if (!small || e != cudaErrorMemoryAllocation) return cuda_fail(ctx, e, "wavefront scratch");
     cudaGetLastError();
+  }
+  if (ropts.mode >= 2 && use_wide(topts, d) && paths_ok(d, *p)) {
+    const cudaError_t e =
+        launch_render_paths(d, cam, *p, accum, ctx->d_segments, next_counter(ctx), ctx->d_err, st);
+    if (e != cudaSuccess) return cuda_fail(ctx, e, "render launch");
+    return RT_SUCCESS;
   }
   cudaError_t e = launch_render(d, cam, *p, accum, ctx->d_segments, ctx->d_err, st);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "render launch");
@@ -1028,7 +1034,7 @@ rt_status rtSetTuning(rt_ctx *ctx, const char *key, int64_t value) {
     return RT_SUCCESS;
   }
   if (k == "render.mode") {
-    if (value < 0 || value > 2) return RT_ERR_INVALID_ARGUMENT;
+    if (value < 0 || value > 3) return RT_ERR_INVALID_ARGUMENT;
     ctx->render_opts.mode = (int)value;
     return RT_SUCCESS;
   }

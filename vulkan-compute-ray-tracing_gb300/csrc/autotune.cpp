@@ -10,7 +10,7 @@
 //                trace.beam,
 //                each candidate timed with CUDA events over `reps` casts
 //                after one warm-up cast;
-//   render       megakernel against wavefront at growing square image sizes
+//   render       without the wavefront (render.mode 3) against it at growing square image sizes
 //                on the scene's camera; render.wavefront_pixels becomes the
 //                smallest size from which the wavefront wins.
 // The reference fixes the launch shape at compile time (local_size 32x32,
@@ -145,7 +145,7 @@ rt_status rtAutotuneRender(rt_ctx *ctx, rt_scene_id scene, uint32_t spp, uint32_
   for (uint32_t side = 256; side <= max_side && s == RT_SUCCESS; side *= 2) {
     float ms[2] = {0.0f, 0.0f};
     for (int mode = 0; mode < 2 && s == RT_SUCCESS; mode++) {
-      s = rtSetTuning(ctx, "render.mode", mode);
+      s = rtSetTuning(ctx, "render.mode", mode ? 1 : 3);
       if (s == RT_SUCCESS) s = time_render(ctx, scene, side, 1, max_bounces, accum, &ms[mode]);
     }
     if (s == RT_SUCCESS && ms[1] < ms[0]) {

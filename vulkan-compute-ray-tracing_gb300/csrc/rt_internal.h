@@ -157,7 +157,21 @@ inline bool cast_gated(const TraceOpts &o, const DevScene &sc) {
 }
 cudaError_t launch_wide_leaf(const DevScene &sc, const rt_ray *rays, uint32_t cap, const uint32_t *d_n,
                              const uint32_t *perm, const uint32_t *list, const uint32_t *list_count, int2 *hits,
-                             uint32_t *counter, uint32_t *err, int minblocks, int refill, cudaStream_t st);
+                             uint32_t *counter, uint32_t *err, int minblocks, int refill, cudaStream_t st,
+                             uint32_t min_rays = 0);
+// Small batches (pool.cu): R rays a warp from shared pools, up to this many
+// rays. A larger scene's rays take longer chains of steps, which the pools
+// shorten, so the GPU may be fuller before a ray per lane wins. us, ray per
+// lane / pools: 1,000 random rays into 20K, 328K, 1.31M triangles 57 / 21, 134
+// / 33, 288 / 70; 32,768 63 / 63, 191 / 89, 431 / 158; 65,536 69 / 96, 200 /
+// 131, 479 / 237; 65,536 camera rays 64 / 147, 188 / 258, 637 / 410.
+inline uint32_t pool_max_rays(const DevScene &sc) { return sc.ntris >= (1u << 20) ? 1u << 16 : 1u << 15; }
+cudaError_t launch_trace_pool(const DevScene &sc, const rt_ray *rays, uint32_t n, rt_hit *hits, uint32_t *counter,
+                              uint32_t *err, bool refine, cudaStream_t st);
+// The same for a device-sized queue, writing (leaf k, t) hits; a queue of more
+// than pool_max_rays is left to launch_wide_leaf with min_rays one above.
+cudaError_t launch_pool_leaf(const DevScene &sc, const rt_ray *rays, uint32_t cap, const uint32_t *d_n,
+                             const uint32_t *perm, int2 *hits, uint32_t *counter, uint32_t *err, cudaStream_t st);
 // Morton bucketing of a ray batch (raysort.cu); `scratch` holds
 // raysort_scratch_bytes(n); *perm_out points into it.
 size_t raysort_scratch_bytes(uint32_t n);
@@ -187,19 +201,26 @@ cudaError_t launch_trace_literal16(const DevScene &sc, const rt_ray *rays, uint3
 cudaError_t launch_render(const DevScene &sc, const rt_camera &cam, const rt_render_params &p, float *accum,
                           unsigned long long *segments, uint32_t *err, cudaStream_t st);
 
+// One-sample renders as one persistent launch of whole paths (paths.cu): same
+// images as launch_render. `counter` is a device word of this launch.
+bool paths_ok(const DevScene &sc, const rt_render_params &p);
+cudaError_t launch_render_paths(const DevScene &sc, const rt_camera &cam, const rt_render_params &p, float *accum,
+                                unsigned long long *segments, uint32_t *counter, uint32_t *err, cudaStream_t st);
+
 // Wavefront render (wavefront.cu): same images as launch_render; `scratch`
 // holds wavefront_scratch_bytes(p, sort). With d_sample_index the kernels read
 // the first sample index from the device at run time instead of
 // p.sample_index.
 size_t wavefront_scratch_bytes(const rt_render_params &p, bool sort);
-// `wide`: bounce rays are cast by the 8-wide caster (launch_wide_leaf).
+// `wide`: bounce rays are cast by the 8-wide caster (launch_wide_leaf), short
+// queues of a render that runs `alone` by launch_pool_leaf.
 cudaError_t launch_render_wavefront(const DevScene &sc, const rt_camera &cam, const rt_render_params &p, float *accum,
                                     unsigned long long *segments, uint32_t *err, void *scratch, bool sort, bool wide,
-                                    cudaStream_t st, const uint32_t *d_sample_index = nullptr);
+                                    cudaStream_t st, const uint32_t *d_sample_index = nullptr, bool alone = false);
 
 // Render launch-shape knobs (rtSetTuning "render.mode").
 struct RenderOpts {
-  int mode = 2;                         // 0 megakernel, 1 wavefront, 2 choose by image size
+  int mode = 2;  // 0 megakernel, 1 wavefront, 2 choose by image size, 3 choose, without the wavefront
   // mode 2: calls of one sample run as a wavefront from this many pixels up,
   // calls of several samples always: the samples share a wave, where the
   // megakernel's threads run them one after the other. Megakernel / wavefront,

@@ -325,6 +325,21 @@ __device__ __forceinline__ int camera_hit(const DevScene &sc, const PathState &p
   return k;
 }
 
+// The image's 8 x 4 tiles: positions 32 t .. 32 t + 31 are tile t's pixels.
+struct Tiles {
+  uint32_t W, H, across, positions;
+};
+inline Tiles tiles_of(const rt_render_params &p) {
+  const uint32_t across = (p.width + 7) / 8;
+  return Tiles{p.width, p.height, across, across * ((p.height + 3) / 4) * 32};
+}
+__device__ __forceinline__ bool tile_pixel(const Tiles &t, uint32_t pos, uint32_t &x, uint32_t &y) {
+  const uint32_t tile = pos >> 5, at = pos & 31u;
+  x = (tile % t.across) * 8 + (at & 7u);
+  y = (tile / t.across) * 4 + (at >> 3);
+  return x < t.W && y < t.H;
+}
+
 // Camera ray direction for pixel (x, y) (comp:371-372).
 __device__ __forceinline__ f3 camera_dir(const rt_camera &cam, uint32_t x, uint32_t y, uint32_t W, uint32_t H) {
   float u = __fdiv_rn((float)x, (float)W), v = __fdiv_rn((float)y, (float)H);
@@ -335,6 +350,21 @@ __device__ __forceinline__ f3 camera_dir(const rt_camera &cam, uint32_t x, uint3
 __device__ __forceinline__ float unorm8(float x) {
   float c = gclamp(x, 0.0f, 1.0f);
   return __fdiv_rn(floorf(__fadd_rn(__fmul_rn(c, 255.0f), 0.5f)), 255.0f);
+}
+
+// Sample s of colour c into the running mean (comp:375-379).
+__device__ __forceinline__ void running_mean(float4 &acc, f3 c, uint32_t s, uint32_t flags) {
+  const float sf = (float)s, keep = gmin(sf, 1.0f), den = __fadd_rn(sf, 1.0f);
+  acc.x = __fdiv_rn(__fadd_rn(c.x, __fmul_rn(__fmul_rn(acc.x, keep), sf)), den);
+  acc.y = __fdiv_rn(__fadd_rn(c.y, __fmul_rn(__fmul_rn(acc.y, keep), sf)), den);
+  acc.z = __fdiv_rn(__fadd_rn(c.z, __fmul_rn(__fmul_rn(acc.z, keep), sf)), den);
+  acc.w = __fdiv_rn(__fadd_rn(1.0f, __fmul_rn(__fmul_rn(acc.w, keep), sf)), den);
+  if (flags & RT_COMPAT_UNORM8) {
+    acc.x = unorm8(acc.x);
+    acc.y = unorm8(acc.y);
+    acc.z = unorm8(acc.z);
+    acc.w = unorm8(acc.w);
+  }
 }
 
 // spp samples of one pixel accumulated into the running mean (comp:375-379).
@@ -363,19 +393,7 @@ __device__ __forceinline__ uint32_t render_pixel(const DevScene &sc, const PathS
     uint32_t s = p.sample_index + k;
     Rng g{(600u * x + y) * (s + 1u)};
     f3 c = ray_color<STACK>(sc, ps, org, d0, k0, t0, p.max_bounces, g, segments, err);
-    float sf = (float)s;
-    float keep = gmin(sf, 1.0f);
-    float den = __fadd_rn(sf, 1.0f);
-    acc.x = __fdiv_rn(__fadd_rn(c.x, __fmul_rn(__fmul_rn(acc.x, keep), sf)), den);
-    acc.y = __fdiv_rn(__fadd_rn(c.y, __fmul_rn(__fmul_rn(acc.y, keep), sf)), den);
-    acc.z = __fdiv_rn(__fadd_rn(c.z, __fmul_rn(__fmul_rn(acc.z, keep), sf)), den);
-    acc.w = __fdiv_rn(__fadd_rn(1.0f, __fmul_rn(__fmul_rn(acc.w, keep), sf)), den);
-    if (p.flags & RT_COMPAT_UNORM8) {
-      acc.x = unorm8(acc.x);
-      acc.y = unorm8(acc.y);
-      acc.z = unorm8(acc.z);
-      acc.w = unorm8(acc.w);
-    }
+    running_mean(acc, c, s, p.flags);
   }
   accum[(size_t)y * p.width + x] = acc;
   return segments;

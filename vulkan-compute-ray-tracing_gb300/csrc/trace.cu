@@ -23,6 +23,7 @@
 #include "rt_internal.h"
 #include "shade.cuh"
 #include "beam.cuh"
+#include "refine.cuh"
 #include "traverse.cuh"
 #include "wide.cuh"
 
@@ -39,35 +40,6 @@ constexpr int kTraceBlock = 128;
 template <int MINB>
 __host__ __device__ constexpr int regs_for() {
   return (65536 / (128 * MINB)) / 8 * 8;
-}
-
-
-struct d3 {
-  double x, y, z;
-};
-__device__ __forceinline__ d3 dsub(d3 a, d3 b) { return d3{__dsub_rn(a.x, b.x), __dsub_rn(a.y, b.y), __dsub_rn(a.z, b.z)}; }
-__device__ __forceinline__ double ddot(d3 a, d3 b) {
-  return __dadd_rn(__dadd_rn(__dmul_rn(a.x, b.x), __dmul_rn(a.y, b.y)), __dmul_rn(a.z, b.z));
-}
-__device__ __forceinline__ d3 dcross(d3 a, d3 b) {
-  return d3{__dsub_rn(__dmul_rn(a.y, b.z), __dmul_rn(b.y, a.z)), __dsub_rn(__dmul_rn(a.z, b.x), __dmul_rn(b.z, a.x)),
-            __dsub_rn(__dmul_rn(a.x, b.y), __dmul_rn(b.x, a.y))};
-}
-
-// triIntersect in fp64 on the original vertices (fp32 inputs widened).
-__device__ __forceinline__ void refine_fp64(const rt_triangle *__restrict__ tris, int tri, f3 o, f3 d, float &t,
-                                            float &u, float &v) {
-  const float4 *T = reinterpret_cast<const float4 *>(tris + tri);
-  float4 a4 = __ldg(T), b4 = __ldg(T + 1), c4 = __ldg(T + 2);
-  d3 v0{a4.x, a4.y, a4.z}, v1{b4.x, b4.y, b4.z}, v2{c4.x, c4.y, c4.z};
-  d3 ro{o.x, o.y, o.z}, rd{d.x, d.y, d.z};
-  d3 a = dsub(v0, v1), b = dsub(v2, v0), p = dsub(v0, ro);
-  d3 n = dcross(b, a);
-  d3 q = dcross(p, rd);
-  double idet = __ddiv_rn(1.0, ddot(rd, n));
-  u = __double2float_rn(__dmul_rn(ddot(q, b), idet));
-  v = __double2float_rn(__dmul_rn(ddot(q, a), idet));
-  t = __double2float_rn(__dmul_rn(ddot(n, p), idet));
 }
 
 constexpr int kDone = INT_MIN;  // no node left: the ray is finished
@@ -479,42 +451,6 @@ __global__ void __launch_bounds__(kBeamRays, MINB)
   }
 }
 
-// Ordered keys for (t, triangle) pairs: ord_f maps fp32 to uint32 so that
-// unsigned order equals float order (-0 is first mapped to +0 by the
-// callers, which compare it equal to +0 as floats do).
-__device__ __forceinline__ uint32_t ord_f(float f) {
-  const uint32_t u = __float_as_uint(f);
-  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
-__device__ __forceinline__ float ord_inv(uint32_t u) {
-  return __uint_as_float((u & 0x80000000u) ? (u & 0x7fffffffu) : ~u);
-}
-
-// triIntersect of test_triangle on one precomputed record, without the
-// acceptance rule: true when tmin < t <= closest and the hit lies inside.
-__device__ __forceinline__ bool tri_candidate(const float4 *__restrict__ tpre, int k, f3 o, f3 d, float tmin,
-                                              float closest, float &t, float &u, float &v) {
-  const float4 *T = tpre + 3ll * k;
-  const float4 t0 = __ldg(T), t1 = __ldg(T + 1), t2 = __ldg(T + 2);
-  const f3 v0 = mk3(t0.x, t0.y, t0.z), n = mk3(t0.w, t1.x, t1.y);
-  const f3 a = mk3(t1.z, t1.w, t2.x), b = mk3(t2.y, t2.z, t2.w);
-  const f3 p = sub3(v0, o);
-  const float idet = __frcp_rn(dot3(d, n));  // correctly rounded 1/x: the value of the IEEE division 1.0f / x
-  t = __fmul_rn(dot3(n, p), idet);
-  if (!(t > tmin && t <= closest)) return false;
-  const f3 q = cross3(p, d);
-  u = __fmul_rn(dot3(q, b), idet);
-  v = __fmul_rn(dot3(q, a), idet);
-  return !(u < 0.0f || u > 1.0f || v < 0.0f || __fadd_rn(u, v) > 1.0f);
-}
-
-// Leaf pool entries per warp (power of two): at most 31 are left after the
-// leaf rounds of an iteration, and each of its VISITS node steps adds at
-// most 8 per lane (31 + 3 * 256 < 1024).
-template <int VISITS>
-__host__ __device__ constexpr int pool_entries() {
-  return VISITS == 1 ? 512 : 1024;
-}
 constexpr int kFinish = 64;  // finished-ray ring per warp (power of two, >= 64)
 template <int VISITS>
 __host__ __device__ constexpr int wide_warp_smem() {
@@ -561,7 +497,8 @@ __global__ void __maxnreg__(regs_for<MINB>()) k_trace_wide(DevScene sc, const fl
                                                                const uint32_t *__restrict__ perm,
                                                                const uint32_t *__restrict__ list,
                                                                const uint32_t *__restrict__ list_count,
-                                                               const uint32_t *gate, int refill, bool refine) {
+                                                               const uint32_t *gate, uint32_t min_rays, int refill,
+                                                               bool refine) {
   if (gate && !*gate) list = perm = nullptr;  // the whole batch, as it is
   // Per warp (wide_warp_smem bytes, dynamic): the lanes' rays (32 x 2
   // float4), closest-hit keys (32 x u64), winning t/u/v/leaf (32 x float4),
@@ -601,6 +538,7 @@ __global__ void __maxnreg__(regs_for<MINB>()) k_trace_wide(DevScene sc, const fl
   };
   const float INF = __int_as_float(0x7f800000);
   if (d_n) n = min(n, *d_n);
+  if (n < min_rays) return;  // k_trace_pool's
   const uint32_t total = list ? min(*list_count, (n + 31) / 32) * 32u : n;
   const float4 *__restrict__ bvh8 = sc.bvh8;
   const int32_t *__restrict__ words8 = reinterpret_cast<const int32_t *>(sc.bvh8);
@@ -854,7 +792,7 @@ cudaError_t launch_wide(const DevScene &sc, const float4 *rays, uint32_t n, int4
     if (e != cudaSuccess) return e;
   }
   kern<<<persistent_grid(kern, n, block, smem), block, smem, st>>>(
-      sc, rays, n, nullptr, hits, counter, err, perm, list, list_count, gate, refill, refine);
+      sc, rays, n, nullptr, hits, counter, err, perm, list, list_count, gate, 0u, refill, refine);
   return cudaGetLastError();
 }
 
@@ -931,7 +869,8 @@ bool wide_ok(const DevScene &sc) {
 
 cudaError_t launch_wide_leaf(const DevScene &sc, const rt_ray *rays, uint32_t cap, const uint32_t *d_n,
                              const uint32_t *perm, const uint32_t *list, const uint32_t *list_count, int2 *hits,
-                             uint32_t *counter, uint32_t *err, int minblocks, int refill, cudaStream_t st) {
+                             uint32_t *counter, uint32_t *err, int minblocks, int refill, cudaStream_t st,
+                             uint32_t min_rays) {
   if (!wide_ok(sc)) return cudaErrorInvalidValue;
   if (g_num_sms == 0) {
     int dev = 0;
@@ -943,7 +882,7 @@ cudaError_t launch_wide_leaf(const DevScene &sc, const rt_ray *rays, uint32_t ca
   auto go = [&](auto kern, size_t warp_smem) {
     const size_t smem = (size_t)(kTraceBlock / 32) * warp_smem;
     kern<<<persistent_grid(kern, cap, kTraceBlock, smem), kTraceBlock, smem, st>>>(
-        sc, r4, cap, d_n, hits, counter, err, perm, list, list_count, nullptr, refill, false);
+        sc, r4, cap, d_n, hits, counter, err, perm, list, list_count, nullptr, min_rays, refill, false);
     return cudaGetLastError();
   };
   const bool narrow = minblocks >= 8;
@@ -961,6 +900,7 @@ cudaError_t launch_trace(const DevScene &sc, const rt_ray *rays, uint32_t n, rt_
                          uint32_t *err, bool refine, const TraceOpts &opts, cudaStream_t st, const uint32_t *perm,
                          uint32_t *chunk_scratch, const RayCells *cells, const uint32_t *gate) {
   if (n == 0) return cudaSuccess;
+  if (n <= pool_max_rays(sc) && cast_direct(opts, sc, n)) return launch_trace_pool(sc, rays, n, hits, counter, err, refine, st);
   if (g_num_sms == 0) {
     int dev = 0;
     cudaGetDevice(&dev);

@@ -56,20 +56,6 @@ struct WfBufs {
 
 size_t a256(size_t x) { return (x + 255) & ~size_t(255); }
 
-// The image's 8 x 4 tiles: positions 32 t .. 32 t + 31 are tile t's pixels.
-struct Tiles {
-  uint32_t W, H, across, positions;
-};
-Tiles tiles_of(const rt_render_params &p) {
-  const uint32_t across = (p.width + 7) / 8;
-  return Tiles{p.width, p.height, across, across * ((p.height + 3) / 4) * 32};
-}
-__device__ __forceinline__ bool tile_pixel(const Tiles &t, uint32_t pos, uint32_t &x, uint32_t &y) {
-  const uint32_t tile = pos >> 5, at = pos & 31u;
-  x = (tile % t.across) * 8 + (at & 7u);
-  y = (tile / t.across) * 4 + (at >> 3);
-  return x < t.W && y < t.H;
-}
 uint32_t wave_samples(const rt_render_params &p, const Tiles &t) {
   return std::max(1u, std::min(p.spp, kWavePaths / std::max(t.positions, 1u)));
 }
@@ -289,19 +275,7 @@ __global__ void k_wf_accumulate(Tiles tiles, uint32_t s0, uint32_t samples, cons
   float4 acc = *out;
   for (uint32_t k = 0; k < samples; k++) {
     const float4 c = white ? make_float4(1.0f, 1.0f, 1.0f, 0.0f) : color[(size_t)k * tiles.positions + pos];
-    float sf = (float)sample_of(s0 + k, d_s);
-    float keep = gmin(sf, 1.0f);
-    float den = __fadd_rn(sf, 1.0f);
-    acc.x = __fdiv_rn(__fadd_rn(c.x, __fmul_rn(__fmul_rn(acc.x, keep), sf)), den);
-    acc.y = __fdiv_rn(__fadd_rn(c.y, __fmul_rn(__fmul_rn(acc.y, keep), sf)), den);
-    acc.z = __fdiv_rn(__fadd_rn(c.z, __fmul_rn(__fmul_rn(acc.z, keep), sf)), den);
-    acc.w = __fdiv_rn(__fadd_rn(1.0f, __fmul_rn(__fmul_rn(acc.w, keep), sf)), den);
-    if (flags & RT_COMPAT_UNORM8) {
-      acc.x = unorm8(acc.x);
-      acc.y = unorm8(acc.y);
-      acc.z = unorm8(acc.z);
-      acc.w = unorm8(acc.w);
-    }
+    running_mean(acc, mk3(c.x, c.y, c.z), sample_of(s0 + k, d_s), flags);
   }
   *out = acc;
 }
@@ -319,7 +293,7 @@ size_t wavefront_scratch_bytes(const rt_render_params &p, bool sort) {
 
 cudaError_t launch_render_wavefront(const DevScene &sc, const rt_camera &cam, const rt_render_params &p, float *accum,
                                     unsigned long long *segments, uint32_t *err, void *scratch, bool sort, bool wide,
-                                    cudaStream_t st, const uint32_t *d_sample_index) {
+                                    cudaStream_t st, const uint32_t *d_sample_index, bool alone) {
   const Tiles tiles = tiles_of(p);
   if (p.width == 0 || p.height == 0 || p.spp == 0) return cudaSuccess;
   const bool use_wide = wide && wide_ok(sc);
@@ -366,8 +340,16 @@ cudaError_t launch_render_wavefront(const DevScene &sc, const rt_camera &cam, co
       uint32_t *perm = nullptr;
       if (sort && (e = launch_raysort(b.rays[in], cap, count, b.sort, &perm, st)) != cudaSuccess) return e;
       if (use_wide) {
-        if ((e = launch_wide_leaf(sc, b.rays[in], cap, count, perm, nullptr, nullptr, b.hits, work + (bounce & 1),
-                                  err, 6, 4, st)) != cudaSuccess)
+        // A short queue of a render that has the GPU to itself is cast from
+        // shared pools: one of the two takes the queue, by its length on the
+        // device. Beside other renders the pools' extra visits cost more than
+        // their shorter chains (a batch of 16 scenes 19.6 ms so, 18.4 without).
+        if (alone && (e = launch_pool_leaf(sc, b.rays[in], cap, count, perm, b.hits, work + (bounce & 1), err, st)) !=
+                         cudaSuccess)
+          return e;
+        if ((!alone || cap > pool_max_rays(sc)) &&
+            (e = launch_wide_leaf(sc, b.rays[in], cap, count, perm, nullptr, nullptr, b.hits, work + (bounce & 1),
+                                  err, 6, 4, st, alone ? pool_max_rays(sc) + 1 : 0)) != cudaSuccess)
           return e;
       } else if (sc.depth <= 32) {
         k_wf_extend<32><<<extend_grid, kWfBlock, 0, st>>>(sc, reinterpret_cast<const float4 *>(b.rays[in]), cap,

@@ -173,4 +173,40 @@ __device__ __forceinline__ int traverse_wide_lane(const DevScene &sc, const Trac
   return best;
 }
 
+// Ordered keys for (t, triangle) pairs: ord_f maps fp32 to uint32 so that
+// unsigned order equals float order (-0 is first mapped to +0 by the
+// callers, which compare it equal to +0 as floats do).
+__device__ __forceinline__ uint32_t ord_f(float f) {
+  const uint32_t u = __float_as_uint(f);
+  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+}
+__device__ __forceinline__ float ord_inv(uint32_t u) {
+  return __uint_as_float((u & 0x80000000u) ? (u & 0x7fffffffu) : ~u);
+}
+
+// triIntersect of test_triangle on one precomputed record, without the
+// acceptance rule: true when tmin < t <= closest and the hit lies inside.
+__device__ __forceinline__ bool tri_candidate(const float4 *__restrict__ tpre, int k, f3 o, f3 d, float tmin,
+                                              float closest, float &t, float &u, float &v) {
+  const float4 *T = tpre + 3ll * k;
+  const float4 t0 = __ldg(T), t1 = __ldg(T + 1), t2 = __ldg(T + 2);
+  const f3 v0 = mk3(t0.x, t0.y, t0.z), n = mk3(t0.w, t1.x, t1.y);
+  const f3 a = mk3(t1.z, t1.w, t2.x), b = mk3(t2.y, t2.z, t2.w);
+  const f3 p = sub3(v0, o);
+  const float idet = __frcp_rn(dot3(d, n));  // correctly rounded 1/x: the value of the IEEE division 1.0f / x
+  t = __fmul_rn(dot3(n, p), idet);
+  if (!(t > tmin && t <= closest)) return false;
+  const f3 q = cross3(p, d);
+  u = __fmul_rn(dot3(q, b), idet);
+  v = __fmul_rn(dot3(q, a), idet);
+  return !(u < 0.0f || u > 1.0f || v < 0.0f || __fadd_rn(u, v) > 1.0f);
+}
+
+// Leaf pool entries per warp (power of two): at most 31 are left after the
+// leaf rounds of an iteration, and each of its VISITS node steps adds at
+// most 8 per lane (31 + 3 * 256 < 1024).
+template <int VISITS>
+__host__ __device__ constexpr int pool_entries() {
+  return VISITS == 1 ? 512 : 1024;
+}
 }  // namespace rtgb
