@@ -116,12 +116,13 @@ __device__ __forceinline__ void pool_step(PoolWarp<R> &S, const DevScene &sc, ui
       const uint32_t l = S.leaves[(head + lane) & (kLeafPool - 1)];
       owner = l & 31u;
       k = (int)(l >> 5);
+      const uint32_t tri = (uint32_t)__ldg(sc.leaf_tri + k);
       const float4 q0 = S.org[owner], q1 = S.dir[owner];
       const unsigned long long cur = V.key[owner];
       if (tri_candidate(sc.tpre, k, mk3(q0.x, q0.y, q0.z), mk3(q1.x, q1.y, q1.z), q1.w,
                         ord_inv((uint32_t)(cur >> 32)), ct, cu, cv)) {
         const unsigned long long key =
-            ((unsigned long long)ord_f(__fadd_rn(ct, 0.0f)) << 32) | (uint32_t)__ldg(sc.leaf_tri + k);
+            ((unsigned long long)ord_f(__fadd_rn(ct, 0.0f)) << 32) | tri;
         if (key < cur) {
           acc = true;
           cand = key;

@@ -710,12 +710,13 @@ __global__ void __maxnreg__(regs_for<MINB>()) k_trace_wide(DevScene sc, const fl
         const uint32_t e = pool[(head + lane) & (kPool - 1)];
         owner = e & 31u;
         k = (int)(e >> 5);
+        const uint32_t tri = (uint32_t)__ldg(sc.leaf_tri + k);
         const float4 q0 = ray_s[owner][0], q1 = ray_s[owner][1];
         const unsigned long long cur = key_v[owner];
         if (tri_candidate(sc.tpre, k, mk3(q0.x, q0.y, q0.z), mk3(q1.x, q1.y, q1.z), q0.w,
                           ord_inv((uint32_t)(cur >> 32)), ct, cu, cv)) {
           const unsigned long long key =
-              ((unsigned long long)ord_f(__fadd_rn(ct, 0.0f)) << 32) | (uint32_t)__ldg(sc.leaf_tri + k);
+              ((unsigned long long)ord_f(__fadd_rn(ct, 0.0f)) << 32) | tri;
           if (key < cur) {
             acc = true;
             cand = key;
