@@ -542,7 +542,8 @@ cudaError_t collapse_choices(const DevScene &d, uint32_t *scr, uint32_t *choice,
 }  // namespace
 
 cudaError_t build_bvh8(const DevScene &d, bool sah, void *bvh8q, uint32_t cap, uint32_t *n8_out,
-                       uint32_t *levels_out, int32_t *root_out, char *errbuf, size_t errlen, cudaStream_t st) {
+                       uint32_t *levels_out, int32_t *root_out, char *errbuf, size_t errlen, cudaMemPool_t pool,
+                       cudaStream_t st) {
   *n8_out = 0;
   *levels_out = 0;
   *root_out = 0;  // node 0
@@ -563,7 +564,7 @@ cudaError_t build_bvh8(const DevScene &d, bool sah, void *bvh8q, uint32_t cap, u
   const size_t sah_words = sah && !leaf_root ? 11ull * n_pairs + d.ntris : 0;
   const size_t words = 64ull * cap + 64 + 3ull * cap + grid + sah_words;
   uint32_t *mem = nullptr;
-  if ((e = cudaMallocAsync((void **)&mem, 4 * words, st)) != cudaSuccess) return e;
+  if ((e = scratch_alloc((void **)&mem, 4 * words, pool, st)) != cudaSuccess) return e;
   float4 *wide = reinterpret_cast<float4 *>(mem);
   uint32_t *ctr = mem + 64ull * cap;
   int32_t *fr0 = reinterpret_cast<int32_t *>(ctr + 64), *fr1 = fr0 + cap;

@@ -965,15 +965,15 @@ cudaError_t enqueue_build(const rt_triangle *d_tris, uint32_t n, const BuildScra
 }  // namespace
 
 rt_status gpu_build_bvh(const rt_triangle *d_tris, uint32_t n, uint32_t bvh_seed, rt_bvh_node *d_nodes,
-                        cudaStream_t st, float *ms_out, uint32_t *depth_out, char *errbuf, size_t errlen,
-                        int test_error_level) {
+                        cudaMemPool_t pool, cudaStream_t st, float *ms_out, uint32_t *depth_out, char *errbuf,
+                        size_t errlen, int test_error_level) {
   rt_status status = RT_SUCCESS;
   unsigned char *mem = nullptr;
   BuildScratch s;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   BUILD_CHECK(cudaEventCreate(&e0));
   BUILD_CHECK(cudaEventCreate(&e1));
-  BUILD_CHECK(cudaMallocAsync((void **)&mem, build_scratch_bytes(n), st));
+  BUILD_CHECK(scratch_alloc((void **)&mem, build_scratch_bytes(n), pool, st));
   s = carve_build(mem, n);
   BUILD_CHECK(cudaEventRecord(e0, st));
   BUILD_CHECK(enqueue_axes(bvh_seed, n, s, st));

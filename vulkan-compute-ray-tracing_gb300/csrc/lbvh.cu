@@ -336,8 +336,8 @@ cudaError_t lbvh_sorted_keys(const rt_triangle *d_tris, uint32_t n, uint32_t *sc
   return e;
 }
 
-rt_status gpu_build_lbvh(const rt_triangle *d_tris, uint32_t n, rt_bvh_node *d_nodes, cudaStream_t st, float *ms_out,
-                         uint32_t *depth_out, char *errbuf, size_t errlen) {
+rt_status gpu_build_lbvh(const rt_triangle *d_tris, uint32_t n, rt_bvh_node *d_nodes, cudaMemPool_t pool,
+                         cudaStream_t st, float *ms_out, uint32_t *depth_out, char *errbuf, size_t errlen) {
   if (n == 0) return RT_ERR_INVALID_ARGUMENT;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   cudaEventCreate(&e0);
@@ -347,7 +347,7 @@ rt_status gpu_build_lbvh(const rt_triangle *d_tris, uint32_t n, rt_bvh_node *d_n
   void *mem = nullptr;
   const size_t sort_words = lbvh_sorted_keys_words(n);
   const size_t words = sort_words + n + n + 2ull * n + n + 8;
-  cudaError_t e = cudaMallocAsync(&mem, 4 * words, st);
+  cudaError_t e = scratch_alloc(&mem, 4 * words, pool, st);
   if (e != cudaSuccess) {
     std::snprintf(errbuf, errlen, "lbvh scratch: %s", cudaGetErrorString(e));
     cudaEventDestroy(e0);

@@ -299,8 +299,8 @@ __global__ void __launch_bounds__(kPlocThreads) k_ploc(const rt_triangle *__rest
 }  // namespace
 
 rt_status gpu_build_ploc(const rt_triangle *d_tris, uint32_t n, uint32_t radius, uint32_t max_rounds,
-                         rt_bvh_node *d_nodes, cudaStream_t st, float *ms_out, uint32_t *depth_out, char *errbuf,
-                         size_t errlen) {
+                         rt_bvh_node *d_nodes, cudaMemPool_t pool, cudaStream_t st, float *ms_out,
+                         uint32_t *depth_out, char *errbuf, size_t errlen) {
   if (n == 0 || radius < 1 || radius > kMaxRadius) return RT_ERR_INVALID_ARGUMENT;
   int dev = 0, sms = 0, per_sm = 0;
   const size_t tile = ploc_tile(radius);
@@ -316,7 +316,7 @@ rt_status gpu_build_ploc(const rt_triangle *d_tris, uint32_t n, uint32_t radius,
   const size_t sort_words = (lbvh_sorted_keys_words(n) + 63) & ~size_t(63);
   const size_t words = sort_words + 16ull * n + ((n + 63ull) & ~63ull) + 2ull * grid + 64;
   uint32_t *w = nullptr;
-  if (e == cudaSuccess) e = cudaMallocAsync((void **)&w, 4 * words, st);
+  if (e == cudaSuccess) e = scratch_alloc((void **)&w, 4 * words, pool, st);
   if (e != cudaSuccess) {
     std::snprintf(errbuf, errlen, "ploc scratch: %s", cudaGetErrorString(e));
     return e == cudaErrorMemoryAllocation ? RT_ERR_OUT_OF_MEMORY : RT_ERR_CUDA;

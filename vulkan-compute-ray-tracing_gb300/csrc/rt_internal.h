@@ -9,6 +9,18 @@
 
 namespace rtgb {
 
+// Stream-ordered scratch from a context's own memory pool (api.cpp). When the
+// device is full, the pool's unused memory is given back and the call made again.
+inline cudaError_t scratch_alloc(void **p, size_t bytes, cudaMemPool_t pool, cudaStream_t st) {
+  cudaError_t e = cudaMallocFromPoolAsync(p, bytes, pool, st);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    cudaMemPoolTrimTo(pool, 0);
+    e = cudaMallocFromPoolAsync(p, bytes, pool, st);
+  }
+  return e;
+}
+
 // Error bits kernels record in the context's device error word.
 enum : uint32_t {
   KERR_STACK_OVERFLOW = 1u,
@@ -71,7 +83,8 @@ uint32_t bvh8_capacity(uint32_t ntris);
 // first; synchronises `st`.
 constexpr size_t kBvh8NodeBytes = 96;
 cudaError_t build_bvh8(const DevScene &d, bool sah, void *bvh8q, uint32_t cap, uint32_t *n8_out,
-                       uint32_t *levels_out, int32_t *root_out, char *errbuf, size_t errlen, cudaStream_t st);
+                       uint32_t *levels_out, int32_t *root_out, char *errbuf, size_t errlen, cudaMemPool_t pool,
+                       cudaStream_t st);
 
 // ---------------------------------------------------------------- relayout.cu
 // Exclusive scan of n words (in may equal out); `sums` needs ceil(n/1024).
@@ -297,8 +310,8 @@ cudaError_t launch_batch_advance(BatchJob *d_jobs, uint32_t n_jobs, cudaStream_t
 // error bit after that level's sort, as an overflow would; the build must
 // then fail with RT_ERR_INTERNAL.
 rt_status gpu_build_bvh(const rt_triangle *d_tris, uint32_t n, uint32_t bvh_seed, rt_bvh_node *d_nodes,
-                        cudaStream_t st, float *ms_out, uint32_t *depth_out, char *errbuf, size_t errlen,
-                        int test_error_level = -1);
+                        cudaMemPool_t pool, cudaStream_t st, float *ms_out, uint32_t *depth_out, char *errbuf,
+                        size_t errlen, int test_error_level = -1);
 
 // ---------------------------------------------------------------- export.cu
 cudaError_t launch_export(const float *in, uint32_t n, float gamma, uint8_t *out, cudaStream_t st);
@@ -312,6 +325,8 @@ bool ctx_scene_dev(rt_ctx *ctx, rt_scene_id id, DevScene *out);
 unsigned long long *ctx_segments(rt_ctx *ctx);
 uint32_t *ctx_err(rt_ctx *ctx);
 uint64_t ctx_budget(rt_ctx *ctx);
+// cudaMalloc that gives the context's unused scratch back before it fails.
+cudaError_t ctx_malloc(rt_ctx *ctx, void **p, size_t bytes);
 int ctx_device(rt_ctx *ctx);
 cudaStream_t ctx_stream(rt_ctx *ctx);
 // True when a batch or a server step gives a job of these params to the
@@ -336,8 +351,8 @@ cudaError_t launch_check_scene(const rt_triangle *tris, uint32_t n, const rt_mat
 // ---------------------------------------------------------------- lbvh.cu
 // A linear BVH (Morton order) in the Bvh.h node layout; not the reference's
 // tree — a separately reported traversal mode.
-rt_status gpu_build_lbvh(const rt_triangle *d_tris, uint32_t n, rt_bvh_node *d_nodes, cudaStream_t st, float *ms_out,
-                         uint32_t *depth_out, char *errbuf, size_t errlen);
+rt_status gpu_build_lbvh(const rt_triangle *d_tris, uint32_t n, rt_bvh_node *d_nodes, cudaMemPool_t pool,
+                         cudaStream_t st, float *ms_out, uint32_t *depth_out, char *errbuf, size_t errlen);
 // Morton-sorted triangle centroids (lbvh.cu), shared by the LBVH and PLOC builders.
 size_t lbvh_sorted_keys_words(uint32_t n);
 cudaError_t lbvh_sorted_keys(const rt_triangle *d_tris, uint32_t n, uint32_t *scratch, uint32_t **codes_out,
@@ -346,8 +361,8 @@ cudaError_t lbvh_sorted_keys(const rt_triangle *d_tris, uint32_t n, uint32_t *sc
 // nearest neighbours searched within `radius` (1..256) positions. Fails with
 // RT_ERR_INTERNAL when max_rounds rounds leave more than one cluster.
 rt_status gpu_build_ploc(const rt_triangle *d_tris, uint32_t n, uint32_t radius, uint32_t max_rounds,
-                         rt_bvh_node *d_nodes, cudaStream_t st, float *ms_out, uint32_t *depth_out, char *errbuf,
-                         size_t errlen);
+                         rt_bvh_node *d_nodes, cudaMemPool_t pool, cudaStream_t st, float *ms_out,
+                         uint32_t *depth_out, char *errbuf, size_t errlen);
 
 // ---------------------------------------------------------------- glibc_rand.cpp
 // glibc's TYPE_3 random() (what rand() returns) after srand(seed).

@@ -179,7 +179,7 @@ void scheduler(rt_server *s) {
         }
       }
       if (st == RT_SUCCESS) {
-        cudaError_t e = cudaMalloc((void **)&q->d_accum, q->accum_bytes);
+        cudaError_t e = ctx_malloc(s->ctx, (void **)&q->d_accum, q->accum_bytes);
         if (e == cudaSuccess) e = cudaMemset(q->d_accum, 0, q->accum_bytes);
         if (e != cudaSuccess) st = e == cudaErrorMemoryAllocation ? RT_ERR_OUT_OF_MEMORY : RT_ERR_CUDA;
       }
@@ -243,7 +243,7 @@ void scheduler(rt_server *s) {
         if (s->scratch[k]) cudaFree(s->scratch[k]);
         s->scratch[k] = nullptr;
         s->scratch_bytes[k] = 0;
-        e = cudaMalloc(&s->scratch[k], need);
+        e = ctx_malloc(s->ctx, &s->scratch[k], need);
         if (e == cudaSuccess) s->scratch_bytes[k] = need;
       }
     }
