@@ -1,12 +1,15 @@
 // Closest-hit ray casting. Persistent launches sized to the SM count fetch
-// work from a global counter. The default whole-warp cast runs two kernels
-// per batch: k_trace_packets takes 32 consecutive rays (Morton order) per
+// work from a global counter. Large batches of rays that share an origin run
+// two kernels: k_trace_packets takes 32 consecutive rays (Morton order) per
 // warp and traverses coherent ones as a packet, listing the rest, and
 // k_trace_wide casts the listed chunks one ray per lane over the 8-wide
 // tree with a shared leaf pool (k_trace_lanes: the same over the binary
-// layout with postponed leaves). With trace.beam, k_trace_beams takes the
-// first kernel's place for sorted batches: one-origin batches are cast per
-// Morton cell as beams (beam.cuh), others in 32-ray chunks as above.
+// layout with postponed leaves). Smaller batches, and those of unrelated
+// origins, go to k_trace_wide as they are; the smallest to the shared node
+// pools of pool.cu (launch_trace has the rules). With trace.beam,
+// k_trace_beams takes the first kernel's place for sorted batches: one-origin
+// batches are cast per Morton cell as beams (beam.cuh), others in 32-ray
+// chunks as above.
 // k_trace is the per-lane refill form (a warp claims new rays as lanes
 // finish), k_trace_literal16 the shader's literal traversal.
 //
@@ -457,6 +460,115 @@ __host__ __device__ constexpr int wide_warp_smem() {
   return 64 * 16 + 32 * 8 + 32 * 16 + pool_entries<VISITS>() * 4 + kFinish * 4 + 16;
 }
 
+// One warp's part of shared memory (wide_warp_smem bytes): the lanes' rays,
+// their closest-hit keys, the winners' t, u, v and leaf, the leaf pool.
+struct WideWarp {
+  float4 ray[32][2];
+  unsigned long long key[32];
+  float4 hit[32];
+  uint32_t pool[1];
+};
+
+// The 32 oldest pooled leaves (all, if fewer), one per lane.
+__device__ __forceinline__ void wide_leaf_round(WideWarp &W, const float4 *__restrict__ tpre,
+                                                const int32_t *__restrict__ leaf_tri, uint32_t mask, uint32_t lane,
+                                                uint32_t &head, uint32_t tail) {
+  volatile WideWarp &V = W;
+  const uint32_t cnt = min(tail - head, 32u);
+  bool acc = false;
+  unsigned long long cand = 0;
+  uint32_t owner = 0;
+  int k = 0;
+  float ct = 0.0f, cu = 0.0f, cv = 0.0f;
+  if (lane < cnt) {
+    const uint32_t e = W.pool[(head + lane) & mask];
+    owner = e & 31u;
+    k = (int)(e >> 5);
+    const uint32_t tri = (uint32_t)__ldg(leaf_tri + k);
+    const float4 q0 = W.ray[owner][0], q1 = W.ray[owner][1];
+    const unsigned long long cur = V.key[owner];
+    if (tri_candidate(tpre, k, mk3(q0.x, q0.y, q0.z), mk3(q1.x, q1.y, q1.z), q0.w, ord_inv((uint32_t)(cur >> 32)),
+                      ct, cu, cv)) {
+      const unsigned long long key = ((unsigned long long)ord_f(__fadd_rn(ct, 0.0f)) << 32) | tri;
+      if (key < cur) {
+        acc = true;
+        cand = key;
+        atomicMin(&W.key[owner], key);
+      }
+    }
+  }
+  __syncwarp();
+  if (acc && V.key[owner] == cand) W.hit[owner] = make_float4(ct, cu, cv, __int_as_float(k));
+  __syncwarp();
+  head += cnt;
+}
+
+// A warp's last rays, when the batch has run out, share their nodes: half of
+// the leaf pool holds nodes then, the other half leaves. What is left of a
+// launch at that point is its longest rays' own chains of node and leaf steps,
+// with most lanes idle; from one pool the lanes walk a ray's frontier side by
+// side. Measured with 4 / 8 / 16 / 24 / 32 rays and without, us: 300,007
+// random rays into 82K triangles 130 / 121 / 107 / 108 / 111, 155; 4.19M into
+// 1.31M triangles 4877 / 4835 / 4583 / 4625 / 4667, 4734; a 1080p frame of 2M
+// triangles 3867 / 3787 / 3705 / 3741 / 3810, 4255; 16 wavefronts side by side
+// 17125 / 16450 / 15826 / 15959 / 16306, 17993 (4 and 8 in a form with a few
+// more spills).
+constexpr int kTailRays = 16;
+constexpr uint32_t kTailNodes = 512, kTailFlush = 8;
+
+// Steps of up to 32 pooled nodes and the leaf rounds that are due, until both
+// pools (count[0] leaves, count[1] nodes) are empty. Every node is numbered
+// above its parent (bvh8.cu), so this ends.
+__device__ __forceinline__ void wide_share_tail(WideWarp *W, uint32_t *count, const float4 *__restrict__ bvh8,
+                                             const float4 *__restrict__ tpre, const int32_t *__restrict__ leaf_tri,
+                                             uint32_t n8, uint32_t room, uint32_t *err) {
+  uint32_t lane;
+  asm("mov.u32 %0, %%laneid;" : "=r"(lane));
+  volatile WideWarp &V = *W;
+  volatile uint32_t *vcount = count;
+  uint32_t *nodes = W->pool + kTailNodes;
+  uint32_t head = 0;
+  for (;;) {
+    uint32_t held = vcount[1];
+    const uint32_t take = min(held, min(32u, max(1u, held < room ? (room - held) / 8 : 0u)));
+    const uint32_t e = lane < take ? nodes[held - 1 - lane] : 0u;
+    __syncwarp();
+    if (lane == 0) vcount[1] = held - take;
+    __syncwarp();
+    if (lane < take) {
+      const uint32_t q = e & 31u, v = e >> 5;
+      if (v >= n8) {
+        atomicOr(err, KERR_BAD_INDEX);
+      } else {
+        const float4 q0 = W->ray[q][0], q1 = W->ray[q][1];
+        const TraceRay r = make_ray(mk3(q0.x, q0.y, q0.z), mk3(q1.x, q1.y, q1.z), q0.w);
+        const uint32_t oct = (uint32_t)ray_octant(r);
+        WideStep ws;
+        wide_node_test(bvh8, (int)v, r, oct, ord_inv((uint32_t)(V.key[q] >> 32)), ws);
+        if (ws.hin) {
+          const uint32_t ranks = rank_bits(ws.hin, oct);
+          const uint32_t at = atomicAdd(count + 1, (uint32_t)__popc(ws.hin));
+#pragma unroll
+          for (uint32_t s = 0; s < 8; s++)
+            if ((ws.hin >> s) & 1u) nodes[at + __popc(ranks >> ((s ^ oct) + 1u))] = ((uint32_t)ws.ref[s] << 5) | q;
+        }
+        if (ws.leafmask) {
+          uint32_t at = atomicAdd(count, (uint32_t)__popc(ws.leafmask));
+#pragma unroll
+          for (uint32_t s = 0; s < 8; s++)
+            if ((ws.leafmask >> s) & 1u) W->pool[at++ & (kTailNodes - 1)] = ((uint32_t)~ws.ref[s] << 5) | q;
+        }
+      }
+    }
+    __syncwarp();
+    held = vcount[1];
+    const uint32_t tail = vcount[0];
+    while (tail - head >= 32u || (tail != head && held < kTailFlush))
+      wide_leaf_round(*W, tpre, leaf_tri, kTailNodes - 1, lane, head, tail);
+    if (held == 0 && tail == head) break;
+  }
+}
+
 // One ray per lane over bvh8 (Ylitie et al., HPG 2017, with explicit child
 // refs). A step tests the lane's 96-byte quantized node (wide.cuh:
 // wide_node_test: three 256-bit loads, eight slot tests with packed FMAs;
@@ -510,11 +622,11 @@ __global__ void __maxnreg__(regs_for<MINB>()) k_trace_wide(DevScene sc, const fl
   const uint32_t warp = threadIdx.x >> 5;
   const uint32_t lt_mask = (1u << lane) - 1u;
   constexpr int kPool = pool_entries<VISITS>();
+  constexpr bool kShareTail = GSTACK <= 32 && kPool >= 2 * (int)kTailNodes;
   float4 *const wbase = s_wide + warp * (wide_warp_smem<VISITS>() / 16);
   float4(*ray_s)[2] = reinterpret_cast<float4(*)[2]>(wbase);
   volatile unsigned long long *key_v = reinterpret_cast<unsigned long long *>(wbase + 64);
-  unsigned long long *key_a = reinterpret_cast<unsigned long long *>(wbase + 64);
-  float4 *hit_s = wbase + 80;
+    float4 *hit_s = wbase + 80;
   uint32_t *pool = reinterpret_cast<uint32_t *>(wbase + 112);
   uint32_t *finish = pool + kPool;
   // The pool's tail: lanes reserve their entries with one shared atomic.
@@ -623,6 +735,51 @@ __global__ void __maxnreg__(regs_for<MINB>()) k_trace_wide(DevScene sc, const fl
     }
     __syncwarp();
 
+    // Nothing left to claim and few rays on the way: their stacks become one
+    // pool of nodes that all lanes take from (unless they hold too many).
+    if (kShareTail && exhausted && __popc(__ballot_sync(0xffffffffu, ray_i >= 0)) <= kTailRays) {
+      const uint32_t room = kTailNodes - 32u - 7u * sc.levels8;  // pool.cuh's bound, for this tree
+      uint32_t mine = 0;
+      if (ray_i >= 0) {
+        mine = __popc(gmask) + (node >= 0 ? 1u : 0u);
+        for (int s = 0; s < gsp; s++) mine += __popc(gstack[s] & 0xffu);
+      }
+      if (__reduce_add_sync(0xffffffffu, mine) <= room) {
+        // Leaves still pooled (fewer than 32) move out of the nodes' half.
+        const uint32_t held = tail - head, leaf = lane < held ? pool[(head + lane) & (kPool - 1)] : 0u;
+        if (lane == 0) {
+          pool_tail[0] = held;
+          pool_tail[1] = 0u;
+        }
+        __syncwarp();
+        if (lane < held) pool[lane] = leaf;
+        if (mine) {
+          uint32_t *to = pool + kTailNodes + atomicAdd(const_cast<uint32_t *>(pool_tail) + 1, mine);
+          // Outermost group first: the pool is taken from its end.
+          for (int s = 0; s <= gsp; s++) {
+            const uint32_t g = s < gsp ? gstack[s] >> 8 : gnode;
+            for (uint32_t m = s < gsp ? gstack[s] & 0xffu : gmask; m;) {
+              const uint32_t rk = 31u - (uint32_t)__clz(m);
+              m ^= 1u << rk;
+              *to++ = ((uint32_t)__ldg(words8 + 24ll * g + 16 + (rk ^ oct)) << 5) | lane;
+            }
+          }
+          if (node >= 0) *to = ((uint32_t)node << 5) | lane;
+        }
+        __syncwarp();
+        wide_share_tail(reinterpret_cast<WideWarp *>(wbase), const_cast<uint32_t *>(pool_tail), bvh8, sc.tpre,
+                        sc.leaf_tri, n8, room, err);
+        __syncwarp();
+        if (lane == 0) pool_tail[0] = 0u;
+        node = -1;
+        gmask = 0;
+        gsp = 0;
+        head = tail = 0;
+        mlp1 = 0;
+        continue;
+      }
+    }
+
 #pragma unroll 1
     for (int visit = 0; visit < VISITS; visit++) {
       if (visit > 0 && !__any_sync(0xffffffffu, ray_i >= 0 && node >= 0)) break;
@@ -700,34 +857,7 @@ __global__ void __maxnreg__(regs_for<MINB>()) k_trace_wide(DevScene sc, const fl
     for (;;) {
       const bool waiting = ray_i >= 0 && node < 0 && gmask == 0 && gsp == 0 && (int)(head - mlp1) < 0;
       if (!__any_sync(0xffffffffu, waiting) && tail - head < 32u) break;
-      const uint32_t cnt = min(tail - head, 32u);
-      bool acc = false;
-      unsigned long long cand = 0;
-      uint32_t owner = 0;
-      int k = 0;
-      float ct = 0.0f, cu = 0.0f, cv = 0.0f;
-      if (lane < cnt) {
-        const uint32_t e = pool[(head + lane) & (kPool - 1)];
-        owner = e & 31u;
-        k = (int)(e >> 5);
-        const uint32_t tri = (uint32_t)__ldg(sc.leaf_tri + k);
-        const float4 q0 = ray_s[owner][0], q1 = ray_s[owner][1];
-        const unsigned long long cur = key_v[owner];
-        if (tri_candidate(sc.tpre, k, mk3(q0.x, q0.y, q0.z), mk3(q1.x, q1.y, q1.z), q0.w,
-                          ord_inv((uint32_t)(cur >> 32)), ct, cu, cv)) {
-          const unsigned long long key =
-              ((unsigned long long)ord_f(__fadd_rn(ct, 0.0f)) << 32) | tri;
-          if (key < cur) {
-            acc = true;
-            cand = key;
-            atomicMin(key_a + owner, key);
-          }
-        }
-      }
-      __syncwarp();
-      if (acc && key_v[owner] == cand) hit_s[owner] = make_float4(ct, cu, cv, __int_as_float(k));
-      __syncwarp();
-      head += cnt;
+      wide_leaf_round(*reinterpret_cast<WideWarp *>(wbase), sc.tpre, sc.leaf_tri, kPool - 1, lane, head, tail);
     }
   }
 }
