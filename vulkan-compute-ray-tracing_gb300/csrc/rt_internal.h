@@ -175,10 +175,13 @@ cudaError_t launch_wide_leaf(const DevScene &sc, const rt_ray *rays, uint32_t ca
 // Small batches (pool.cu): R rays a warp from shared pools, up to this many
 // rays. A larger scene's rays take longer chains of steps, which the pools
 // shorten, so the GPU may be fuller before a ray per lane wins. us, ray per
-// lane / pools: 1,000 random rays into 20K, 328K, 1.31M triangles 57 / 21, 134
-// / 33, 288 / 70; 32,768 63 / 63, 191 / 89, 431 / 158; 65,536 69 / 96, 200 /
-// 131, 479 / 237; 65,536 camera rays 64 / 147, 188 / 258, 637 / 410.
-inline uint32_t pool_max_rays(const DevScene &sc) { return sc.ntris >= (1u << 20) ? 1u << 16 : 1u << 15; }
+// lane / pools, random rays (camera rays): 1,000 into 20K, 328K, 1.31M
+// triangles 32 / 21, 75 / 32, 149 / 67; 16,384 into 20K 37 / 42 (41 / 36),
+// into 82K 53 / 49 (58 / 48); 32,768 into 82K 57 / 72 (68 / 77), into 328K
+// 101 / 88 (131 / 103); 65,536 into 1.31M 300 / 231 (565 / 409).
+inline uint32_t pool_max_rays(const DevScene &sc) {
+  return sc.ntris >= (1u << 20) ? 1u << 16 : sc.ntris >= (1u << 18) ? 1u << 15 : 1u << 14;
+}
 cudaError_t launch_trace_pool(const DevScene &sc, const rt_ray *rays, uint32_t n, rt_hit *hits, uint32_t *counter,
                               uint32_t *err, bool refine, cudaStream_t st);
 // The same for a device-sized queue, writing (leaf k, t) hits; a queue of more
