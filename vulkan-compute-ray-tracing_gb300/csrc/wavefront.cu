@@ -87,6 +87,15 @@ WfBufs carve(void *scratch, uint32_t cap, uint32_t positions) {
 // device (batched jobs advanced by a captured graph).
 __device__ __forceinline__ uint32_t sample_of(uint32_t s, const uint32_t *d_s) { return d_s ? *d_s + s : s; }
 
+// Camera rays are packets where triangles are large beside the pixels, and
+// rays of their own where a packet's rays soon part: from this many triangles
+// a pixel up. us a frame of one sample, packets / own rays: 100K triangles in a
+// Cornell box at 2.5 triangles a pixel 1350 / 1360, 1.5 1459 / 1492, 0.1
+// 6720 / 7313; a grid mesh of 512K at 12.8 728 / 461, 3.5 1020 / 706, 1.1 1148
+// / 957; a finer one of 84M at 200 x 200 14101 / 2005, 1024 x 1000 22057 /
+// 13424.
+constexpr uint32_t kOwnRayTris = 3;
+
 // The camera rays, a warp per tile: a packet where the tile's rays suit one
 // (warp_is_coherent), else each lane's own traversal.
 template <int STACK>
@@ -112,6 +121,19 @@ __global__ void __launch_bounds__(kWfBlock, 12) k_wf_camera(DevScene sc, rt_came
 #undef RTGB_CALL
   }
   if (active) hits[pos] = make_int2(k, __float_as_int(closest));
+}
+
+// The camera rays as a queue for the 8-wide caster; tile positions outside the
+// image get a ray of no length.
+__global__ void __launch_bounds__(kWfBlock) k_wf_rays(rt_camera cam, Tiles tiles, float4 *__restrict__ rays) {
+  const uint32_t pos = blockIdx.x * kWfBlock + threadIdx.x;
+  if (pos >= tiles.positions) return;
+  uint32_t x, y;
+  const bool active = tile_pixel(tiles, pos, x, y);
+  const f3 o = ld3(cam.origin);
+  const f3 d = active ? normalize3(camera_dir(cam, x, y, tiles.W, tiles.H)) : mk3(1.0f, 0.0f, 0.0f);
+  rays[2ull * pos] = make_float4(o.x, o.y, o.z, kTmin);
+  rays[2ull * pos + 1] = make_float4(d.x, d.y, d.z, active ? kTmax : -1.0f);
 }
 
 // Bounce rays where the 8-wide caster is not used: a warp takes 32 queued
@@ -310,7 +332,15 @@ cudaError_t launch_render_wavefront(const DevScene &sc, const rt_camera &cam, co
   const uint32_t shade_grid = std::min((cap + kShadeBlock - 1) / kShadeBlock, (uint32_t)g_sms * 8u);
   uint32_t extend_grid = 0;
   cudaError_t e = cudaSuccess;
-  if (p.max_bounces > 0) {
+  if (p.max_bounces > 0 && use_wide && sc.ntris / kOwnRayTris >= tiles.positions) {
+    if ((e = cudaMemsetAsync(b.counts, 0, 4 * kCountWords, st)) != cudaSuccess) return e;
+    k_wf_rays<<<tile_grid, kWfBlock, 0, st>>>(cam, tiles, reinterpret_cast<float4 *>(b.rays[0]));
+    const bool pool = alone && tiles.positions <= pool_max_rays(sc);
+    if ((e = pool ? launch_pool_leaf(sc, b.rays[0], tiles.positions, nullptr, nullptr, b.cam_hits, work, err, st)
+                  : launch_wide_leaf(sc, b.rays[0], tiles.positions, nullptr, nullptr, nullptr, nullptr, b.cam_hits,
+                                     work, err, 6, 4, st)) != cudaSuccess)
+      return e;
+  } else if (p.max_bounces > 0) {
     if (sc.depth <= 32)
       k_wf_camera<32><<<tile_grid, kWfBlock, 0, st>>>(sc, cam, tiles, b.cam_hits, err);
     else
