@@ -241,7 +241,7 @@ rt_status rtTraceClosestHost(rt_ctx *ctx, rt_scene_id scene, const rt_ray *h_ray
  *                   same without the wavefront;
  *                   images are identical in every mode
  *   "render.wavefront_pixels"  the mode-2 threshold of rtRender for calls of
- *                   one sample (default 2^18 pixels: 512 x 512 and up)
+ *                   one sample (default 2^17 pixels: 363 x 363 and up)
  *   "render.batch_wavefront_pixels"  the split of batches and of the
  *                   render server's steps: jobs from this many pixels up run
  *                   as wavefronts side by side on side streams, the rest in

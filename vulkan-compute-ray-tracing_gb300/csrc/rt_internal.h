@@ -237,13 +237,16 @@ cudaError_t launch_render_wavefront(const DevScene &sc, const rt_camera &cam, co
 // Render launch-shape knobs (rtSetTuning "render.mode").
 struct RenderOpts {
   int mode = 2;  // 0 megakernel, 1 wavefront, 2 choose by image size, 3 choose, without the wavefront
-  // mode 2: calls of one sample run as a wavefront from this many pixels up,
-  // calls of several samples always: the samples share a wave, where the
-  // megakernel's threads run them one after the other. Megakernel / wavefront,
-  // Cornell box with 12K triangles, 8 bounces, us: 1 sample 256 x 256 762 /
-  // 1077, 384 x 384 1364 / 1294, 512 x 512 2261 / 1721; 4 samples 48 x 48
-  // 2354 / 983, 256 x 256 3009 / 1717, 512 x 512 8897 / 4344.
-  uint64_t wavefront_pixels = 1u << 18;
+  // mode 2: calls of one sample run as a wavefront from this many pixels up
+  // (below, paths.cu up to 65,536 and the megakernel between), calls of
+  // several samples always: the samples share a wave, where the megakernel's
+  // threads run them one after the other. Megakernel / wavefront, Cornell box
+  // of 1K, 12K, 100K triangles, mesh of 512K, 8 bounces, 1 sample, us: 288 x
+  // 288 386 / 409, 1005 / 843, 1752 / 1497, 800 / 589; 352 x 352 459 / 458,
+  // 1256 / 950, 2367 / 1664, 967 / 677; 511 x 512 842 / 573, 2285 / 1334, 3920
+  // / 2238, 1300 / 806. 4 samples, 12K: 48 x 48 2354 / 983, 512 x 512 8897 /
+  // 4344.
+  uint64_t wavefront_pixels = 1u << 17;
   int batch_streams = 16;                // side streams a batch spreads its wavefront jobs over (1..16)
   // Batches and the render server: jobs from this many pixels up run as
   // wavefronts on side streams (the rest in the persistent tile launch).
