@@ -8,8 +8,10 @@ traced against the mesh through the C ABI —
     the sphere, tmin 1e-4.
 The mesh is the icosahedron subdivided 8 times (1,310,720 triangles), radius
 1, vertices displaced radially by 0.05*N(0,1); its BVH is built on the GPU
-node-for-node as the reference's Bvh.h builds it. All inputs are seeded
-synthetic data (no public dataset is involved).
+node-for-node as the reference's Bvh.h builds it, and rays are cast on the
+PLOC tree built beside it ("bvh.cast_tree", the default; the hits do not
+depend on the tree). All inputs are seeded synthetic data (no public dataset
+is involved).
 
 Reported on the one JSON line:
   value      rays/s (Mrays/s) with rays resident in HBM (device API); the
@@ -453,8 +455,9 @@ def run_gpu(args):
                 "frac": dom["frac"], "traffic": dom.get("traffic"), "peak_kind": peak_kind,
                 "dram_frac": dom.get("dram_frac"), "issue_frac": dom.get("issue_frac"),
                 "note": "achieved/frac: the oracle's algorithmic bytes (48 B per node or triangle record of the "
-                        "culled traversal of the reference tree, + 48 B ray and hit) over the live time; "
-                        "frac > 1 is L1/L2 reuse. dram_frac: the ncu capture's DRAM bytes over the live time "
+                        "culled traversal of the reference tree, + 48 B ray and hit) over the live time, the "
+                        "same work whatever tree the cast takes; "
+                        "frac > 1 is L1/L2 reuse and the cast tree's fewer visits. dram_frac: the ncu capture's DRAM bytes over the live time "
                         "against the HBM peak; issue_frac: its issued warp instructions over 4 issue slots per SM "
                         "per cycle at the sampled SM clock — the bound these kernels meet",
                 "per_kernel": {e["kernel"]: e for e in per}}
@@ -462,7 +465,8 @@ def run_gpu(args):
         "metric": METRIC, "value": value, "unit": "Mrays/s", "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": ms_max / args.steps, "higher_is_better": True,
         "scaling": "weak", "vs_baseline": None, "dtype": "f32", "data": "synthetic (seeded)",
-        "config": {"workload": WORKLOAD, "rays_per_step": rays_step, "bvh": "reference Bvh.h tree built on GPU",
+        "config": {"workload": WORKLOAD, "rays_per_step": rays_step, "bvh": "reference Bvh.h tree built on GPU, "
+                   + ("rays cast on the PLOC tree beside it" if ctx.get_tuning("bvh.cast_tree") else "rays cast on it"),
                    "l2": "inputs larger than L2 (rays 268 MB + hits 134 MB + scene 147 MB per step)",
                    "parallelism": f"replicas x{world}", "coherent_grays": RAYS_PER_BATCH / coh_ms / 1e6,
                    "incoherent_grays": RAYS_PER_BATCH / inc_ms / 1e6, "bvh_build_ms": info.build_ms,
@@ -481,9 +485,9 @@ def run_gpu(args):
         "gpu_launches": 18 * args.steps,
         "clocks": clocks,
     }
-    # Separately reported: the same workload on trees that are not the
-    # reference's (1 a linear BVH, 2 agglomerative clustering); the hits are
-    # identical, only the traversal work differs.
+    # Separately reported: the same workload in scenes whose only tree is not
+    # the reference's (1 a linear BVH, 2 agglomerative clustering); the hits
+    # are identical, only the build and the traversal work differ.
     for key, builder in (("lbvh_mode", 1), ("ploc_mode", 2)):
         ctx.set_tuning("bvh.builder", builder)
         sc_l = ctx.upload_scene(tris, mats)
@@ -692,7 +696,7 @@ def batch_c2(ctx, n_scenes: int, reps: int, modes=("plain_one_launch", "plain", 
             "modes": res, "speedup_vs_one_launch_per_request": ratio("plain_one_launch"),
             "speedup_vs_rtrender_per_request": ratio("plain"),
             "plain_forms": "plain_one_launch: one k_render launch per request, the reference's one dispatch per "
-                           "frame; plain: rtRender per request (megakernel below 2^20 pixels, wavefront above)",
+                           "frame; plain: rtRender per request",
             "setup_s": setup_s, "bvh_build_ms_total": build_ms, "reps": reps,
             "e2e": {"value": len(jobs) / e2e_s, "unit": "renders/s", "h2d_bytes_per_step": 0,
                     "d2h_bytes_per_step": d2h}}
@@ -744,8 +748,7 @@ def serve_c3(ctx, n_scenes: int, n_requests: int, rates, sides=(256, 512, 1024),
                         f"scenes, sides {tuple(sides)}, spp 1-{spp_max}, 8 bounces, 150 GB budget",
             "value": best, "unit": "renders/s", "rates": out, "speedup_vs_plain": ratios,
             "speedup_vs_one_launch_per_request": ratios_one,
-            "plain_forms": "plain: one request at a time with rtRender's split (megakernel below 512^2, wavefront "
-                           "from there up); plain_one_launch: one request at a time, one megakernel launch per "
+            "plain_forms": "plain: one request at a time through rtRender; plain_one_launch: one request at a time, one megakernel launch per "
                            "request",
             "e2e": {"value": best, "unit": "renders/s",
                     "note": "requests submitted from the host with each image copied back to host memory; "

@@ -6,14 +6,15 @@
 // The reference's tree splits every node at the median along a random axis
 // (Bvh.h:160-175); sibling boxes overlap heavily and a ray visits hundreds of
 // nodes. Closest-hit results do not depend on the tree (only the order in
-// which equal-t candidates are met does), so a tighter tree is a separate,
-// separately reported mode ("bvh.builder" = 1), not a replacement.
+// which equal-t candidates are met does), so this one can be the scene's only
+// tree ("bvh.builder" = 1). Its Morton sort also starts the PLOC build
+// (ploc.cu), whose tree rays are cast on by default.
 //
 // Steps: centroid bounds -> 30-bit Morton code per triangle -> stable radix
-// sort (k_morton_sort) -> one thread per inner node
-// finds its key range and split from the longest common prefixes of
-// neighbouring (code, index) keys -> leaves walk to the root with an atomic
-// visit count per inner node; the second child to arrive writes the union.
+// sort (k_morton_sort) -> one thread per inner node finds its key range and
+// split from the longest common prefixes of neighbouring (code, index) keys
+// -> leaves walk to the root with an atomic visit count per inner node; the
+// second child to arrive writes the union.
 // Leaf boxes are padded by 1e-4 exactly as Bvh.h pads them (Bvh.h:94-98).
 #include <cuda_runtime.h>
 

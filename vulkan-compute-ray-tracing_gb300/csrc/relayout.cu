@@ -1,4 +1,5 @@
-// Traversal layout derived from the reference node array (Bvh.h layout).
+// Traversal layout derived from a node array in Bvh.h layout (the tree rays
+// are cast on: the cast tree, or the scene's own).
 //
 // The reference traverses its 48-byte nodes one at a time and reads a node's
 // box when the node itself is popped (ray-trace-compute.comp:280-307), so a
@@ -6,9 +7,9 @@
 // boxes of BOTH children (64 bytes, four 16-byte loads), so one fetch decides
 // which children to descend into, and leaves point straight at a
 // precomputed triangle record. The tree itself — every box, every split —
-// is the reference's, unchanged.
+// is unchanged.
 //
-// Inner nodes keep the reference's relative order (rank among inner nodes);
+// Inner nodes keep the array's relative order (rank among inner nodes);
 // leaves are numbered by rank among leaves, and tpre/leaf_tri are stored in
 // that order so neighbouring leaves sit in neighbouring records.
 #include <cuda_runtime.h>

@@ -4,6 +4,9 @@
 // are coherent: a warp traces its camera segment as one packet, once per
 // call (render_pixel). The number of traced segments (camera + secondary rays) is
 // reduced per warp and added to a 64-bit counter for throughput reporting.
+// It takes calls of one sample too large for paths.cu and too small for the
+// wavefront, the shader's literal traversal, and what has no scratch for
+// either.
 #include <cuda_runtime.h>
 
 #include "rt_internal.h"
