@@ -1,5 +1,5 @@
-"""The shared-memory denoise kernel (radius up to 8) against the per-pixel
-one, which takes over in CTAs that see a texel that is not finite: planted
+"""The shared-memory denoise kernel (radius up to 8, images of some hundred
+16 x 16 blocks up) against the per-pixel one, which takes over in CTAs that see a texel that is not finite: planted
 infinities switch 32 x 16 pixel blocks from one to the other, and every pixel
 whose taps do not meet one keeps its value bit for bit."""
 import numpy as np
@@ -20,7 +20,7 @@ def denoise(rt, ctx, img, sigma, ksigma, threshold=0.1, mix=0.75):
 
 
 @pytest.mark.parametrize("radius", [0, 1, 2, 3, 4, 5, 7, 8])
-@pytest.mark.parametrize("w,h", [(96, 80), (95, 49), (31, 17)])
+@pytest.mark.parametrize("w,h", [(96, 80), (31, 17), (400, 223), (351, 229), (33, 1700), (1703, 31)])
 def test_tile_kernel_equals_per_pixel(rt, ctx, w, h, radius):
     img = np.random.default_rng(w + radius).uniform(0, 2, (h, w, 4)).astype(np.float32)
     img[::7, ::5] = -0.0
@@ -46,7 +46,16 @@ def test_tile_kernel_equals_per_pixel(rt, ctx, w, h, radius):
 @pytest.mark.parametrize("w,h", [(1, 1), (3, 2), (33, 5), (64, 33)])
 @pytest.mark.parametrize("radius", [2, 8, 9])
 def test_small_images_match_oracle(rt, orc, ctx, w, h, radius):
-    # Images smaller than the kernel wrap several times; 9 is the per-pixel kernel.
+    # Images smaller than the kernel wrap several times.
+    img = np.random.default_rng(w * h).uniform(0, 1, (h, w, 4)).astype(np.float32)
+    got = denoise(rt, ctx, img, float(radius), 1.0)
+    want = orc.denoise(img, float(radius), 1.0, 0.1, 0.75)
+    assert (np.abs(got.astype(np.float64) - want) / (1.0 + np.abs(want))).max() <= 2e-5
+
+
+@pytest.mark.parametrize("radius", [1, 4, 8, 9])
+@pytest.mark.parametrize("w,h", [(256, 144), (256, 160), (256, 304), (256, 320), (271, 305)])
+def test_sizes_around_the_rule_match_oracle(rt, orc, ctx, w, h, radius):
     img = np.random.default_rng(w * h).uniform(0, 1, (h, w, 4)).astype(np.float32)
     got = denoise(rt, ctx, img, float(radius), 1.0)
     want = orc.denoise(img, float(radius), 1.0, 0.1, 0.75)

@@ -80,7 +80,7 @@ __device__ __noinline__ void denoise_pixel(const float4 *__restrict__ in, int W,
   out[(size_t)py * W + px] = lerp4(c, f, p.mix);
 }
 
-// Radii above kTileRadius.
+// Radii above kTileRadius, and small images.
 __global__ void k_denoise(const float4 *__restrict__ in, int W, int H, DenoiseParams p, float4 *__restrict__ out) {
   const int px = blockIdx.x * blockDim.x + threadIdx.x, py = blockIdx.y * blockDim.y + threadIdx.y;
   if (px < W && py < H) denoise_pixel(in, W, H, p, px, py, out);
@@ -223,6 +223,8 @@ __global__ void __launch_bounds__(32 * kTileRows, 2) k_denoise_tile(const float4
   }
 }
 
+int g_sms = 0;
+
 }  // namespace
 
 cudaError_t launch_denoise(const float *in, uint32_t W, uint32_t H, float sigma, float ksigma, float threshold,
@@ -239,7 +241,19 @@ cudaError_t launch_denoise(const float *in, uint32_t W, uint32_t H, float sigma,
   p.inv_thr_sqrt2pi = kInvSqrt2Pi / threshold;
   p.mix = mix;
   const int radius = (int)p.radius;
-  if (radius <= kTileRadius) {
+  const dim3 pixels(16, 16), pixel_grid((W + 15) / 16, (H + 15) / 16);
+  // An image of at most a 16 x 16 block an SM (two, where a block has few taps)
+  // takes as long as one block, and the tile kernel's is longer. us, per pixel /
+  // tile: 200 x 150 (130 blocks) radius 2 10.3 / 12.3, 4 20.6 / 24.6, 8 65.8 /
+  // 71.8; 33 x 1080 (204) 12.3 / 12.2, 30.6 / 23.6, 98.4 / 71.7; radius 1 256 x
+  // 256 (256) 6.2 / 8.3, 384 x 256 (384) 8.2 / 8.3, 640 x 480 16.4 / 10.3.
+  if (g_sms == 0) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&g_sms, cudaDevAttrMultiProcessorCount, dev);
+  }
+  const uint64_t small = (uint64_t)g_sms * (radius <= 1 ? 2 : 1);
+  if (radius <= kTileRadius && (uint64_t)pixel_grid.x * pixel_grid.y > small) {
     int taps = 0;
     for (float x = -p.radius; x <= p.radius; x += 1.0f) {
       const float pt = std::sqrt(p.rad_q - x * x);
@@ -255,8 +269,7 @@ cudaError_t launch_denoise(const float *in, uint32_t W, uint32_t H, float sigma,
                                               reinterpret_cast<float4 *>(out));
     return cudaGetLastError();
   }
-  dim3 block(16, 16), grid((W + 15) / 16, (H + 15) / 16);
-  k_denoise<<<grid, block, 0, st>>>(reinterpret_cast<const float4 *>(in), (int)W, (int)H, p,
+  k_denoise<<<pixel_grid, pixels, 0, st>>>(reinterpret_cast<const float4 *>(in), (int)W, (int)H, p,
                                      reinterpret_cast<float4 *>(out));
   return cudaGetLastError();
 }
