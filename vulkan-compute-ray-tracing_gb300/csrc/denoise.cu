@@ -46,8 +46,8 @@ __device__ __forceinline__ float4 lerp4(float4 a, float4 b, float w) {
 }
 
 // One pixel, every tap fetched from the image.
-__device__ __noinline__ void denoise_pixel(const float4 *__restrict__ in, int W, int H, const DenoiseParams &p, int px,
-                                           int py, float4 *__restrict__ out) {
+__device__ __forceinline__ void denoise_pixel(const float4 *__restrict__ in, int W, int H, const DenoiseParams &p,
+                                              int px, int py, float4 *__restrict__ out) {
   const float4 c = in[(size_t)py * W + px];
   float z = 0.0f;
   float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -78,6 +78,12 @@ __device__ __noinline__ void denoise_pixel(const float4 *__restrict__ in, int W,
   }
   const float4 f = make_float4(__fdiv_rn(a.x, z), __fdiv_rn(a.y, z), __fdiv_rn(a.z, z), __fdiv_rn(a.w, z));
   out[(size_t)py * W + px] = lerp4(c, f, p.mix);
+}
+
+// As a call, for the tile kernel: its own loop keeps its registers.
+__device__ __noinline__ void denoise_pixel_call(const float4 *__restrict__ in, int W, int H, const DenoiseParams &p,
+                                                int px, int py, float4 *__restrict__ out) {
+  denoise_pixel(in, W, H, p, px, py, out);
 }
 
 // Radii above kTileRadius, and small images.
@@ -177,7 +183,7 @@ __global__ void __launch_bounds__(32 * kTileRows, 2) k_denoise_tile(const float4
   const int py = y0 + warp;
   if (!__syncthreads_and(finite)) {
     for (int px = x0 + lane; px < min(W, x0 + kTileCols); px += 32)
-      if (py < H) denoise_pixel(in, W, H, p, px, py, out);
+      if (py < H) denoise_pixel_call(in, W, H, p, px, py, out);
     return;
   }
   // This warp's row of the table.
