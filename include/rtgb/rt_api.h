@@ -283,6 +283,9 @@ rt_status rtTraceClosestHost(rt_ctx *ctx, rt_scene_id scene, const rt_ray *h_ray
  *                   an error bit in its device error word after the sort of
  *                   this tree level, as a sort overflow would, so the upload
  *                   must fail with RT_ERR_INTERNAL
+ *   "scene.test_stage_error"  test hook (default 0, off): 1 = the GPU check of
+ *                   a large scene's triangles ends as if memory had run out
+ *                   after its allocation; the host then checks them
  * Values persist for the context; rtAutotuneTrace / rtAutotuneRender write
  * them. Unknown keys return RT_ERR_INVALID_ARGUMENT. */
 rt_status rtSetTuning(rt_ctx *ctx, const char *key, int64_t value);

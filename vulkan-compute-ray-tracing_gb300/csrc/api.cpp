@@ -212,14 +212,28 @@ struct TriangleStage {
     std::memcpy(&f, &found.max_coord, 4);
     return f;
   }
-  cudaError_t load(rt_ctx *ctx, const rt_triangle *tris, uint32_t nt, const rt_material *mats, uint32_t nm) {
+  // Holds no memory after an error: what was found counts only after success.
+  cudaError_t load(rt_ctx *ctx, const rt_triangle *tris, uint32_t nt, const rt_material *mats, uint32_t nm,
+                   bool test_error) {
+    cudaError_t e = enqueue_and_read(ctx, tris, nt, mats, nm);
+    if (test_error) {
+      found = SceneCheck{};
+      e = cudaErrorMemoryAllocation;
+    }
+    if (e == cudaErrorMemoryAllocation) cudaGetLastError();
+    if (e != cudaSuccess) {
+      cudaStreamSynchronize(st);  // a copy may still read the caller's triangles
+      release();
+    }
+    return e;
+  }
+  cudaError_t enqueue_and_read(rt_ctx *ctx, const rt_triangle *tris, uint32_t nt, const rt_material *mats, uint32_t nm) {
     const size_t tri_bytes = align256(sizeof(rt_triangle) * (size_t)nt), mat_bytes = align256(sizeof(rt_material) * (size_t)nm);
     st = ctx->stream;
     cudaError_t e = cudaSetDevice(ctx->device);
     if (e == cudaSuccess) e = scratch_alloc((void **)&mem, tri_bytes + mat_bytes + 256 + 4ull * nt, ctx->pool, st);
     if (e != cudaSuccess) {
       mem = nullptr;
-      if (e == cudaErrorMemoryAllocation) cudaGetLastError();
       return e;
     }
     auto *d_tris = (rt_triangle *)mem;
@@ -426,7 +440,12 @@ rt_status rtUploadScene(rt_ctx *ctx, const rt_triangle *tris, uint32_t nt, const
   // for the message where a triangle is bad, here.
   TriangleStage stage;
   if (nt >= kStageMinTris) {
-    const cudaError_t se = stage.load(ctx, tris, nt, mats, nm);
+    bool test_error;
+    {
+      std::lock_guard<std::mutex> g(ctx->mu);
+      test_error = ctx->build_opts.test_stage_error != 0;
+    }
+    const cudaError_t se = stage.load(ctx, tris, nt, mats, nm, test_error);
     if (se != cudaSuccess && se != cudaErrorMemoryAllocation) return cuda_fail(ctx, se, "upload triangles");
   }
   const bool staged = stage.mem && !stage.found.bad;
@@ -1079,6 +1098,11 @@ rt_status rtSetTuning(rt_ctx *ctx, const char *key, int64_t value) {
     ctx->build_opts.collapse = (int)value;
     return RT_SUCCESS;
   }
+  if (k == "scene.test_stage_error") {
+    if (value < 0 || value > 1) return RT_ERR_INVALID_ARGUMENT;
+    ctx->build_opts.test_stage_error = (int)value;
+    return RT_SUCCESS;
+  }
   if (k == "bvh.test_error_level") {
     if (value < -1 || value > 64) return RT_ERR_INVALID_ARGUMENT;
     ctx->build_opts.test_error_level = (int)value;
@@ -1198,6 +1222,10 @@ rt_status rtGetTuning(rt_ctx *ctx, const char *key, int64_t *value) {
   }
   if (k == "bvh.ploc_radius") {
     *value = ctx->build_opts.ploc_radius;
+    return RT_SUCCESS;
+  }
+  if (k == "scene.test_stage_error") {
+    *value = ctx->build_opts.test_stage_error;
     return RT_SUCCESS;
   }
   if (k == "bvh.test_error_level") {

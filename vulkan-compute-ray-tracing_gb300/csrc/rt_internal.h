@@ -290,6 +290,7 @@ struct BuildOpts {
   // 14.4 / 5.1 ms, a 256 x 256 Cornell frame 1.27 / 0.80 ms.
   int cast_tree = 1;
   int test_error_level = -1;  // test hook of gpu_build_bvh's error word (-1: off)
+  int test_stage_error = 0;   // test hook: the GPU check of an upload's triangles runs out of memory
 };
 
 // One job of a batched render (render.cu: k_render_batch).
