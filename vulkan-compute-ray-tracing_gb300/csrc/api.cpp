@@ -917,12 +917,14 @@ rt_status rtRender(rt_ctx *ctx, rt_scene_id id, const rt_render_params *p, float
     ropts = ctx->render_opts;
     topts = ctx->trace_opts;
   }
-  // A call of several samples of a small image is a wavefront only where its
-  // scratch can be had and the stream is not being captured (a graph would
-  // get memory nodes it did not have as one launch); else one launch.
+  // A call of several samples of a small image is a wavefront, and one of one
+  // sample a launch of paths.cu, only where its scratch can be had and the
+  // stream is not being captured (a graph would get memory nodes it did not
+  // have as one launch); else the megakernel, which needs none.
   const bool small = ropts.mode == 2 && (uint64_t)p->width * p->height < ropts.wavefront_pixels;
+  const bool paths = ropts.mode >= 2 && use_wide(topts, d) && paths_ok(d, *p);
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-  if (small && p->spp > 1) CK(cudaStreamIsCapturing(st, &capture), "capture status");
+  if ((small && p->spp > 1) || paths) CK(cudaStreamIsCapturing(st, &capture), "capture status");
   if (use_wavefront(ropts, *p) && !(small && capture != cudaStreamCaptureStatusNone)) {
     void *scratch = nullptr;
     cudaError_t e = scratch_alloc(&scratch, wavefront_scratch_bytes(*p, ropts.sort != 0), ctx->pool, st);
@@ -936,11 +938,19 @@ rt_status rtRender(rt_ctx *ctx, rt_scene_id id, const rt_render_params *p, float
     if (!small || e != cudaErrorMemoryAllocation) return cuda_fail(ctx, e, "wavefront scratch");
     cudaGetLastError();
   }
-  if (ropts.mode >= 2 && use_wide(topts, d) && paths_ok(d, *p)) {
-    const cudaError_t e =
-        launch_render_paths(d, cam, *p, accum, ctx->d_segments, next_counter(ctx), ctx->d_err, st);
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "render launch");
-    return RT_SUCCESS;
+  if (paths && capture == cudaStreamCaptureStatusNone) {
+    // The work counter is this call's own: a word of the context's ring could
+    // be a later call's too, in a replayed graph or on a stream held back.
+    uint32_t *counter = nullptr;
+    cudaError_t e = scratch_alloc((void **)&counter, 4, ctx->pool, st);
+    if (e == cudaSuccess) {
+      e = launch_render_paths(d, cam, *p, accum, ctx->d_segments, counter, ctx->d_err, st);
+      cudaFreeAsync(counter, st);
+      if (e != cudaSuccess) return cuda_fail(ctx, e, "render launch");
+      return RT_SUCCESS;
+    }
+    if (e != cudaErrorMemoryAllocation) return cuda_fail(ctx, e, "path counter");
+    cudaGetLastError();
   }
   cudaError_t e = launch_render(d, cam, *p, accum, ctx->d_segments, ctx->d_err, st);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "render launch");
