@@ -283,6 +283,8 @@ rt_status rtTraceClosestHost(rt_ctx *ctx, rt_scene_id scene, const rt_ray *h_ray
  *                   an error bit in its device error word after the sort of
  *                   this tree level, as a sort overflow would, so the upload
  *                   must fail with RT_ERR_INTERNAL
+ *   "test.alloc_limit"  test hook (default 0, off): the context's device
+ *                   allocations above this many bytes fail as on a full device
  *   "scene.test_stage_error"  test hook (default 0, off): 1 = the GPU check of
  *                   a large scene's triangles ends as if memory had run out
  *                   after its allocation; the host then checks them

@@ -50,3 +50,28 @@ def test_a_check_that_runs_out_of_memory_leaves_the_hosts(rt, ctx, tune, n):
         assert len(want) and np.array_equal(sc.lights().view(np.uint32), want.view(np.uint32))
     finally:
         sc.release()
+
+
+@pytest.mark.parametrize("spp", [1, 3])
+@pytest.mark.parametrize("side", [48, 256, 362, 363, 400, 511])
+def test_renders_without_scratch_are_one_launch(rt, ctx, tune, side, spp):
+    import torch
+    tris, mats, _ = rt.gen_cornell(8, 1500)
+    sc = ctx.upload_scene(tris, mats)
+    try:
+        sc.set_camera(rt.camera_look_at([0.2, 0.1, -14], [0, 0, 0], [0, 1, 0], 40.0, side, side))
+        images = []
+        for limit in (0, 1):
+            tune(test__alloc_limit=limit)
+            img = torch.zeros((side, side, 4), device="cuda")
+            torch.cuda.synchronize()
+            sc.render(img, side, side, spp, 5)
+            ctx.synchronize()
+            images.append(img)
+        assert torch.equal(images[0], images[1])
+        big = torch.zeros((512, 512, 4), device="cuda")
+        with pytest.raises(rt.RtError):  # from 2^18 pixels the scratch is a condition
+            sc.render(big, 512, 512, spp, 5)
+    finally:
+        tune(test__alloc_limit=0)
+        sc.release()

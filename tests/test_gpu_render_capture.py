@@ -1,6 +1,8 @@
 """Renders of small images in captured graphs and on several streams: every
 image bit for bit, whatever else is under way, and no memory of a graph's own
 where the call was one launch."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -21,6 +23,44 @@ def captured(sc, image, width, height, **kw):
     with torch.cuda.graph(g, stream=s):
         sc.render(image, width, height, stream=s.cuda_stream, **kw)
     return g
+
+
+def node_types(graph):
+    """The kinds of the graph's nodes (CUgraphNodeType)."""
+    drv = ctypes.CDLL("libcuda.so.1")
+    g, n = ctypes.c_void_p(graph.raw_cuda_graph()), ctypes.c_size_t(0)
+    assert drv.cuGraphGetNodes(g, None, ctypes.byref(n)) == 0
+    nodes = (ctypes.c_void_p * n.value)()
+    assert drv.cuGraphGetNodes(g, nodes, ctypes.byref(n)) == 0
+    out = []
+    for node in nodes:
+        t = ctypes.c_int(-1)
+        assert drv.cuGraphNodeGetType(ctypes.c_void_p(node), ctypes.byref(t)) == 0
+        out.append(t.value)
+    return out
+
+
+KERNEL, MEM_ALLOC, MEM_FREE = 0, 10, 11
+
+
+@pytest.mark.parametrize("spp", [1, 3])
+@pytest.mark.parametrize("side", [64, 256, 362, 363, 400, 511])
+def test_captured_renders_are_one_launch(rt, ctx, side, spp):
+    import torch
+    sc = scene(rt, ctx, side=side)
+    try:
+        image, want = torch.zeros((side, side, 4), device="cuda"), torch.zeros((side, side, 4), device="cuda")
+        g = captured(sc, image, side, side, spp=spp, max_bounces=5)
+        types = node_types(g)
+        assert MEM_ALLOC not in types and MEM_FREE not in types and types.count(KERNEL) == 1
+        g.instantiate()
+        g.replay()
+        torch.cuda.synchronize()
+        sc.render(want, side, side, spp, 5)
+        ctx.synchronize()
+        assert torch.equal(image, want)
+    finally:
+        sc.release()
 
 
 def test_replays_and_live_calls_keep_their_own_counters(rt, ctx):

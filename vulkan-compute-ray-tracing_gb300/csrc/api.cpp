@@ -62,7 +62,7 @@ struct rt_ctx {
   // keeps up to kPoolKeep of it over synchronisations (the default pool gives
   // everything back: 0.13 ms a call, and 0.7 of a 1.31M-triangle upload); the rest
   // goes back at once, all of it with the context or when memory runs out.
-  cudaMemPool_t pool = nullptr;
+  ScratchPool pool;
   std::mutex mu;
   std::unordered_map<uint32_t, Scene *> scenes;
   uint32_t next_id = 1;
@@ -307,9 +307,9 @@ rt_status rtCreate(rt_ctx **out, const rt_ctx_desc *desc) {
     props.allocType = cudaMemAllocationTypePinned;
     props.location.type = cudaMemLocationTypeDevice;
     props.location.id = ctx->device;
-    e = cudaMemPoolCreate(&ctx->pool, &props);
+    e = cudaMemPoolCreate(&ctx->pool.pool, &props);
     uint64_t keep = kPoolKeep;
-    if (e == cudaSuccess) e = cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    if (e == cudaSuccess) e = cudaMemPoolSetAttribute(ctx->pool.pool, cudaMemPoolAttrReleaseThreshold, &keep);
   }
   if (e == cudaSuccess) e = cudaMalloc((void **)&ctx->d_err, 64);
   if (e == cudaSuccess) e = cudaMemset(ctx->d_err, 0, 64);
@@ -347,7 +347,7 @@ rt_status rtDestroy(rt_ctx *ctx) {
   if (ctx->d_counters) cudaFree(ctx->d_counters);
   if (ctx->d_segments) cudaFree(ctx->d_segments);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
-  if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
+  if (ctx->pool.pool) cudaMemPoolDestroy(ctx->pool.pool);
   delete ctx;
   return RT_SUCCESS;
 }
@@ -917,14 +917,14 @@ rt_status rtRender(rt_ctx *ctx, rt_scene_id id, const rt_render_params *p, float
     ropts = ctx->render_opts;
     topts = ctx->trace_opts;
   }
-  // A call of several samples of a small image is a wavefront, and one of one
-  // sample a launch of paths.cu, only where its scratch can be had and the
-  // stream is not being captured (a graph would get memory nodes it did not
-  // have as one launch); else the megakernel, which needs none.
-  const bool small = ropts.mode == 2 && (uint64_t)p->width * p->height < ropts.wavefront_pixels;
+  // Below kOneLaunchPixels a call is a wavefront or a launch of paths.cu only
+  // where its scratch can be had and the stream is not being captured (a graph
+  // with memory nodes cannot run twice at once); else the megakernel, which
+  // needs no memory.
+  const bool small = ropts.mode >= 2 && (uint64_t)p->width * p->height < std::max(kOneLaunchPixels, ropts.wavefront_pixels);
   const bool paths = ropts.mode >= 2 && use_wide(topts, d) && paths_ok(d, *p);
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-  if ((small && p->spp > 1) || paths) CK(cudaStreamIsCapturing(st, &capture), "capture status");
+  if (small) CK(cudaStreamIsCapturing(st, &capture), "capture status");
   if (use_wavefront(ropts, *p) && !(small && capture != cudaStreamCaptureStatusNone)) {
     void *scratch = nullptr;
     cudaError_t e = scratch_alloc(&scratch, wavefront_scratch_bytes(*p, ropts.sort != 0), ctx->pool, st);
@@ -1108,6 +1108,11 @@ rt_status rtSetTuning(rt_ctx *ctx, const char *key, int64_t value) {
     ctx->build_opts.collapse = (int)value;
     return RT_SUCCESS;
   }
+  if (k == "test.alloc_limit") {
+    if (value < 0) return RT_ERR_INVALID_ARGUMENT;
+    ctx->pool.test_limit.store((uint64_t)value);
+    return RT_SUCCESS;
+  }
   if (k == "scene.test_stage_error") {
     if (value < 0 || value > 1) return RT_ERR_INVALID_ARGUMENT;
     ctx->build_opts.test_stage_error = (int)value;
@@ -1234,6 +1239,10 @@ rt_status rtGetTuning(rt_ctx *ctx, const char *key, int64_t *value) {
     *value = ctx->build_opts.ploc_radius;
     return RT_SUCCESS;
   }
+  if (k == "test.alloc_limit") {
+    *value = (int64_t)ctx->pool.test_limit.load();
+    return RT_SUCCESS;
+  }
   if (k == "scene.test_stage_error") {
     *value = ctx->build_opts.test_stage_error;
     return RT_SUCCESS;
@@ -1287,10 +1296,11 @@ rt_status rtSynchronize(rt_ctx *ctx, void *stream) {
 namespace rtgb {
 
 cudaError_t ctx_malloc(rt_ctx *ctx, void **p, size_t bytes) {
+  if (ctx->pool.test_full(bytes)) return cudaErrorMemoryAllocation;
   cudaError_t e = cudaMalloc(p, bytes);
   if (e == cudaErrorMemoryAllocation) {
     cudaGetLastError();
-    cudaMemPoolTrimTo(ctx->pool, 0);
+    cudaMemPoolTrimTo(ctx->pool.pool, 0);
     e = cudaMalloc(p, bytes);
   }
   return e;

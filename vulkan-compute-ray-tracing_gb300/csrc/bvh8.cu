@@ -542,7 +542,7 @@ cudaError_t collapse_choices(const DevScene &d, uint32_t *scr, uint32_t *choice,
 }  // namespace
 
 cudaError_t build_bvh8(const DevScene &d, bool sah, void *bvh8q, uint32_t cap, uint32_t *n8_out,
-                       uint32_t *levels_out, int32_t *root_out, char *errbuf, size_t errlen, cudaMemPool_t pool,
+                       uint32_t *levels_out, int32_t *root_out, char *errbuf, size_t errlen, ScratchPool &pool,
                        cudaStream_t st) {
   *n8_out = 0;
   *levels_out = 0;

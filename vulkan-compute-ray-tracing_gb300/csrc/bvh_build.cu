@@ -965,7 +965,7 @@ cudaError_t enqueue_build(const rt_triangle *d_tris, uint32_t n, const BuildScra
 }  // namespace
 
 rt_status gpu_build_bvh(const rt_triangle *d_tris, uint32_t n, uint32_t bvh_seed, rt_bvh_node *d_nodes,
-                        cudaMemPool_t pool, cudaStream_t st, float *ms_out, uint32_t *depth_out, char *errbuf,
+                        ScratchPool &pool, cudaStream_t st, float *ms_out, uint32_t *depth_out, char *errbuf,
                         size_t errlen, int test_error_level) {
   rt_status status = RT_SUCCESS;
   unsigned char *mem = nullptr;

@@ -337,7 +337,7 @@ cudaError_t lbvh_sorted_keys(const rt_triangle *d_tris, uint32_t n, uint32_t *sc
   return e;
 }
 
-rt_status gpu_build_lbvh(const rt_triangle *d_tris, uint32_t n, rt_bvh_node *d_nodes, cudaMemPool_t pool,
+rt_status gpu_build_lbvh(const rt_triangle *d_tris, uint32_t n, rt_bvh_node *d_nodes, ScratchPool &pool,
                          cudaStream_t st, float *ms_out, uint32_t *depth_out, char *errbuf, size_t errlen) {
   if (n == 0) return RT_ERR_INVALID_ARGUMENT;
   cudaEvent_t e0 = nullptr, e1 = nullptr;

@@ -299,7 +299,7 @@ __global__ void __launch_bounds__(kPlocThreads) k_ploc(const rt_triangle *__rest
 }  // namespace
 
 rt_status gpu_build_ploc(const rt_triangle *d_tris, uint32_t n, uint32_t radius, uint32_t max_rounds,
-                         rt_bvh_node *d_nodes, cudaMemPool_t pool, cudaStream_t st, float *ms_out,
+                         rt_bvh_node *d_nodes, ScratchPool &pool, cudaStream_t st, float *ms_out,
                          uint32_t *depth_out, char *errbuf, size_t errlen) {
   if (n == 0 || radius < 1 || radius > kMaxRadius) return RT_ERR_INVALID_ARGUMENT;
   int dev = 0, sms = 0, per_sm = 0;

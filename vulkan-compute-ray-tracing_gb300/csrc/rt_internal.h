@@ -4,19 +4,32 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "rtgb/rt_api.h"
 #include "rtgb/rt_types.h"
 
 namespace rtgb {
 
-// Stream-ordered scratch from a context's own memory pool (api.cpp). When the
-// device is full, the pool's unused memory is given back and the call made again.
-inline cudaError_t scratch_alloc(void **p, size_t bytes, cudaMemPool_t pool, cudaStream_t st) {
-  cudaError_t e = cudaMallocFromPoolAsync(p, bytes, pool, st);
+// A context's own memory pool (api.cpp).
+struct ScratchPool {
+  cudaMemPool_t pool = nullptr;
+  std::atomic<uint64_t> test_limit{0};  // test hook: larger allocations fail as on a full device (0: off)
+  bool test_full(size_t bytes) const {
+    const uint64_t limit = test_limit.load(std::memory_order_relaxed);
+    return limit && bytes > limit;
+  }
+};
+
+// Stream-ordered scratch from the pool. When the device is full, the pool's
+// unused memory is given back and the call made again.
+inline cudaError_t scratch_alloc(void **p, size_t bytes, ScratchPool &pool, cudaStream_t st) {
+  if (pool.test_full(bytes)) return cudaErrorMemoryAllocation;
+  cudaError_t e = cudaMallocFromPoolAsync(p, bytes, pool.pool, st);
   if (e == cudaErrorMemoryAllocation) {
     cudaGetLastError();
-    cudaMemPoolTrimTo(pool, 0);
-    e = cudaMallocFromPoolAsync(p, bytes, pool, st);
+    cudaMemPoolTrimTo(pool.pool, 0);
+    e = cudaMallocFromPoolAsync(p, bytes, pool.pool, st);
   }
   return e;
 }
@@ -83,7 +96,7 @@ uint32_t bvh8_capacity(uint32_t ntris);
 // first; synchronises `st`.
 constexpr size_t kBvh8NodeBytes = 96;
 cudaError_t build_bvh8(const DevScene &d, bool sah, void *bvh8q, uint32_t cap, uint32_t *n8_out,
-                       uint32_t *levels_out, int32_t *root_out, char *errbuf, size_t errlen, cudaMemPool_t pool,
+                       uint32_t *levels_out, int32_t *root_out, char *errbuf, size_t errlen, ScratchPool &pool,
                        cudaStream_t st);
 
 // ---------------------------------------------------------------- relayout.cu
@@ -234,6 +247,12 @@ cudaError_t launch_render_wavefront(const DevScene &sc, const rt_camera &cam, co
                                     unsigned long long *segments, uint32_t *err, void *scratch, bool sort, bool wide,
                                     cudaStream_t st, const uint32_t *d_sample_index = nullptr, bool alone = false);
 
+// Renders of fewer pixels can fall back from a form that takes scratch to the
+// megakernel in one launch: a fixed size, whatever the tuning. From here up the
+// wavefront is the faster form of every call by so much that its scratch is a
+// condition (1024 x 1024, 12K triangles, 4 samples: 546 / 837 Mrays/s).
+constexpr uint64_t kOneLaunchPixels = 1u << 18;
+
 // Render launch-shape knobs (rtSetTuning "render.mode").
 struct RenderOpts {
   int mode = 2;  // 0 megakernel, 1 wavefront, 2 choose by image size, 3 choose, without the wavefront
@@ -317,7 +336,7 @@ cudaError_t launch_batch_advance(BatchJob *d_jobs, uint32_t n_jobs, cudaStream_t
 // error bit after that level's sort, as an overflow would; the build must
 // then fail with RT_ERR_INTERNAL.
 rt_status gpu_build_bvh(const rt_triangle *d_tris, uint32_t n, uint32_t bvh_seed, rt_bvh_node *d_nodes,
-                        cudaMemPool_t pool, cudaStream_t st, float *ms_out, uint32_t *depth_out, char *errbuf,
+                        ScratchPool &pool, cudaStream_t st, float *ms_out, uint32_t *depth_out, char *errbuf,
                         size_t errlen, int test_error_level = -1);
 
 // ---------------------------------------------------------------- export.cu
@@ -358,7 +377,7 @@ cudaError_t launch_check_scene(const rt_triangle *tris, uint32_t n, const rt_mat
 // ---------------------------------------------------------------- lbvh.cu
 // A linear BVH (Morton order) in the Bvh.h node layout; not the reference's
 // tree — a separately reported traversal mode.
-rt_status gpu_build_lbvh(const rt_triangle *d_tris, uint32_t n, rt_bvh_node *d_nodes, cudaMemPool_t pool,
+rt_status gpu_build_lbvh(const rt_triangle *d_tris, uint32_t n, rt_bvh_node *d_nodes, ScratchPool &pool,
                          cudaStream_t st, float *ms_out, uint32_t *depth_out, char *errbuf, size_t errlen);
 // Morton-sorted triangle centroids (lbvh.cu), shared by the LBVH and PLOC builders.
 size_t lbvh_sorted_keys_words(uint32_t n);
@@ -368,7 +387,7 @@ cudaError_t lbvh_sorted_keys(const rt_triangle *d_tris, uint32_t n, uint32_t *sc
 // nearest neighbours searched within `radius` (1..256) positions. Fails with
 // RT_ERR_INTERNAL when max_rounds rounds leave more than one cluster.
 rt_status gpu_build_ploc(const rt_triangle *d_tris, uint32_t n, uint32_t radius, uint32_t max_rounds,
-                         rt_bvh_node *d_nodes, cudaMemPool_t pool, cudaStream_t st, float *ms_out,
+                         rt_bvh_node *d_nodes, ScratchPool &pool, cudaStream_t st, float *ms_out,
                          uint32_t *depth_out, char *errbuf, size_t errlen);
 
 // ---------------------------------------------------------------- glibc_rand.cpp
