@@ -240,8 +240,10 @@ rt_status rtTraceClosestHost(rt_ctx *ctx, rt_scene_id scene, const rt_ray *h_ray
  *                   one launch whose warps follow a few paths each; 3 the
  *                   same without the wavefront;
  *                   images are identical in every mode
- *   "render.wavefront_pixels"  the mode-2 threshold of rtRender for calls of
- *                   one sample (default 2^17 pixels: 363 x 363 and up)
+ *   "render.wavefront_pixels"  the mode-2 threshold of rtRender: at the
+ *                   default, 2^17 (363 x 363), that of calls of one sample,
+ *                   calls of more being wavefronts at every size; any other
+ *                   value, of calls of any number of samples (2^31: never)
  *   "render.batch_wavefront_pixels"  the split of batches and of the
  *                   render server's steps: jobs from this many pixels up run
  *                   as wavefronts side by side on side streams, the rest in
@@ -303,11 +305,11 @@ rt_status rtGetTuning(rt_ctx *ctx, const char *key, int64_t *value);
  * are returned in Grays/s (either pointer may be NULL). Synchronous. */
 rt_status rtAutotuneTrace(rt_ctx *ctx, rt_scene_id scene, const rt_ray *d_rays, uint32_t n, rt_hit *d_hits,
                           uint32_t reps, double *start_grays, double *best_grays);
-/* Times megakernel against wavefront renders of the scene (its current
- * camera; max_bounces; one sample, as calls of more samples run as
- * wavefronts at every size) at square sizes 256, 512, ... up to max_side
- * (256..4096) and sets render.wavefront_pixels to the smallest size from
- * which the wavefront is faster (2^31 when it never is). Images
+/* Times renders of the scene without the wavefront (render.mode 3) against
+ * wavefront renders (its current camera; spp samples, max_bounces) at square
+ * sizes 256, 512, ... up to max_side (256..4096) and sets
+ * render.wavefront_pixels, for calls of any number of samples, to the smallest
+ * size from which the wavefront is faster (2^31 when it never is). Images
  * are identical either way. Synchronous; allocates one image of max_side^2
  * pixels for the duration of the call. */
 rt_status rtAutotuneRender(rt_ctx *ctx, rt_scene_id scene, uint32_t spp, uint32_t max_bounces, uint32_t max_side,

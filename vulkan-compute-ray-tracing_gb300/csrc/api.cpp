@@ -921,7 +921,7 @@ rt_status rtRender(rt_ctx *ctx, rt_scene_id id, const rt_render_params *p, float
   // where its scratch can be had and the stream is not being captured (a graph
   // with memory nodes cannot run twice at once); else the megakernel, which
   // needs no memory.
-  const bool small = ropts.mode >= 2 && (uint64_t)p->width * p->height < std::max(kOneLaunchPixels, ropts.wavefront_pixels);
+  const bool small = one_launch_fallback(ropts, *p);
   const bool paths = ropts.mode >= 2 && use_wide(topts, d) && paths_ok(d, *p);
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
   if (small) CK(cudaStreamIsCapturing(st, &capture), "capture status");

@@ -140,13 +140,12 @@ rt_status rtAutotuneRender(rt_ctx *ctx, rt_scene_id scene, uint32_t spp, uint32_
   cudaError_t e = cudaMalloc((void **)&accum, 16ull * max_side * max_side);
   if (e != cudaSuccess) return e == cudaErrorMemoryAllocation ? RT_ERR_OUT_OF_MEMORY : RT_ERR_CUDA;
   // Smallest size from which the wavefront wins; 2^31 when it never does.
-  // One sample a call: calls of more run as wavefronts at every size.
   int64_t threshold = 1ll << 31;
   for (uint32_t side = 256; side <= max_side && s == RT_SUCCESS; side *= 2) {
     float ms[2] = {0.0f, 0.0f};
     for (int mode = 0; mode < 2 && s == RT_SUCCESS; mode++) {
       s = rtSetTuning(ctx, "render.mode", mode ? 1 : 3);
-      if (s == RT_SUCCESS) s = time_render(ctx, scene, side, 1, max_bounces, accum, &ms[mode]);
+      if (s == RT_SUCCESS) s = time_render(ctx, scene, side, spp, max_bounces, accum, &ms[mode]);
     }
     if (s == RT_SUCCESS && ms[1] < ms[0]) {
       threshold = (int64_t)side * side;

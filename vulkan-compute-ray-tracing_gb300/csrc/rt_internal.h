@@ -9,6 +9,8 @@
 #include "rtgb/rt_api.h"
 #include "rtgb/rt_types.h"
 
+#include "routes.h"
+
 namespace rtgb {
 
 // A context's own memory pool (api.cpp).
@@ -246,54 +248,6 @@ size_t wavefront_scratch_bytes(const rt_render_params &p, bool sort);
 cudaError_t launch_render_wavefront(const DevScene &sc, const rt_camera &cam, const rt_render_params &p, float *accum,
                                     unsigned long long *segments, uint32_t *err, void *scratch, bool sort, bool wide,
                                     cudaStream_t st, const uint32_t *d_sample_index = nullptr, bool alone = false);
-
-// Renders of fewer pixels can fall back from a form that takes scratch to the
-// megakernel in one launch: a fixed size, whatever the tuning. From here up the
-// wavefront is the faster form of every call by so much that its scratch is a
-// condition (1024 x 1024, 12K triangles, 4 samples: 546 / 837 Mrays/s).
-constexpr uint64_t kOneLaunchPixels = 1u << 18;
-
-// Render launch-shape knobs (rtSetTuning "render.mode").
-struct RenderOpts {
-  int mode = 2;  // 0 megakernel, 1 wavefront, 2 choose by image size, 3 choose, without the wavefront
-  // mode 2: calls of one sample run as a wavefront from this many pixels up
-  // (below, paths.cu up to 65,536 and the megakernel between), calls of
-  // several samples always: the samples share a wave, where the megakernel's
-  // threads run them one after the other. Megakernel / wavefront, Cornell box
-  // of 1K, 12K, 100K triangles, mesh of 512K, 8 bounces, 1 sample, us: 288 x
-  // 288 386 / 409, 1005 / 843, 1752 / 1497, 800 / 589; 352 x 352 459 / 458,
-  // 1256 / 950, 2367 / 1664, 967 / 677; 511 x 512 842 / 573, 2285 / 1334, 3920
-  // / 2238, 1300 / 806. 4 samples, 12K: 48 x 48 2354 / 983, 512 x 512 8897 /
-  // 4344.
-  uint64_t wavefront_pixels = 1u << 17;
-  int batch_streams = 16;                // side streams a batch spreads its wavefront jobs over (1..16)
-  // Batches and the render server: jobs from this many pixels up run as
-  // wavefronts on side streams (the rest in the persistent tile launch).
-  // Jobs that run side by side keep the GPU busy at any size, and queued
-  // bounce rays in the 8-wide caster beat the megakernel's diverged lanes,
-  // so all of them do by default; a render alone keeps wavefront_pixels.
-  uint64_t batch_wavefront_pixels = 1;
-  // Wavefront renders: reorder each bounce's rays by Morton key of origin and
-  // direction before casting them (1) or cast them in queue order (0). The
-  // queue keeps the shading warps' order, which is close to the camera
-  // tiles' order, and the 8-wide caster takes them faster unsorted; the
-  // closest-hit entry points keep trace.sort.
-  int sort = 0;
-};
-// True when a render of these params goes to the wavefront kernels.
-inline bool use_wavefront(const RenderOpts &o, const rt_render_params &p) {
-  if (p.flags & RT_COMPAT_STACK16) return false;  // the literal 16-entry traversal is megakernel-only
-  const uint64_t pixels = (uint64_t)p.width * p.height;
-  return pixels < (1ull << 31) && (o.mode == 1 || (o.mode == 2 && (p.spp > 1 || pixels >= o.wavefront_pixels)));
-}
-// True when a job of a batch or a server step goes to the wavefront kernels.
-inline bool use_wavefront_batched(const RenderOpts &o, const rt_render_params &p) {
-  rt_render_params one = p;
-  one.spp = 1;
-  RenderOpts b = o;
-  b.wavefront_pixels = o.batch_wavefront_pixels;
-  return use_wavefront(b, one);
-}
 
 // Tree used when a scene is uploaded without nodes (rtSetTuning "bvh.builder").
 struct BuildOpts {
