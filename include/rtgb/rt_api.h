@@ -235,15 +235,18 @@ rt_status rtTraceClosestHost(rt_ctx *ctx, rt_scene_id scene, const rt_ray *h_ray
  *                   reported as RT_ERR_STACK_OVERFLOW)
  *   "render.mode"   0 megakernel (one thread runs a pixel's whole path),
  *                   1 wavefront (per-bounce kernels over compacted queues),
- *                   2 (default) wavefront for calls of several samples and
- *                   from render.wavefront_pixels up, and up to 65,536 pixels
- *                   one launch whose warps follow a few paths each; 3 the
- *                   same without the wavefront;
+ *                   2 (default) by sizes: wavefront from 2^18 pixels up, and
+ *                   below for calls of several samples and from
+ *                   render.wavefront_pixels up, where triangles or samples are
+ *                   many enough; up to 65,536 pixels of one sample one launch
+ *                   whose warps follow a few paths each; else the megakernel,
+ *                   also where a smaller call cannot have scratch or its
+ *                   stream is captured; 3 the same without the wavefront;
  *                   images are identical in every mode
  *   "render.wavefront_pixels"  the mode-2 threshold of rtRender: at the
- *                   default, 2^17 (363 x 363), that of calls of one sample,
- *                   calls of more being wavefronts at every size; any other
- *                   value, of calls of any number of samples (2^31: never)
+ *                   default, 2^17 (363 x 363), that of calls of one sample;
+ *                   any other value, of calls of any number of samples and
+ *                   scenes of any size (2^31: never)
  *   "render.batch_wavefront_pixels"  the split of batches and of the
  *                   render server's steps: jobs from this many pixels up run
  *                   as wavefronts side by side on side streams, the rest in
@@ -269,10 +272,10 @@ rt_status rtTraceClosestHost(rt_ctx *ctx, rt_scene_id scene, const rt_ray *h_ray
  *                   tree built beside the reference's, whose tighter boxes
  *                   they cross faster; 0 = on the reference's own. The hits
  *                   are identical; rtDownloadBvh and the 16-entry compat
- *                   traversal read the reference's nodes either way. A tree
- *                   deeper than 64 levels, no memory for its scratch, or a
- *                   vertex coordinate above 1024 in magnitude leaves the
- *                   casts on the reference's
+ *                   traversal read the reference's nodes either way. Fewer
+ *                   than 32 triangles, a tree deeper than 64 levels, no memory
+ *                   for its scratch, or a vertex coordinate above 1024 in
+ *                   magnitude leaves the casts on the reference's
  *   "bvh.ploc_radius"  positions on either side the PLOC builder
  *                   (bvh.builder 2, bvh.cast_tree 1) searches for nearest
  *                   neighbours, 1..256 (default 16)

@@ -26,6 +26,10 @@ namespace {
 constexpr uint32_t kCounterRing = 1024;
 constexpr uint64_t kPoolKeep = 1ull << 30;  // scratch a context keeps (an upload of 1.31M triangles takes half)
 constexpr uint32_t kMaxTreeDepth = 64;     // the traversal stacks' largest size
+// Below, the reference's tree is as quick to cast on: us a frame of 256 x 256, 8
+// bounces, on the reference's / on PLOC: 12 triangles (a bare Cornell box) 65 /
+// 70, 32 89 / 85.
+constexpr uint32_t kCastTreeMinTris = 32;
 constexpr uint32_t kCastTreeRounds = 512;  // a PLOC tree of 64 levels takes fewer
 // A triangle whose fp32 t errs by more than the boxes' padding (1e-4) can be
 // found in one visiting order and pruned in another, so that a hit would
@@ -583,7 +587,7 @@ rt_status rtUploadScene(rt_ctx *ctx, const rt_triangle *tris, uint32_t nt, const
     // the boxes nest so that it grows too deep for the traversal stacks, they
     // are cast on the reference's; also where coordinates are so large that
     // an fp32 rounding nears the boxes' padding (kCastTreeMaxCoord).
-    if (builder == 0 && cast_tree && nt > 2 && max_coord <= kCastTreeMaxCoord) {
+    if (builder == 0 && cast_tree && nt >= kCastTreeMinTris && max_coord <= kCastTreeMaxCoord) {
       const cudaError_t ce = scratch_alloc((void **)&cast_scratch, sizeof(rt_bvh_node) * nnodes, ctx->pool, st);
       uint32_t cast_depth = 0;
       if (ce != cudaSuccess) {
@@ -925,7 +929,7 @@ rt_status rtRender(rt_ctx *ctx, rt_scene_id id, const rt_render_params *p, float
   const bool paths = ropts.mode >= 2 && use_wide(topts, d) && paths_ok(d, *p);
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
   if (small) CK(cudaStreamIsCapturing(st, &capture), "capture status");
-  if (use_wavefront(ropts, *p) && !(small && capture != cudaStreamCaptureStatusNone)) {
+  if (use_wavefront(ropts, d.ntris, *p) && !(small && capture != cudaStreamCaptureStatusNone)) {
     void *scratch = nullptr;
     cudaError_t e = scratch_alloc(&scratch, wavefront_scratch_bytes(*p, ropts.sort != 0), ctx->pool, st);
     if (e == cudaSuccess) {

@@ -27,7 +27,6 @@ namespace rtgb {
 namespace {
 
 constexpr int kShadeAt = 4, kClaimAt = 2;
-constexpr uint64_t kPathsMaxPixels = 1u << 16;  // above, the megakernel up to the wavefront's sizes
 
 template <int R>
 struct PathsWarp {
@@ -141,8 +140,7 @@ cudaError_t go(const DevScene &sc, const rt_camera &cam, const rt_render_params 
 }  // namespace
 
 bool paths_ok(const DevScene &sc, const rt_render_params &p) {
-  return wide_ok(sc) && p.spp == 1 && p.max_bounces > 0 && !(p.flags & RT_COMPAT_STACK16) &&
-         (uint64_t)p.width * p.height <= kPathsMaxPixels;
+  return wide_ok(sc) && p.spp == 1 && p.max_bounces > 0 && !(p.flags & RT_COMPAT_STACK16) && paths_fit(sc.ntris, p);
 }
 
 cudaError_t launch_render_paths(const DevScene &sc, const rt_camera &cam, const rt_render_params &p, float *accum,

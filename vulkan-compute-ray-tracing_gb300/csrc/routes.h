@@ -15,20 +15,65 @@ namespace rtgb {
 // condition (1024 x 1024, 12K triangles, 4 samples: 546 / 837 Mrays/s).
 constexpr uint64_t kOneLaunchPixels = 1u << 18;
 
+// Calls of several samples below that size run as a wavefront from this many
+// samples up (~0: never), else as the megakernel. A wavefront runs the samples
+// side by side, where the megakernel's threads run them one after the other,
+// but pays three launches a bounce (about 15 us) whether paths are left or not:
+// it wants triangles enough to make a path's steps dear, or samples enough, the
+// more the longer the paths may be and the fewer triangles there are. us,
+// megakernel / wavefront, 256 x 256, 8 bounces: Cornell box of 12 triangles, 2
+// samples 119 / 219, 16 (128 x 128) 655 / 257; of 312, 2 samples 292 / 346, 8
+// and 4 bounces with 4 samples 587 / 423 and 304 / 246; of 1K, 2 samples 495 /
+// 456; of 12K 1488 / 912; an icosphere in the open of 320, 2 samples 93 / 193, 4
+// (4 bounces) 109 / 128, 8 (128 x 128) 213 / 197; of 5120, 2 samples 284 / 288.
+// One bounce, 2 samples: 1K 32 / 44, 16 x 16 91 / 35, 12K 84 / 90. Of images of
+// few pixels, or narrower than a tile of 8 x 4, most lanes are idle: 4096 x 1, 2
+// samples, 12K 24 / 139, 100K 375 / 232.
+inline uint64_t wave_min_samples(uint32_t ntris, const rt_render_params &p) {
+  const uint64_t pixels = (uint64_t)p.width * p.height, bounces = p.max_bounces, never = ~0ull;
+  if (pixels < 64 || (p.height < 4 && ntris < 50000) || (p.width < 8 && (ntris < 1000 || bounces <= 1))) return never;
+  if (bounces <= 1) return ntris >= 10000 || (ntris >= 1000 && pixels <= 1024) ? 2 : 16;
+  if (ntris >= 1000) return 2;
+  return ntris >= 100 ? std::max<uint64_t>(4, bounces) : 4 * bounces;
+}
+
+// Calls of one sample run in paths.cu up to this many pixels (tile positions,
+// of an image narrower than a tile), else in the megakernel: a warp's pools
+// shorten a path's chain of steps, which few triangles make short anyway, and
+// cost more the fuller the GPU is. us, megakernel / paths.cu, 8 bounces: Cornell
+// box of 12 triangles 64 x 64 57 / 59, 256 x 256 70 / 150; of 32, 32 x 32 67 /
+// 55; of 112, 96 x 96 92 / 86, 180 x 180 98 / 129; of 1K, 180 x 180 223 / 198,
+// 256 x 256 266 / 325; of 3K, 96 x 96 361 / 140, 256 x 256 433 / 463; of 12K, 256
+// x 256 740 / 714. One bounce: of 312, 32 x 32 28 / 18, 128 x 128 20 / 30; of 1K,
+// 128 x 128 30 / 35, 180 x 180 28 / 41. One pixel, 5120 triangles: 8 / 10.
+constexpr uint64_t kPathsMinPixels = 8;
+inline uint64_t paths_max_pixels(uint32_t ntris, uint32_t bounces) {
+  if (ntris < 30) return 0;
+  if (ntris < 100) return 1u << 10;
+  if (ntris < 1000) return bounces <= 1 ? 1u << 11 : 10000;
+  if (ntris < 10000) return bounces <= 1 ? 1u << 14 : 1u << 15;
+  return 1u << 16;
+}
+inline bool paths_fit(uint32_t ntris, const rt_render_params &p) {
+  const uint64_t pixels = (uint64_t)p.width * p.height;
+  const bool thin = p.width < 8 || p.height < 4;
+  const uint64_t extent = thin ? (uint64_t)((p.width + 7) / 8) * ((p.height + 3) / 4) * 32 : pixels;
+  return pixels >= kPathsMinPixels && extent <= paths_max_pixels(ntris, p.max_bounces);
+}
+
 constexpr uint64_t kWavefrontPixels = 1u << 17;
+constexpr uint32_t kWavefrontTris = 1000;
 
 // Render launch-shape knobs (rtSetTuning "render.mode").
 struct RenderOpts {
-  int mode = 2;  // 0 megakernel, 1 wavefront, 2 choose by image size, 3 choose, without the wavefront
-  // mode 2, at this value: calls of one sample run as a wavefront from 2^17 pixels up
-  // (below, paths.cu up to 65,536 and the megakernel between), calls of
-  // several samples always: the samples share a wave, where the megakernel's
-  // threads run them one after the other. Megakernel / wavefront, Cornell box
-  // of 1K, 12K, 100K triangles, mesh of 512K, 8 bounces, 1 sample, us: 288 x
-  // 288 386 / 409, 1005 / 843, 1752 / 1497, 800 / 589; 352 x 352 459 / 458,
-  // 1256 / 950, 2367 / 1664, 967 / 677; 511 x 512 842 / 573, 2285 / 1334, 3920
-  // / 2238, 1300 / 806. 4 samples, 12K: 48 x 48 2354 / 983, 512 x 512 8897 /
-  // 4344.
+  int mode = 2;  // 0 megakernel, 1 wavefront, 2 choose by sizes, 3 choose, without the wavefront
+  // mode 2, at this value: every call is a wavefront from kOneLaunchPixels up;
+  // below, those of several samples by wave_min_samples, those of one from this
+  // many pixels up in scenes of kWavefrontTris, the rest in paths.cu (paths_fit)
+  // or the megakernel. One sample, 8 bounces, us, megakernel / wavefront: 380 x
+  // 380, Cornell box of 112 triangles 210 / 299, 312 294 / 356, 1K 480 / 466,
+  // 12K 1264 / 939, an icosphere of 320 86 / 200; 511 x 512, 100K 3920 / 2238, a
+  // mesh of 512K 1300 / 806.
   // Any other value is the caller's own line, for calls of any number of
   // samples (2^31: never).
   uint64_t wavefront_pixels = kWavefrontPixels;
@@ -46,13 +91,15 @@ struct RenderOpts {
   // closest-hit entry points keep trace.sort.
   int sort = 0;
 };
-// True when a render of these params goes to the wavefront kernels.
-inline bool use_wavefront(const RenderOpts &o, const rt_render_params &p) {
+// True when a render of a scene of ntris triangles goes to the wavefront kernels.
+inline bool use_wavefront(const RenderOpts &o, uint32_t ntris, const rt_render_params &p) {
   if (p.flags & RT_COMPAT_STACK16) return false;  // the literal 16-entry traversal is megakernel-only
   const uint64_t pixels = (uint64_t)p.width * p.height;
   if (pixels >= (1ull << 31)) return false;
   if (o.mode != 2) return o.mode == 1;
-  return pixels >= o.wavefront_pixels || (o.wavefront_pixels == kWavefrontPixels && p.spp > 1);
+  if (o.wavefront_pixels != kWavefrontPixels) return pixels >= o.wavefront_pixels;
+  if (pixels >= kOneLaunchPixels) return true;
+  return p.spp > 1 ? p.spp >= wave_min_samples(ntris, p) : pixels >= kWavefrontPixels && ntris >= kWavefrontTris;
 }
 // True when a job of a batch or a server step goes to the wavefront kernels.
 inline bool use_wavefront_batched(const RenderOpts &o, const rt_render_params &p) {
