@@ -171,14 +171,17 @@ rt_status rtTraceClosestHost(rt_ctx *ctx, rt_scene_id scene, const rt_ray *h_ray
  *                   ray's input index; scratch comes from the stream-ordered
  *                   pool), except those that trace.packet_min_rays leaves as
  *                   they are
- *   "trace.packet_min_rays"  batches below this many rays (default 2^20)
- *                   go to the 8-wide caster in input order, without the sort
- *                   or the packet pass; so do larger ones whose rays mostly
- *                   have origins of their own. The smallest (up to 16,384
- *                   rays, 32,768 from 2^18 triangles up, 65,536 from 2^20) are
- *                   cast a few rays a warp. Only while trace.wide,
- *                   trace.packet and trace.defer are 1, trace.refill is 32 and
- *                   no beams are asked for. Results are identical either way
+ *   "trace.packet_min_rays"  batches below this many rays (default 2^20) go
+ *                   to the 8-wide caster in input order, without the sort or
+ *                   the packet pass; so do larger ones whose rays mostly have
+ *                   origins of their own. The line is 13/16 of the value in
+ *                   scenes of 4,096 to 100,000 triangles, and from 2^19
+ *                   triangles up the value times triangles / 2^19. The smallest
+ *                   batches (up to 16,384 rays, 32,768 from 2^18 triangles up,
+ *                   65,536 from 2^20) are cast a few rays a warp. Only while
+ *                   trace.wide, trace.packet and trace.defer are 1,
+ *                   trace.refill is 32 and no beams are asked for. Results are
+ *                   identical either way
  *   "trace.packet"  1 (default) = a warp whose 32 rays share an origin and
  *                   point within ~18 degrees traverses them as one packet
  *                   (one node sequence, every lane busy); 0 = always one

@@ -34,6 +34,7 @@ extern "C" int batched(int mode, uint64_t pixels, uint32_t w, uint32_t h, uint32
 extern "C" int fallback(int mode, uint64_t pixels, uint32_t w, uint32_t h) {
   return one_launch_fallback(opts(mode, pixels), params(w, h, 1, 8, 0));
 }
+extern "C" int direct(uint32_t ntris, uint32_t n, uint32_t line) { return direct_rays(ntris, n, line); }
 """
 
 
@@ -107,3 +108,16 @@ def test_larger_scenes_keep_their_waves_and_paths(routes):
     for ntris in (1, 12, 320, 1 << 20):  # from 2^18 pixels up, and many samples
         assert routes.wavefront(2, 0, 512, 512, 1, 1, 0, ntris) and routes.wavefront(2, 0, 64, 64, 64, 8, 0, ntris)
     assert not routes.paths(1 << 20, 257, 256, 8)
+
+
+def test_batches_that_are_cast_as_they_are(routes):
+    line = 1 << 20
+    for ntris in (1, 1280, 100000, 327680, 1 << 19):
+        assert routes.direct(ntris, line - 1, line) and not routes.direct(ntris, line, line)
+    for ntris in (4096, 20480, 81920, 99999):  # packets pay sooner
+        assert routes.direct(ntris, 851967, line) and not routes.direct(ntris, 851968, line)
+    for ntris in (1310720, 2048012):  # and later where triangles outnumber the rays
+        assert routes.direct(ntris, 2 * ntris - 1, line) and not routes.direct(ntris, 2 * ntris, line)
+    for ntris in (1, 20480, 1 << 30):
+        assert not routes.direct(ntris, 1, 0)  # 0: never
+        assert routes.direct(ntris, 0xf0000000, 0xffffffff) == (not 4096 <= ntris < 100000)

@@ -832,6 +832,7 @@ rt_status rtTraceClosestHost(rt_ctx *ctx, rt_scene_id id, const rt_ray *h_rays, 
   // camera rays want large chunks (packets, trace.packet_min_rays).
   constexpr uint32_t kHostSplit = 1u << 19;
   const uint32_t chunk = n <= opts.host_chunk ? std::min(opts.host_chunk, std::max(kHostSplit, n / 4 + 1)) : opts.host_chunk;
+  const uint32_t chunk_rays = std::min(n, chunk);
   const size_t io_bytes = (size_t)chunk * (sizeof(rt_ray) + sizeof(rt_hit));
   const size_t chunk_bytes = (trace_chunk_scratch_bytes(chunk) + 255) & ~size_t(255);
   const size_t need = io_bytes + chunk_bytes + raysort_scratch_bytes(chunk);
@@ -875,7 +876,9 @@ rt_status rtTraceClosestHost(rt_ctx *ctx, rt_scene_id id, const rt_ray *h_rays, 
     uint32_t *perm = nullptr;
     uint32_t *chunks = (uint32_t *)((char *)lane->stage[s] + io_bytes);
     RayCells cells;
-    const bool direct = cast_direct(opts, d, m), sorted = !direct && opts.sort && m >= 65536;
+    // A large rest takes the whole chunks' route: camera rays 5M into 20K
+    // triangles 1450 us, with the last 0.8M cast as they are 1630.
+    const bool direct = cast_direct(opts, d, m <= kHostSplit ? m : chunk_rays), sorted = !direct && opts.sort && m >= 65536;
     const bool beams = sorted && opts.packet && beam_cast(opts, d);
     const uint32_t *gate = nullptr;
     if (e == cudaSuccess && sorted)

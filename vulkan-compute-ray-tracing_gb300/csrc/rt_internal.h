@@ -118,11 +118,9 @@ struct TraceOpts {
   int sort = 1;     // 1: cast rays in Morton order of origin and direction (raysort.cu)
   int packet = 1;   // 1: warps of coherent rays traverse as one packet (traverse_packet)
   // Smaller batches go straight to the 8-wide caster, in input order: neither
-  // the sort nor the packets pay there. Sorted packets / direct, us: 2^18
-  // camera rays into 20K, 328K, 1.31M triangles 161 / 120, 625 / 315, 1423 /
-  // 812; 2^20 271 / 340, 765 / 864, 1815 / 1899; 2^18 random rays 173 / 108,
-  // 355 / 286, 755 / 658.
-  uint32_t packet_min_rays = 1u << 20;
+  // the sort nor the packets pay there (direct_rays in routes.h: the line
+  // moves with the scene's size).
+  uint32_t packet_min_rays = kPacketMinRays;
   int beam = 0;     // sorted one-origin batches traverse the sort's cell tiles as beams (beam.cuh):
                     // 1 always, 0 never, 2 on Bvh.h's median-split trees (DevScene::median_tree)
   int beam_round = 64;  // leaves a beam round collects before its rays test them (16..256)
@@ -176,7 +174,8 @@ inline bool use_wide(const TraceOpts &o, const DevScene &sc) {
   return o.wide && sc.ntris >= o.wide_min_tris && wide_ok(sc);
 }
 inline bool cast_direct(const TraceOpts &o, const DevScene &sc, uint32_t n) {
-  return o.refill >= 32 && o.packet && o.defer && !beam_cast(o, sc) && use_wide(o, sc) && n < o.packet_min_rays;
+  return o.refill >= 32 && o.packet && o.defer && !beam_cast(o, sc) && use_wide(o, sc) &&
+         direct_rays(sc.ntris, n, o.packet_min_rays);
 }
 // True when a sorted batch's order and packets are worth having only if its
 // rays share origins (gate_out of launch_raysort): the rest are cast directly.
