@@ -75,3 +75,71 @@ def test_renders_without_scratch_are_one_launch(rt, ctx, tune, side, spp):
     finally:
         tune(test__alloc_limit=0)
         sc.release()
+
+
+def one_sample_limit(side):
+    """Bytes that hold a sample's paths of a side x side image, not two samples'."""
+    return 140 * side * side
+
+
+def test_large_renders_take_a_sample_at_a_time(rt, ctx, tune):
+    import torch
+    tris, mats, _ = rt.gen_cornell(8, 1500)
+    sc = ctx.upload_scene(tris, mats)
+    try:
+        sc.set_camera(rt.camera_look_at([0.2, 0.1, -14], [0, 0, 0], [0, 1, 0], 40.0, 512, 512))
+        images = []
+        for limit in (0, one_sample_limit(512)):
+            tune(test__alloc_limit=limit)
+            img = torch.zeros((512, 512, 4), device="cuda")
+            torch.cuda.synchronize()
+            sc.render(img, 512, 512, 4, 5)
+            ctx.synchronize()
+            images.append(img)
+        assert torch.equal(images[0], images[1])
+    finally:
+        tune(test__alloc_limit=0)
+        sc.release()
+
+
+def test_batches_take_a_sample_at_a_time(rt, ctx, tune):
+    import torch
+    scenes = [ctx.upload_scene(*rt.gen_cornell(8 + i, 1500)[:2]) for i in range(3)]
+    try:
+        cam = rt.camera_look_at([0.2, 0.1, -14], [0, 0, 0], [0, 1, 0], 40.0, 128, 128)
+        images = []
+        for limit in (0, one_sample_limit(128)):
+            tune(test__alloc_limit=limit)
+            imgs = [torch.zeros((128, 128, 4), device="cuda") for _ in scenes]
+            torch.cuda.synchronize()
+            b = ctx.batch([rt.make_job(s, cam, i, 128, 128, 16, 4) for s, i in zip(scenes, imgs)])
+            b.launch()
+            ctx.synchronize()
+            b.launch_graph()
+            ctx.synchronize()
+            b.destroy()
+            images.append(imgs)
+        assert all(torch.equal(a, b) for a, b in zip(*images))
+        tune(test__alloc_limit=1000)
+        with pytest.raises(rt.RtError):
+            ctx.batch([rt.make_job(scenes[0], cam, images[0][0], 128, 128, 16, 4)])
+    finally:
+        tune(test__alloc_limit=0)
+        for s in scenes:
+            s.release()
+
+
+def test_the_server_takes_a_sample_at_a_time(rt, ctx, tune):
+    from rtgb import serve
+    data = rt.gen_cornell(8, 300)
+    cam = rt.camera_look_at([0.2, 0.1, -14], [0, 0, 0], [0, 1, 0], 40.0, 128, 128)
+    images = []
+    for limit in (0, one_sample_limit(128)):
+        tune(test__alloc_limit=limit)
+        with serve.Server(ctx, max_active=4, spp_per_step=8) as srv:
+            h = srv.add_scene(*data)
+            ids = [srv.submit(h, cam, 128, 128, 8, 4) for _ in range(3)]
+            for i in ids:
+                assert srv.wait(i, 60000).state == serve.DONE
+            images += [srv.image(i).copy() for i in ids]
+    assert all(np.array_equal(i, images[0]) for i in images) and images[0].any()

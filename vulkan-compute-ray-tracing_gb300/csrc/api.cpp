@@ -934,9 +934,15 @@ rt_status rtRender(rt_ctx *ctx, rt_scene_id id, const rt_render_params *p, float
   if (small) CK(cudaStreamIsCapturing(st, &capture), "capture status");
   if (use_wavefront(ropts, d.ntris, *p) && !(small && capture != cudaStreamCaptureStatusNone)) {
     void *scratch = nullptr;
-    cudaError_t e = scratch_alloc(&scratch, wavefront_scratch_bytes(*p, ropts.sort != 0), ctx->pool, st);
+    uint32_t wave = kWavePaths;
+    cudaError_t e = scratch_alloc(&scratch, wavefront_scratch_bytes(*p, ropts.sort != 0, wave), ctx->pool, st);
+    if (e == cudaErrorMemoryAllocation && p->spp > 1) {
+      cudaGetLastError();
+      wave = kOneSample;
+      e = scratch_alloc(&scratch, wavefront_scratch_bytes(*p, ropts.sort != 0, wave), ctx->pool, st);
+    }
     if (e == cudaSuccess) {
-      e = launch_render_wavefront(d, cam, *p, accum, ctx->d_segments, ctx->d_err, scratch, ropts.sort != 0,
+      e = launch_render_wavefront(d, cam, *p, accum, ctx->d_segments, ctx->d_err, scratch, wave, ropts.sort != 0,
                                   use_wide(topts, d), st, nullptr, true);
       cudaFreeAsync(scratch, st);
       if (e != cudaSuccess) return cuda_fail(ctx, e, "render launch");
@@ -1355,6 +1361,7 @@ struct rt_batch {
   static constexpr int kSides = 16;
   int sides = 0;
   void *wf_scratch[kSides] = {};
+  uint32_t wave = kWavePaths;  // kOneSample where memory was short
   bool wf_sort = false;
   bool wf_wide = true;
   uint32_t wf_wide_min = 0;
@@ -1407,6 +1414,24 @@ rt_status make_jobs(rt_ctx *ctx, const rt_render_job *jobs, uint32_t n, std::vec
 
 bool wavefront_job(const RenderOpts &o, const rt_render_params &p) { return use_wavefront_batched(o, p); }
 
+// Each side stream's scratch, for the largest of its jobs; none after an error.
+cudaError_t batch_scratch(rt_ctx *ctx, rt_batch *b, uint32_t wave) {
+  cudaError_t e = cudaSuccess;
+  b->wave = wave;
+  for (int k = 0; k < b->sides && e == cudaSuccess; k++) {
+    size_t bytes = 0;
+    for (size_t j = k; j < b->wf.size(); j += (size_t)b->sides)
+      bytes = std::max(bytes, wavefront_scratch_bytes(b->wf[j].p, b->wf_sort, wave));
+    e = ctx_malloc(ctx, &b->wf_scratch[k], bytes);
+    if (e != cudaSuccess) b->wf_scratch[k] = nullptr;
+  }
+  for (int k = 0; k < b->sides && e != cudaSuccess; k++) {
+    if (b->wf_scratch[k]) cudaFree(b->wf_scratch[k]);
+    b->wf_scratch[k] = nullptr;
+  }
+  return e;
+}
+
 cudaError_t batch_enqueue(rt_ctx *ctx, rt_batch *b, cudaStream_t st) {
   cudaError_t e = cudaSuccess;
   const int sides = b->sides;
@@ -1417,8 +1442,9 @@ cudaError_t batch_enqueue(rt_ctx *ctx, rt_batch *b, cudaStream_t st) {
     for (size_t j = 0; j < b->wf.size() && e == cudaSuccess; j++) {
       const BatchJob &J = b->wf[j];
       const int k = (int)(j % (size_t)sides);
-      e = launch_render_wavefront(J.sc, J.cam, J.p, J.accum, ctx->d_segments, ctx->d_err, b->wf_scratch[k], b->wf_sort, b->wf_wide && J.sc.ntris >= b->wf_wide_min,
-                                  b->side[k], &b->d_wf[j].p.sample_index);
+      e = launch_render_wavefront(J.sc, J.cam, J.p, J.accum, ctx->d_segments, ctx->d_err, b->wf_scratch[k], b->wave,
+                                  b->wf_sort, b->wf_wide && J.sc.ntris >= b->wf_wide_min, b->side[k],
+                                  &b->d_wf[j].p.sample_index);
     }
     for (int k = 0; k < sides && e == cudaSuccess; k++) e = cudaEventRecord(b->join[k], b->side[k]);
   }
@@ -1458,12 +1484,10 @@ rt_status rtBatchCreate(rt_ctx *ctx, const rt_render_job *jobs, uint32_t n_jobs,
   std::vector<BatchJob> tiles_jobs;
   rt_batch *b = new rt_batch();
   uint64_t tiles = 0;
-  size_t wf_bytes = 0;
   b->max_depth = 1;
   for (const BatchJob &J : host) {
     if (wavefront_job(ropts, J.p)) {
       b->wf.push_back(J);
-      wf_bytes = std::max(wf_bytes, wavefront_scratch_bytes(J.p, ropts.sort != 0));
     } else {
       BatchJob T = J;
       T.tile_begin = (uint32_t)tiles;
@@ -1491,9 +1515,13 @@ rt_status rtBatchCreate(rt_ctx *ctx, const rt_render_job *jobs, uint32_t n_jobs,
     const int sides =
         (int)std::min<size_t>(b->wf.size(), (size_t)std::clamp(ropts.batch_streams, 1, rt_batch::kSides));
     b->sides = sides;
+    if (e == cudaSuccess) e = batch_scratch(ctx, b, kWavePaths);
+    if (e == cudaErrorMemoryAllocation) {
+      cudaGetLastError();
+      e = batch_scratch(ctx, b, kOneSample);
+    }
     for (int k = 0; k < sides && e == cudaSuccess; k++) {
-      e = ctx_malloc(ctx, &b->wf_scratch[k], wf_bytes);
-      if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->side[k], cudaStreamNonBlocking);
+      e = cudaStreamCreateWithFlags(&b->side[k], cudaStreamNonBlocking);
       if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->join[k], cudaEventDisableTiming);
     }
   }

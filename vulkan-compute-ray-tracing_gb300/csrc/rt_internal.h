@@ -237,16 +237,23 @@ bool paths_ok(const DevScene &sc, const rt_render_params &p);
 cudaError_t launch_render_paths(const DevScene &sc, const rt_camera &cam, const rt_render_params &p, float *accum,
                                 unsigned long long *segments, uint32_t *counter, uint32_t *err, cudaStream_t st);
 
+// Paths of one wave of a wavefront render: samples of a call are added until
+// this many run together. A wave of fewer leaves the GPU idle in every bounce's
+// tail: 500 x 375, 4 samples, 100K triangles in one wave 6.1 ms, in the
+// megakernel 12.3; larger waves cost scratch (108 B a path). kOneSample: a
+// sample at a time, the least scratch, where that of a whole wave cannot be had.
+constexpr uint32_t kWavePaths = 1u << 20, kOneSample = 1;
 // Wavefront render (wavefront.cu): same images as launch_render; `scratch`
-// holds wavefront_scratch_bytes(p, sort). With d_sample_index the kernels read
-// the first sample index from the device at run time instead of
+// holds wavefront_scratch_bytes(p, sort, wave_paths). With d_sample_index the
+// kernels read the first sample index from the device at run time instead of
 // p.sample_index.
-size_t wavefront_scratch_bytes(const rt_render_params &p, bool sort);
+size_t wavefront_scratch_bytes(const rt_render_params &p, bool sort, uint32_t wave_paths);
 // `wide`: bounce rays are cast by the 8-wide caster (launch_wide_leaf), short
 // queues of a render that runs `alone` by launch_pool_leaf.
 cudaError_t launch_render_wavefront(const DevScene &sc, const rt_camera &cam, const rt_render_params &p, float *accum,
-                                    unsigned long long *segments, uint32_t *err, void *scratch, bool sort, bool wide,
-                                    cudaStream_t st, const uint32_t *d_sample_index = nullptr, bool alone = false);
+                                    unsigned long long *segments, uint32_t *err, void *scratch, uint32_t wave_paths,
+                                    bool sort, bool wide, cudaStream_t st, const uint32_t *d_sample_index = nullptr,
+                                    bool alone = false);
 
 // Tree used when a scene is uploaded without nodes (rtSetTuning "bvh.builder").
 struct BuildOpts {

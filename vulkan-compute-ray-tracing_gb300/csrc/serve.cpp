@@ -85,6 +85,7 @@ struct rt_server {
   cudaEvent_t fork = nullptr, join[kSides] = {};
   void *scratch[kSides] = {};
   size_t scratch_bytes[kSides] = {};
+  uint32_t wave = kWavePaths;  // kOneSample once memory was short
 };
 
 namespace {
@@ -141,6 +142,26 @@ void admit(rt_server *s, std::vector<SrvReq *> &admitted, std::vector<rt_scene_i
     q->start_ms = now_ms(s);
     admitted.push_back(q);
   }
+}
+
+// Grows the side streams' scratch to what their jobs of this step take.
+cudaError_t side_scratch(rt_server *s, const std::vector<BatchJob> &wf, int sides, bool sort) {
+  cudaError_t e = cudaSuccess;
+  for (int k = 0; k < sides && e == cudaSuccess; k++) {
+    size_t need = 0;
+    for (size_t j = k; j < wf.size(); j += rt_server::kSides)
+      need = std::max(need, wavefront_scratch_bytes(wf[j].p, sort, s->wave));
+    if (need <= s->scratch_bytes[k]) continue;
+    if (s->scratch[k]) cudaFree(s->scratch[k]);
+    s->scratch[k] = nullptr;
+    s->scratch_bytes[k] = 0;
+    e = ctx_malloc(s->ctx, &s->scratch[k], need);
+    if (e == cudaSuccess)
+      s->scratch_bytes[k] = need;
+    else
+      s->scratch[k] = nullptr;
+  }
+  return e;
 }
 
 void scheduler(rt_server *s) {
@@ -235,17 +256,11 @@ void scheduler(rt_server *s) {
     }
     cudaError_t e = cudaSuccess;
     const int sides = (int)std::min<size_t>(wf.size(), rt_server::kSides);
-    for (int k = 0; k < sides && e == cudaSuccess; k++) {
-      size_t need = 0;
-      for (size_t j = k; j < wf.size(); j += rt_server::kSides)
-        need = std::max(need, wavefront_scratch_bytes(wf[j].p, sort));
-      if (need > s->scratch_bytes[k]) {
-        if (s->scratch[k]) cudaFree(s->scratch[k]);
-        s->scratch[k] = nullptr;
-        s->scratch_bytes[k] = 0;
-        e = ctx_malloc(s->ctx, &s->scratch[k], need);
-        if (e == cudaSuccess) s->scratch_bytes[k] = need;
-      }
+    e = side_scratch(s, wf, sides, sort);
+    if (e == cudaErrorMemoryAllocation && s->wave != kOneSample) {
+      cudaGetLastError();
+      s->wave = kOneSample;
+      e = side_scratch(s, wf, sides, sort);
     }
     if (e == cudaSuccess && sides) {
       e = cudaEventRecord(s->fork, s->stream);
@@ -254,7 +269,7 @@ void scheduler(rt_server *s) {
         const int k = (int)(j % rt_server::kSides);
         const BatchJob &J = wf[j];
         e = launch_render_wavefront(J.sc, J.cam, J.p, J.accum, ctx_segments(s->ctx), ctx_err(s->ctx), s->scratch[k],
-                                    sort, wide && J.sc.ntris >= wide_min, s->side[k]);
+                                    s->wave, sort, wide && J.sc.ntris >= wide_min, s->side[k]);
       }
       for (int k = 0; k < sides && e == cudaSuccess; k++) e = cudaEventRecord(s->join[k], s->side[k]);
     }

@@ -1,6 +1,6 @@
 // Wavefront render: the bounce loop of ray-trace-compute.comp:314-338 split
 // into kernels over queues of live paths. A path is one sample of one pixel;
-// the samples of a call run together, as many at a time as kWavePaths holds.
+// the samples of a call run together, as many at a time as a wave (kWavePaths) holds.
 //
 //   camera      closest triangle of every pixel's camera ray, once per call
 //               (the ray carries no jitter), 8 x 4 pixel tiles as packets
@@ -33,12 +33,6 @@ namespace {
 
 constexpr int kWfBlock = 128, kShadeBlock = 256;
 
-// Paths of one wave: samples of a call are added until this many run
-// together. A wave of fewer leaves the GPU idle in every bounce's tail: 500 x
-// 375, 4 samples, 100K triangles in one wave 6.1 ms, in the megakernel 12.3;
-// larger waves cost scratch (108 B a path).
-constexpr uint32_t kWavePaths = 1u << 20;
-
 // Device words of a wave. Queue lengths and the caster's work counters are
 // used in turn; shading clears the ones its next bounce needs.
 enum : uint32_t { kCountQueue = 0, kCountWork = 4, kCountWords = 64 };
@@ -56,8 +50,8 @@ struct WfBufs {
 
 size_t a256(size_t x) { return (x + 255) & ~size_t(255); }
 
-uint32_t wave_samples(const rt_render_params &p, const Tiles &t) {
-  return std::max(1u, std::min(p.spp, kWavePaths / std::max(t.positions, 1u)));
+uint32_t wave_samples(const rt_render_params &p, const Tiles &t, uint32_t wave_paths) {
+  return std::max(1u, std::min(p.spp, wave_paths / std::max(t.positions, 1u)));
 }
 
 WfBufs carve(void *scratch, uint32_t cap, uint32_t positions) {
@@ -306,16 +300,17 @@ int g_sms = 0;
 
 }  // namespace
 
-size_t wavefront_scratch_bytes(const rt_render_params &p, bool sort) {
+size_t wavefront_scratch_bytes(const rt_render_params &p, bool sort, uint32_t wave_paths) {
   const Tiles t = tiles_of(p);
-  const size_t cap = (size_t)t.positions * wave_samples(p, t);
+  const size_t cap = (size_t)t.positions * wave_samples(p, t, wave_paths);
   return 2 * (a256(sizeof(rt_ray) * cap) + a256(4 * cap)) + a256(8 * cap) + a256(8ull * t.positions) + a256(16 * cap) +
          a256(4 * cap) + a256(4ull * kCountWords) + (sort ? a256(raysort_scratch_bytes((uint32_t)cap)) : 0);
 }
 
 cudaError_t launch_render_wavefront(const DevScene &sc, const rt_camera &cam, const rt_render_params &p, float *accum,
-                                    unsigned long long *segments, uint32_t *err, void *scratch, bool sort, bool wide,
-                                    cudaStream_t st, const uint32_t *d_sample_index, bool alone) {
+                                    unsigned long long *segments, uint32_t *err, void *scratch,
+                                    uint32_t wave_paths, bool sort, bool wide, cudaStream_t st,
+                                    const uint32_t *d_sample_index, bool alone) {
   const Tiles tiles = tiles_of(p);
   if (p.width == 0 || p.height == 0 || p.spp == 0) return cudaSuccess;
   const bool use_wide = wide && wide_ok(sc);
@@ -324,7 +319,7 @@ cudaError_t launch_render_wavefront(const DevScene &sc, const rt_camera &cam, co
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&g_sms, cudaDevAttrMultiProcessorCount, dev);
   }
-  const uint32_t samples = wave_samples(p, tiles), cap = tiles.positions * samples;
+  const uint32_t samples = wave_samples(p, tiles, wave_paths), cap = tiles.positions * samples;
   WfBufs b = carve(scratch, cap, tiles.positions);
   uint32_t *queue = b.counts + kCountQueue, *work = b.counts + kCountWork;
   float4 *image = reinterpret_cast<float4 *>(accum);
