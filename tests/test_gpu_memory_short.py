@@ -143,3 +143,29 @@ def test_the_server_takes_a_sample_at_a_time(rt, ctx, tune):
                 assert srv.wait(i, 60000).state == serve.DONE
             images += [srv.image(i).copy() for i in ids]
     assert all(np.array_equal(i, images[0]) for i in images) and images[0].any()
+
+
+@pytest.mark.parametrize("n", [32, 1000])
+def test_no_memory_for_the_cast_tree_leaves_the_references(rt, ctx, tune, n):
+    # The cast tree's build takes half a megabyte at least; the scene and its
+    # other scratch stay below the limit.
+    import torch
+    tris, mats = soup(rt, n)
+    rays = torch.from_numpy(rt.gen_random_rays(3, 20000, -5, 5)).cuda()
+    trees = []
+    for limit in (0, 400000):
+        tune(test__alloc_limit=limit)
+        hits = torch.zeros((len(rays), 4), device="cuda")
+        torch.cuda.synchronize()
+        sc = ctx.upload_scene(tris, mats)
+        sc.trace(rays, len(rays), hits)
+        ctx.synchronize()
+        trees.append((hits, sc.bvh(), sc.info().device_bytes))
+        sc.release()
+    assert torch.equal(trees[0][0].view(torch.int32), trees[1][0].view(torch.int32))
+    assert np.array_equal(trees[0][1].view(np.uint32), trees[1][1].view(np.uint32)) and trees[0][2] == trees[1][2]
+    tune(test__alloc_limit=0, bvh__builder=2)
+    ctx.upload_scene(tris, mats).release()
+    tune(test__alloc_limit=400000)
+    with pytest.raises(rt.RtError):  # the scene's only tree
+        ctx.upload_scene(tris, mats)

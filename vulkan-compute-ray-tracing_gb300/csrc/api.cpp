@@ -603,6 +603,9 @@ rt_status rtUploadScene(rt_ctx *ctx, const rt_triangle *tris, uint32_t nt, const
           cast_nodes = cast_scratch;
           d.depth = cast_depth;
           median_tree = false;
+        } else {
+          cudaFreeAsync(cast_scratch, st);  // not held where memory may be short
+          cast_scratch = nullptr;
         }
       }
     }
