@@ -48,7 +48,7 @@ typedef uint32_t rt_scene_id;
 
 typedef struct rt_ctx_desc {
   int device;                /* CUDA device ordinal */
-  uint64_t hbm_budget_bytes; /* resident-scene budget; 0 = 80% of free HBM */
+  uint64_t hbm_budget_bytes; /* resident-scene budget; 0 = 80% of free HBM (scratch is apart: mem.scratch_keep) */
   uint32_t flags;            /* reserved, 0 */
   uint32_t _reserved;
 } rt_ctx_desc;
@@ -296,6 +296,12 @@ rt_status rtTraceClosestHost(rt_ctx *ctx, rt_scene_id scene, const rt_ray *h_ray
  *                   folded pairs chosen by the surface area heuristic
  *                   (least summed node area: fewer node visits), 0 the
  *                   largest child opened first; the hits are the same
+ *   "mem.scratch_keep"  bytes of device scratch the context keeps between calls
+ *                   (default 2^30; 0: none, which costs a call after a
+ *                   synchronisation 0.13 ms), outside hbm_budget_bytes.
+ *                   Setting it gives what is kept above it back at once, for
+ *                   another allocator of the process that needs the memory;
+ *                   the context's own allocations take it back by themselves
  *   "bvh.test_error_level"  test hook (default -1, off): builder 0 records
  *                   an error bit in its device error word after the sort of
  *                   this tree level, as a sort overflow would, so the upload

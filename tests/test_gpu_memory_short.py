@@ -169,3 +169,23 @@ def test_no_memory_for_the_cast_tree_leaves_the_references(rt, ctx, tune, n):
     tune(test__alloc_limit=400000)
     with pytest.raises(rt.RtError):  # the scene's only tree
         ctx.upload_scene(tris, mats)
+
+
+def test_kept_scratch_is_given_back_when_asked(rt):
+    import torch
+    torch.cuda.synchronize()
+    free0 = torch.cuda.mem_get_info()[0]
+    with rt.Context(0) as own:
+        assert own.get_tuning("mem.scratch_keep") == 1 << 30
+        mats = rt.gen_cornell(1, 0)[1]
+        own.upload_scene(rt.gen_icosphere(1, 8), mats).release()
+        torch.cuda.synchronize()
+        kept = free0 - torch.cuda.mem_get_info()[0]
+        own.set_tuning("mem.scratch_keep", 0)
+        held = free0 - torch.cuda.mem_get_info()[0]
+        assert held < 128 << 20 and held < kept
+        own.upload_scene(rt.gen_icosphere(1, 8), mats).release()
+        torch.cuda.synchronize()
+        assert free0 - torch.cuda.mem_get_info()[0] < 128 << 20
+        with pytest.raises(rt.RtError):
+            own.set_tuning("mem.scratch_keep", -1)

@@ -24,7 +24,6 @@ using namespace rtgb;
 namespace {
 
 constexpr uint32_t kCounterRing = 1024;
-constexpr uint64_t kPoolKeep = 1ull << 30;  // scratch a context keeps (an upload of 1.31M triangles takes half)
 constexpr uint32_t kMaxTreeDepth = 64;     // the traversal stacks' largest size
 // Below, the reference's tree is as quick to cast on: us a frame of 256 x 256, 8
 // bounces, on the reference's / on PLOC: 12 triangles (a bare Cornell box) 65 /
@@ -67,9 +66,10 @@ struct rt_ctx {
   int device = 0;
   cudaStream_t stream = nullptr;
   // Scratch of this context's calls, on whichever stream they run. The pool
-  // keeps up to kPoolKeep of it over synchronisations (the default pool gives
-  // everything back: 0.13 ms a call, and 0.7 of a 1.31M-triangle upload); the rest
-  // goes back at once, all of it with the context or when memory runs out.
+  // keeps up to mem.scratch_keep of it over synchronisations (the default pool
+  // gives everything back: 0.13 ms a call, and 0.7 of a 1.31M-triangle upload);
+  // the rest goes back at once, all of it with the context or when one of the
+  // context's own allocations finds no memory.
   ScratchPool pool;
   std::mutex mu;
   std::unordered_map<uint32_t, Scene *> scenes;
@@ -316,8 +316,8 @@ rt_status rtCreate(rt_ctx **out, const rt_ctx_desc *desc) {
     props.location.type = cudaMemLocationTypeDevice;
     props.location.id = ctx->device;
     e = cudaMemPoolCreate(&ctx->pool.pool, &props);
-    uint64_t keep = kPoolKeep;
-    if (e == cudaSuccess) e = cudaMemPoolSetAttribute(ctx->pool.pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    if (e == cudaSuccess)
+      e = cudaMemPoolSetAttribute(ctx->pool.pool, cudaMemPoolAttrReleaseThreshold, &ctx->pool.keep);
   }
   if (e == cudaSuccess) e = cudaMalloc((void **)&ctx->d_err, 64);
   if (e == cudaSuccess) e = cudaMemset(ctx->d_err, 0, 64);
@@ -1128,6 +1128,18 @@ rt_status rtSetTuning(rt_ctx *ctx, const char *key, int64_t value) {
     ctx->build_opts.collapse = (int)value;
     return RT_SUCCESS;
   }
+  if (k == "mem.scratch_keep") {
+    if (value < 0) return RT_ERR_INVALID_ARGUMENT;
+    uint64_t keep = (uint64_t)value;
+    cudaError_t e = cudaMemPoolSetAttribute(ctx->pool.pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    if (e == cudaSuccess) e = cudaMemPoolTrimTo(ctx->pool.pool, (size_t)keep);
+    if (e != cudaSuccess) {  // not by fail(), which takes the lock
+      ctx->last_error = std::string("scratch keep: ") + cudaGetErrorString(e);
+      return RT_ERR_CUDA;
+    }
+    ctx->pool.keep = keep;
+    return RT_SUCCESS;
+  }
   if (k == "test.alloc_limit") {
     if (value < 0) return RT_ERR_INVALID_ARGUMENT;
     ctx->pool.test_limit.store((uint64_t)value);
@@ -1257,6 +1269,10 @@ rt_status rtGetTuning(rt_ctx *ctx, const char *key, int64_t *value) {
   }
   if (k == "bvh.ploc_radius") {
     *value = ctx->build_opts.ploc_radius;
+    return RT_SUCCESS;
+  }
+  if (k == "mem.scratch_keep") {
+    *value = (int64_t)ctx->pool.keep;
     return RT_SUCCESS;
   }
   if (k == "test.alloc_limit") {

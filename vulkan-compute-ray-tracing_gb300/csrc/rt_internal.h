@@ -16,6 +16,7 @@ namespace rtgb {
 // A context's own memory pool (api.cpp).
 struct ScratchPool {
   cudaMemPool_t pool = nullptr;
+  uint64_t keep = 1ull << 30;  // release threshold (an upload of 1.31M triangles takes a quarter)
   std::atomic<uint64_t> test_limit{0};  // test hook: larger allocations fail as on a full device (0: off)
   bool test_full(size_t bytes) const {
     const uint64_t limit = test_limit.load(std::memory_order_relaxed);
