@@ -246,7 +246,8 @@ cudaError_t launch_denoise(const float *in, uint32_t W, uint32_t H, float sigma,
   p.inv_thr_q2 = 0.5f / (threshold * threshold);
   p.inv_thr_sqrt2pi = kInvSqrt2Pi / threshold;
   p.mix = mix;
-  const int radius = (int)p.radius;
+  const bool tile_radius = p.radius <= (float)kTileRadius;  // not one that is NaN (kSigma 0, sigma infinite)
+  const int radius = tile_radius ? (int)p.radius : kTileRadius + 1;
   const dim3 pixels(16, 16), pixel_grid((W + 15) / 16, (H + 15) / 16);
   // An image of at most a 16 x 16 block an SM (two, where a block has few taps)
   // takes as long as one block, and the tile kernel's is longer. us, per pixel /
@@ -259,7 +260,7 @@ cudaError_t launch_denoise(const float *in, uint32_t W, uint32_t H, float sigma,
     cudaDeviceGetAttribute(&g_sms, cudaDevAttrMultiProcessorCount, dev);
   }
   const uint64_t small = (uint64_t)g_sms * (radius <= 1 ? 2 : 1);
-  if (radius <= kTileRadius && (uint64_t)pixel_grid.x * pixel_grid.y > small) {
+  if (tile_radius && (uint64_t)pixel_grid.x * pixel_grid.y > small) {
     int taps = 0;
     for (float x = -p.radius; x <= p.radius; x += 1.0f) {
       const float pt = std::sqrt(p.rad_q - x * x);
