@@ -167,9 +167,7 @@ cudaError_t launch_trace(const DevScene &sc, const rt_ray *rays, uint32_t n, rt_
                          const uint32_t *perm = nullptr, uint32_t *chunk_scratch = nullptr,
                          const RayCells *cells = nullptr, const uint32_t *gate = nullptr);
 size_t trace_chunk_scratch_bytes(uint32_t n);
-// The 8-wide caster over listed 32-ray chunks of a device-sized queue
-// (*d_n rays, at most cap), writing (leaf k, t) hits; wide_ok tells whether
-// the scene's bvh8 can take it.
+// wide_ok tells whether a scene's 8-wide nodes can be cast on.
 bool wide_ok(const DevScene &sc);
 inline bool use_wide(const TraceOpts &o, const DevScene &sc) {
   return o.wide && sc.ntris >= o.wide_min_tris && wide_ok(sc);
@@ -183,9 +181,11 @@ inline bool cast_direct(const TraceOpts &o, const DevScene &sc, uint32_t n) {
 inline bool cast_gated(const TraceOpts &o, const DevScene &sc) {
   return o.refill >= 32 && o.packet && o.defer && !beam_cast(o, sc) && use_wide(o, sc);
 }
+// The 8-wide caster over a device-sized queue (*d_n rays, at most cap, in the
+// order of perm, if given), writing (leaf k, t) hits; a queue of fewer than
+// min_rays is left to launch_pool_leaf.
 cudaError_t launch_wide_leaf(const DevScene &sc, const rt_ray *rays, uint32_t cap, const uint32_t *d_n,
-                             const uint32_t *perm, const uint32_t *list, const uint32_t *list_count, int2 *hits,
-                             uint32_t *counter, uint32_t *err, int minblocks, int refill, cudaStream_t st,
+                             const uint32_t *perm, int2 *hits, uint32_t *counter, uint32_t *err, cudaStream_t st,
                              uint32_t min_rays = 0);
 // Small batches (pool.cu): R rays a warp from shared pools, up to this many
 // rays. A larger scene's rays take longer chains of steps, which the pools

@@ -626,7 +626,7 @@ __global__ void __maxnreg__(regs_for<MINB>()) k_trace_wide(DevScene sc, const fl
   float4 *const wbase = s_wide + warp * (wide_warp_smem<VISITS>() / 16);
   float4(*ray_s)[2] = reinterpret_cast<float4(*)[2]>(wbase);
   volatile unsigned long long *key_v = reinterpret_cast<unsigned long long *>(wbase + 64);
-    float4 *hit_s = wbase + 80;
+  float4 *hit_s = wbase + 80;
   uint32_t *pool = reinterpret_cast<uint32_t *>(wbase + 112);
   uint32_t *finish = pool + kPool;
   // The pool's tail: lanes reserve their entries with one shared atomic.
@@ -843,7 +843,7 @@ __global__ void __maxnreg__(regs_for<MINB>()) k_trace_wide(DevScene sc, const fl
   #pragma unroll
         for (int s = 0; s < 8; s++) {
           if (!((leafmask >> s) & 1u)) continue;
-          // Leaf refs were range-checked when the bvh8 was built (k_encode8).
+          // Leaf refs were range-checked when the bvh8 was built (k_quantize8).
           pool[pos & (kPool - 1)] = ((uint32_t)~ref[s] << 5) | lane;
           pos++;
         }
@@ -999,8 +999,7 @@ bool wide_ok(const DevScene &sc) {
 }
 
 cudaError_t launch_wide_leaf(const DevScene &sc, const rt_ray *rays, uint32_t cap, const uint32_t *d_n,
-                             const uint32_t *perm, const uint32_t *list, const uint32_t *list_count, int2 *hits,
-                             uint32_t *counter, uint32_t *err, int minblocks, int refill, cudaStream_t st,
+                             const uint32_t *perm, int2 *hits, uint32_t *counter, uint32_t *err, cudaStream_t st,
                              uint32_t min_rays) {
   if (!wide_ok(sc)) return cudaErrorInvalidValue;
   if (g_num_sms == 0) {
@@ -1008,21 +1007,17 @@ cudaError_t launch_wide_leaf(const DevScene &sc, const rt_ray *rays, uint32_t ca
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev);
   }
+  constexpr int kRefill = 4;
   const float4 *r4 = reinterpret_cast<const float4 *>(rays);
-  // minblocks 8: one node step per iteration (64 registers); otherwise three.
-  auto go = [&](auto kern, size_t warp_smem) {
-    const size_t smem = (size_t)(kTraceBlock / 32) * warp_smem;
+  auto go = [&](auto kern) {
+    const size_t smem = (size_t)(kTraceBlock / 32) * wide_warp_smem<3>();
     kern<<<persistent_grid(kern, cap, kTraceBlock, smem), kTraceBlock, smem, st>>>(
-        sc, r4, cap, d_n, hits, counter, err, perm, list, list_count, nullptr, min_rays, refill, false);
+        sc, r4, cap, d_n, hits, counter, err, perm, nullptr, nullptr, nullptr, min_rays, kRefill, false);
     return cudaGetLastError();
   };
-  const bool narrow = minblocks >= 8;
-  const size_t s1 = wide_warp_smem<1>(), s3 = wide_warp_smem<3>();
-  if (sc.levels8 <= 16)
-    return narrow ? go(k_trace_wide<16, 8, true, 1>, s1) : go(k_trace_wide<16, 6, true, 3>, s3);
-  if (sc.levels8 <= 32)
-    return narrow ? go(k_trace_wide<32, 8, true, 1>, s1) : go(k_trace_wide<32, 6, true, 3>, s3);
-  return narrow ? go(k_trace_wide<64, 8, true, 1>, s1) : go(k_trace_wide<64, 6, true, 3>, s3);
+  if (sc.levels8 <= 16) return go(k_trace_wide<16, 6, true, 3>);
+  if (sc.levels8 <= 32) return go(k_trace_wide<32, 6, true, 3>);
+  return go(k_trace_wide<64, 6, true, 3>);
 }
 
 size_t trace_chunk_scratch_bytes(uint32_t n) { return 4ull * (64 + (n + 31) / 32); }

@@ -332,8 +332,8 @@ cudaError_t launch_render_wavefront(const DevScene &sc, const rt_camera &cam, co
     k_wf_rays<<<tile_grid, kWfBlock, 0, st>>>(cam, tiles, reinterpret_cast<float4 *>(b.rays[0]));
     const bool pool = alone && tiles.positions <= pool_max_rays(sc);
     if ((e = pool ? launch_pool_leaf(sc, b.rays[0], tiles.positions, nullptr, nullptr, b.cam_hits, work, err, st)
-                  : launch_wide_leaf(sc, b.rays[0], tiles.positions, nullptr, nullptr, nullptr, nullptr, b.cam_hits,
-                                     work, err, 6, 4, st)) != cudaSuccess)
+                  : launch_wide_leaf(sc, b.rays[0], tiles.positions, nullptr, nullptr, b.cam_hits, work, err, st)) !=
+        cudaSuccess)
       return e;
   } else if (p.max_bounces > 0) {
     if (sc.depth <= 32)
@@ -373,8 +373,8 @@ cudaError_t launch_render_wavefront(const DevScene &sc, const rt_camera &cam, co
                          cudaSuccess)
           return e;
         if ((!alone || cap > pool_max_rays(sc)) &&
-            (e = launch_wide_leaf(sc, b.rays[in], cap, count, perm, nullptr, nullptr, b.hits, work + (bounce & 1),
-                                  err, 6, 4, st, alone ? pool_max_rays(sc) + 1 : 0)) != cudaSuccess)
+            (e = launch_wide_leaf(sc, b.rays[in], cap, count, perm, b.hits, work + (bounce & 1), err, st,
+                                  alone ? pool_max_rays(sc) + 1 : 0)) != cudaSuccess)
           return e;
       } else if (sc.depth <= 32) {
         k_wf_extend<32><<<extend_grid, kWfBlock, 0, st>>>(sc, reinterpret_cast<const float4 *>(b.rays[in]), cap,

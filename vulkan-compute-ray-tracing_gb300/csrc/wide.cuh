@@ -152,7 +152,7 @@ __device__ __forceinline__ int traverse_wide_lane(const DevScene &sc, const Trac
     }
     WideStep ws;
     wide_node_test(sc.bvh8, node, r, oct, closest, ws);
-    // Leaf refs were range-checked when the bvh8 was built (k_encode8).
+    // Leaf refs were range-checked when the bvh8 was built (k_quantize8).
     for (uint32_t m = ws.leafmask; m; m &= m - 1u)
       test_triangle(sc.tpre, sc.leaf_tri, ~pick8(ws.ref, (uint32_t)(__ffs(m) - 1)), r, closest, best, bu, bv);
     const int node_idx = node;
