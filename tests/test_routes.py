@@ -34,7 +34,8 @@ extern "C" int batched(int mode, uint64_t pixels, uint32_t w, uint32_t h, uint32
 extern "C" int fallback(int mode, uint64_t pixels, uint32_t w, uint32_t h) {
   return one_launch_fallback(opts(mode, pixels), params(w, h, 1, 8, 0));
 }
-extern "C" int direct(uint32_t ntris, uint32_t n, uint32_t line) { return direct_rays(ntris, n, line); }
+extern "C" int direct(uint32_t ntris, uint32_t n, uint32_t line) { return direct_rays(ntris, n, line, false); }
+extern "C" int chunk(uint32_t ntris, uint32_t n, uint32_t line) { return direct_rays(ntris, n, line, true); }
 """
 
 
@@ -117,7 +118,8 @@ def test_batches_that_are_cast_as_they_are(routes):
     for ntris in (4096, 20480, 81920, 99999):  # packets pay sooner
         assert routes.direct(ntris, 851967, line) and not routes.direct(ntris, 851968, line)
     for ntris in (1310720, 2048012):  # and later where triangles outnumber the rays
-        assert routes.direct(ntris, 2 * ntris - 1, line) and not routes.direct(ntris, 2 * ntris, line)
+        assert routes.direct(ntris, 3 * ntris // 2 - 1, line) and not routes.direct(ntris, 3 * ntris // 2, line)
+        assert routes.chunk(ntris, line - 1, line) and not routes.chunk(ntris, line, line)  # not beside other casts
     for ntris in (1, 20480, 1 << 30):
         assert not routes.direct(ntris, 1, 0)  # 0: never
         assert routes.direct(ntris, 0xf0000000, 0xffffffff) == (not 4096 <= ntris < 100000)

@@ -885,7 +885,8 @@ rt_status rtTraceClosestHost(rt_ctx *ctx, rt_scene_id id, const rt_ray *h_rays, 
     RayCells cells;
     // A large rest takes the whole chunks' route: camera rays 5M into 20K
     // triangles 1450 us, with the last 0.8M cast as they are 1630.
-    const bool direct = cast_direct(opts, d, m <= kHostSplit ? m : chunk_rays), sorted = !direct && opts.sort && m >= 65536;
+    const bool direct = cast_direct(opts, d, m <= kHostSplit ? m : chunk_rays, true);
+    const bool sorted = !direct && opts.sort && m >= 65536;
     const bool beams = sorted && opts.packet && beam_cast(opts, d);
     const uint32_t *gate = nullptr;
     if (e == cudaSuccess && sorted)

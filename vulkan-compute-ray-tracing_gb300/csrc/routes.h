@@ -9,25 +9,28 @@
 
 namespace rtgb {
 
-// Batches of fewer than this many rays, and of fewer than twice the triangles,
+// Batches of fewer than this many rays, and of fewer than 3/2 of the triangles,
 // are cast as they are, in input order: sorting them and tracing packets pays
 // where many camera rays meet each triangle. us, cast as they are / sorted and
 // in packets, camera rays into an icosphere: 1,280 triangles 1.05M rays 207 /
 // 231, 2.1M 381 / 374; 5,120 triangles 0.79M 203 / 200, 1.05M 257 / 237; 82K
 // 0.79M 362 / 300, 1.05M 456 / 336; 328K 1.05M 773 / 788; 1.31M triangles 1.05M
-// 1518 / 2460, 2.1M 2828 / 3004, 3.1M 4112 / 3815; into a grid mesh of 2.05M
-// triangles 3.1M 915 / 1013, 4.2M 1191 / 1203. Random rays are cast as they are
-// on either side, above the line after the 0.05 ms that finding out takes, so
+// 1523 / 2478, 1.9M 2585 / 2923, 2.1M 2835 / 3016, 3M 3947 / 3852; into a grid
+// mesh of 2.05M triangles 3.1M 915 / 1013. Random rays are cast as they are on
+// either side, above the line after the 0.05 ms that finding out takes, so
 // between 4,096 and 100,000 triangles the line is drawn at 13/16: the lowest
 // where the casts of the reference's tree in packets (0.79M into 82K 356, 0.92M
-// 382) would have been quicker.
+// 382) would have been quicker. Beside another batch packets' fewer instructions
+// count for more: two of 1.05M into 1.31M triangles 2848 / 3249, of 1.9M 4992 /
+// 4574. The chunks of a host batch always run so (2 x 4.19M through host arrays
+// from two threads, chunks of 2.1M: 767 / 950 Mrays/s) and keep the plain line.
 constexpr uint32_t kPacketMinRays = 1u << 20;
-inline bool direct_rays(uint32_t ntris, uint32_t n, uint32_t packet_min_rays) {
+inline bool direct_rays(uint32_t ntris, uint32_t n, uint32_t packet_min_rays, bool overlapped) {
   uint64_t line = packet_min_rays;
   if (ntris >= 4096 && ntris < 100000)
     line = line * 13 / 16;
-  else
-    line = std::max(line, line * 2 * ntris / kPacketMinRays);
+  else if (!overlapped)
+    line = std::max(line, line * 3 * ntris / (2 * kPacketMinRays));
   return n < line;
 }
 

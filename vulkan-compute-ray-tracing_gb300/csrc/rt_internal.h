@@ -147,9 +147,10 @@ inline int trace_stack_entries(const TraceOpts &o, const DevScene &sc) {
   return o.stack > need ? (o.stack <= 32 ? 32 : 64) : need;
 }
 
-// True when a batch of n rays goes to the 8-wide caster as it is.
 inline bool beam_cast(const TraceOpts &o, const DevScene &sc) { return o.beam == 1 || (o.beam == 2 && sc.median_tree); }
-inline bool cast_direct(const TraceOpts &o, const DevScene &sc, uint32_t n);
+// True when a batch of n rays goes to the 8-wide caster as it is; `overlapped`:
+// beside other casts.
+inline bool cast_direct(const TraceOpts &o, const DevScene &sc, uint32_t n, bool overlapped = false);
 
 // `counter` is a device word private to this launch (work distribution);
 // `refine` recomputes t, u, v of the winning triangle in fp64.
@@ -172,9 +173,9 @@ bool wide_ok(const DevScene &sc);
 inline bool use_wide(const TraceOpts &o, const DevScene &sc) {
   return o.wide && sc.ntris >= o.wide_min_tris && wide_ok(sc);
 }
-inline bool cast_direct(const TraceOpts &o, const DevScene &sc, uint32_t n) {
+inline bool cast_direct(const TraceOpts &o, const DevScene &sc, uint32_t n, bool overlapped) {
   return o.refill >= 32 && o.packet && o.defer && !beam_cast(o, sc) && use_wide(o, sc) &&
-         direct_rays(sc.ntris, n, o.packet_min_rays);
+         direct_rays(sc.ntris, n, o.packet_min_rays, overlapped);
 }
 // True when a sorted batch's order and packets are worth having only if its
 // rays share origins (gate_out of launch_raysort): the rest are cast directly.
