@@ -352,8 +352,8 @@ rt_status rtReadSegmentCounter(rt_ctx *ctx, uint64_t *out, int reset);
  * callers that may not allocate device memory — a host application whose
  * device memory is owned by another allocator or runtime, or code running
  * where cudaMalloc is forbidden. It allocates nothing: its scratch is a
- * fixed array inside the library (about 3.9 MB on every GPU that loads the
- * library, held until the process exits) plus static host buffers.
+ * fixed array inside the library (about 2 MB on every GPU that loads the
+ * library, held until the process exits) plus one static host word.
  *   d_triangles  n triangles in device memory (Bvh.h layout); a vertex
  *                coordinate that is NaN or infinite returns
  *                RT_ERR_INVALID_SCENE before any sorting starts
@@ -391,7 +391,11 @@ typedef struct rt_render_job {
 rt_status rtRenderBatch(rt_ctx *ctx, const rt_render_job *jobs, uint32_t n_jobs, void *stream);
 
 /* A resident job table for repeated batched launches. Scenes named by the
- * jobs must stay resident while the batch exists. */
+ * jobs must stay resident while the batch exists. Each side stream holds the
+ * scratch of its largest wavefront job for the batch's lifetime: 108 bytes a
+ * path (8 more, and 4 MB, with render.sort) of its pixels times the samples that fit 2^20
+ * paths, or of one sample where that memory cannot be had; outside
+ * hbm_budget_bytes. */
 typedef struct rt_batch rt_batch;
 rt_status rtBatchCreate(rt_ctx *ctx, const rt_render_job *jobs, uint32_t n_jobs, rt_batch **out);
 rt_status rtBatchDestroy(rt_ctx *ctx, rt_batch *batch);

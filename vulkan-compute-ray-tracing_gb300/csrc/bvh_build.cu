@@ -6,9 +6,9 @@
 //     the right (Bvh.h:175-197); the DFS stack pops the right child first and
 //     the creation counter names children 2k+1 / 2k+2 when the k-th inner
 //     node is popped (Bvh.h:178-192). So indices, child links and the order
-//     in which nodes draw rand() depend on n alone; the host derives them
-//     in O(n) (pop rank of the right child = parent + 1, of the left child =
-//     parent + 2*|right| ; inner rank = pop rank - leaves popped before).
+//     in which nodes draw rand() depend on n alone: pop rank of the right
+//     child = parent + 1, of the left child = parent + 2*|right|; inner
+//     rank = pop rank - leaves popped before (child_item).
 //   * Axis. rand() % 3 once per popped node, leaves included (Bvh.h:160):
 //     glibc's sequence (glibc_rand.cpp), drawn by k_axes.
 //   * Which triangles a child receives, and in what order, is the sorted
@@ -21,7 +21,7 @@
 // GPU organisation. All triangles live in one array `idx`; a node owns the
 // slice [off, off+n), and sorting a node in place leaves its children's
 // slices in their input order. A node's slice, indices and draw follow from
-// its path alone (item_at), so no kernel reads a node table. The build runs
+// its path alone (item_below), so no kernel reads a node table. The build runs
 // level by level from the root:
 //   1. Levels whose nodes exceed kSegCap (k_big_level): one cooperative grid
 //      partitions every range of the level at once, a round per introsort
