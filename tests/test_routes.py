@@ -92,7 +92,7 @@ def test_small_scenes_keep_the_megakernel(routes):
         assert not routes.paths(12, side, side, 8) and not routes.paths(20, side, side, 1)
     assert not routes.wavefront(2, 0, 256, 256, 2, 1, 0, 1012)
     assert not routes.wavefront(2, 0, 4096, 1, 4, 8, 0, 12012) and not routes.wavefront(2, 0, 1, 1, 2, 8, 0, 12012)
-    assert not routes.paths(112, 128, 128, 8) and not routes.paths(1012, 256, 256, 8)
+    assert not routes.paths(112, 128, 128, 8) and not routes.paths(1012, 256, 256, 4) and not routes.paths(5120, 256, 256, 3)
     assert not routes.paths(12012, 1, 65536, 8) and not routes.paths(12012, 1, 1, 8)
     assert not routes.wavefront(2, 0, 1, 1, 16, 8, 0, 1 << 20) and not routes.wavefront(2, 0, 1, 4096, 4, 4, 0, 320)
 
@@ -103,9 +103,10 @@ def test_larger_scenes_keep_their_waves_and_paths(routes):
             for w, h in ((48, 48), (500, 375), (256, 256), (1024, 48), (511, 513)):
                 assert routes.wavefront(2, 0, w, h, spp, 2, 0, ntris) and routes.wavefront(2, 0, w, h, spp, 8, 0, ntris)
         assert routes.wavefront(2, 0, 362, 363, 1, 8, 0, ntris) and not routes.wavefront(2, 0, 362, 362, 1, 8, 0, ntris)
-        for side in (3, 48, 128, 181):
+        for side in (3, 48, 128, 181, 256):
             assert routes.paths(ntris, side, side, 8)
         assert routes.paths(ntris, 256, 256, 2) == (ntris >= 10000)
+        assert routes.paths(ntris, 512, 128, 1) and not routes.paths(ntris, 128, 513, 8)
     for ntris in (1, 12, 320, 1 << 20):  # from 2^18 pixels up, and many samples
         assert routes.wavefront(2, 0, 512, 512, 1, 1, 0, ntris) and routes.wavefront(2, 0, 64, 64, 64, 8, 0, ntris)
     assert not routes.paths(1 << 20, 257, 256, 8)
@@ -116,7 +117,7 @@ def test_batches_that_are_cast_as_they_are(routes):
     for ntris in (1, 1280, 100000, 327680, 1 << 19):
         assert routes.direct(ntris, line - 1, line) and not routes.direct(ntris, line, line)
     for ntris in (4096, 20480, 81920, 99999):  # packets pay sooner
-        assert routes.direct(ntris, 851967, line) and not routes.direct(ntris, 851968, line)
+        assert routes.direct(ntris, 917503, line) and not routes.direct(ntris, 917504, line)
     for ntris in (1310720, 2048012):  # and later where triangles outnumber the rays
         assert routes.direct(ntris, 3 * ntris // 2 - 1, line) and not routes.direct(ntris, 3 * ntris // 2, line)
         assert routes.chunk(ntris, line - 1, line) and not routes.chunk(ntris, line, line)  # not beside other casts

@@ -18,9 +18,9 @@ namespace rtgb {
 // 1523 / 2478, 1.9M 2585 / 2923, 2.1M 2835 / 3016, 3M 3947 / 3852; into a grid
 // mesh of 2.05M triangles 3.1M 915 / 1013. Random rays are cast as they are on
 // either side, above the line after the 0.05 ms that finding out takes, so
-// between 4,096 and 100,000 triangles the line is drawn at 13/16: the lowest
-// where the casts of the reference's tree in packets (0.79M into 82K 356, 0.92M
-// 382) would have been quicker. Beside another batch packets' fewer instructions
+// between 4,096 and 100,000 triangles the line is drawn at 7/8, from where casts on
+// the reference's tree in packets were clearly quicker (0.79M into 82K 356, 0.92M
+// 382). Beside another batch packets' fewer instructions
 // count for more: two of 1.05M into 1.31M triangles 2848 / 3249, of 1.9M 4992 /
 // 4574. The chunks of a host batch always run so (2 x 4.19M through host arrays
 // from two threads, chunks of 2.1M: 767 / 950 Mrays/s) and keep the plain line.
@@ -28,7 +28,7 @@ constexpr uint32_t kPacketMinRays = 1u << 20;
 inline bool direct_rays(uint32_t ntris, uint32_t n, uint32_t packet_min_rays, bool overlapped) {
   uint64_t line = packet_min_rays;
   if (ntris >= 4096 && ntris < 100000)
-    line = line * 13 / 16;
+    line = line * 7 / 8;
   else if (!overlapped)
     line = std::max(line, line * 3 * ntris / (2 * kPacketMinRays));
   return n < line;
@@ -68,22 +68,28 @@ inline uint64_t wave_min_samples(uint32_t ntris, const rt_render_params &p) {
 // cost more the fuller the GPU is. us, megakernel / paths.cu, 8 bounces: Cornell
 // box of 12 triangles 64 x 64 57 / 59, 256 x 256 70 / 150; of 32, 32 x 32 67 /
 // 55; of 112, 96 x 96 92 / 86, 180 x 180 98 / 129; of 1K, 180 x 180 223 / 198,
-// 256 x 256 266 / 325; of 3K, 96 x 96 361 / 140, 256 x 256 433 / 463; of 12K, 256
-// x 256 740 / 714. One bounce: of 312, 32 x 32 28 / 18, 128 x 128 20 / 30; of 1K,
-// 128 x 128 30 / 35, 180 x 180 28 / 41. One pixel, 5120 triangles: 8 / 10.
+// 256 x 256 266 / 325 and with 3 bounces 106 / 180 (the megakernel on the
+// reference's tree 406 and 153: the line keeps clear of what was slower than
+// that); of 3K, 96 x 96 361 / 140, 256 x 256 433 / 463; of 12K, 256 x 256 740 /
+// 714. One bounce: of 312, 32 x 32 28 / 18, 128 x 128 20 / 30; of 1K, 128 x 128 30
+// / 35, 180 x 180 28 / 41. Wide images, whose side rays leave the scene sooner,
+// take less: 443 x 110, 3K, 2 bounces 102 / 74 (221 x 221 101 / 126); 1024 x 48, 1K,
+// 8 bounces 216 / 129, 1 bounce 41 / 28. One pixel, 5120 triangles: 8 / 10.
 constexpr uint64_t kPathsMinPixels = 8;
-inline uint64_t paths_max_pixels(uint32_t ntris, uint32_t bounces) {
+inline uint64_t paths_max_pixels(uint32_t ntris, const rt_render_params &p) {
+  const uint32_t bounces = p.max_bounces;
+  const bool wide = p.width >= 4ull * p.height;
   if (ntris < 30) return 0;
   if (ntris < 100) return 1u << 10;
   if (ntris < 1000) return bounces <= 1 ? 1u << 11 : 10000;
-  if (ntris < 10000) return bounces <= 1 ? 1u << 14 : 1u << 15;
-  return 1u << 16;
+  if (ntris >= 10000 || wide || bounces >= (ntris < 3000 ? 5 : 4)) return 1u << 16;
+  return bounces <= 1 && ntris < 3000 ? 1u << 14 : 1u << 15;
 }
 inline bool paths_fit(uint32_t ntris, const rt_render_params &p) {
   const uint64_t pixels = (uint64_t)p.width * p.height;
   const bool thin = p.width < 8 || p.height < 4;
   const uint64_t extent = thin ? (uint64_t)((p.width + 7) / 8) * ((p.height + 3) / 4) * 32 : pixels;
-  return pixels >= kPathsMinPixels && extent <= paths_max_pixels(ntris, p.max_bounces);
+  return pixels >= kPathsMinPixels && extent <= paths_max_pixels(ntris, p);
 }
 
 constexpr uint64_t kWavefrontPixels = 1u << 17;
