@@ -182,7 +182,7 @@ rt_status rtTraceClosestHost(rt_ctx *ctx, rt_scene_id scene, const rt_ray *h_ray
  *                   to the 8-wide caster in input order, without the sort or
  *                   the packet pass; so do larger ones whose rays mostly have
  *                   origins of their own. The line is 7/8 of the value in
- *                   scenes of 4,096 to 100,000 triangles, and above 2^20 * 2/3
+ *                   scenes of 10,000 to 100,000 triangles, and above 2^20 * 2/3
  *                   triangles the value times triangles * 3/2 / 2^20 (not for
  *                   chunks of a host batch). The smallest
  *                   batches (up to 16,384 rays, 32,768 from 2^18 triangles up,

@@ -114,13 +114,13 @@ def test_larger_scenes_keep_their_waves_and_paths(routes):
 
 def test_batches_that_are_cast_as_they_are(routes):
     line = 1 << 20
-    for ntris in (1, 1280, 100000, 327680, 1 << 19):
+    for ntris in (1, 1280, 9999, 100000, 327680, 1 << 19):
         assert routes.direct(ntris, line - 1, line) and not routes.direct(ntris, line, line)
-    for ntris in (4096, 20480, 81920, 99999):  # packets pay sooner
+    for ntris in (10000, 20480, 81920, 99999):  # packets pay sooner
         assert routes.direct(ntris, 917503, line) and not routes.direct(ntris, 917504, line)
     for ntris in (1310720, 2048012):  # and later where triangles outnumber the rays
         assert routes.direct(ntris, 3 * ntris // 2 - 1, line) and not routes.direct(ntris, 3 * ntris // 2, line)
         assert routes.chunk(ntris, line - 1, line) and not routes.chunk(ntris, line, line)  # not beside other casts
     for ntris in (1, 20480, 1 << 30):
         assert not routes.direct(ntris, 1, 0)  # 0: never
-        assert routes.direct(ntris, 0xf0000000, 0xffffffff) == (not 4096 <= ntris < 100000)
+        assert routes.direct(ntris, 0xf0000000, 0xffffffff) == (not 10000 <= ntris < 100000)

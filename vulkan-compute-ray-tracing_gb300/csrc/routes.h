@@ -17,17 +17,18 @@ namespace rtgb {
 // 0.79M 362 / 300, 1.05M 456 / 336; 328K 1.05M 773 / 788; 1.31M triangles 1.05M
 // 1523 / 2478, 1.9M 2585 / 2923, 2.1M 2835 / 3016, 3M 3947 / 3852; into a grid
 // mesh of 2.05M triangles 3.1M 915 / 1013. Random rays are cast as they are on
-// either side, above the line after the 0.05 ms that finding out takes, so
-// between 4,096 and 100,000 triangles the line is drawn at 7/8, from where casts on
-// the reference's tree in packets were clearly quicker (0.79M into 82K 356, 0.92M
-// 382). Beside another batch packets' fewer instructions
-// count for more: two of 1.05M into 1.31M triangles 2848 / 3249, of 1.9M 4992 /
-// 4574. The chunks of a host batch always run so (2 x 4.19M through host arrays
-// from two threads, chunks of 2.1M: 767 / 950 Mrays/s) and keep the plain line.
+// either side, above the line after the 0.05 ms that finding out takes, so the
+// line is drawn at 7/8 only where casts in packets on the reference's tree were
+// clearly quicker (82K triangles 0.79M 356, 0.92M 382, 20K 1.05M 290; 5,120 1.05M
+// 250): between 10,000 and 100,000 triangles. Beside another batch packets' fewer
+// instructions count for more: two of 1.05M into 1.31M triangles 2848 / 3249, of
+// 1.9M 4992 / 4574. The chunks of a host batch always run so (2 x 4.19M through
+// host arrays from two threads, chunks of 2.1M: 767 / 950 Mrays/s) and keep the
+// plain line.
 constexpr uint32_t kPacketMinRays = 1u << 20;
 inline bool direct_rays(uint32_t ntris, uint32_t n, uint32_t packet_min_rays, bool overlapped) {
   uint64_t line = packet_min_rays;
-  if (ntris >= 4096 && ntris < 100000)
+  if (ntris >= 10000 && ntris < 100000)
     line = line * 7 / 8;
   else if (!overlapped)
     line = std::max(line, line * 3 * ntris / (2 * kPacketMinRays));
